@@ -668,20 +668,35 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
     return rc;
   ff.erfc_tab = nullptr;
   ff.vir_tab = nullptr;
+  ff.pair_tab = nullptr;
   ff.etab_key0 = ff.etab_nseg = 0;
   if (c.ewald) {
     std::vector<double> et, vt;
-    double *d_et = nullptr, *d_vt = nullptr;
+    double *d_et = nullptr, *d_vt = nullptr, *d_pt = nullptr;
     erfc_table(ff.alpha, ff.rcutCoulSq, et, &ff.etab_key0, &ff.etab_nseg);
     erfc_table(ff.alpha, ff.rcutCoulSq, vt, &ff.etab_key0, &ff.etab_nseg,
                true);
-    if ((rc = Alloc(&d_et, et.size())) ||
+    // FF::pair_tab
+    const std::vector<double> *src[2] = {&et, &vt};
+    std::vector<double> pt((size_t)ff.etab_nseg * 16);
+    for (int seg = 0; seg < ff.etab_nseg; ++seg)
+      for (int w = 0; w < 2; ++w) {
+        const double *cf = src[w]->data() + (size_t)seg * (ETAB_DEG + 1);
+        double *o = pt.data() + ((size_t)seg * 2 + w) * 8;
+        const float hi[4] = {(float)cf[6], (float)cf[7], (float)cf[8], 0.0f};
+        std::memcpy(o, cf, 6 * sizeof(double));
+        std::memcpy(o + 6, hi, sizeof(hi));
+      }
+    if ((rc = Alloc(&d_pt, pt.size())) ||
+        (rc = up(d_pt, pt.data(), pt.size() * sizeof(double))) ||
+        (rc = Alloc(&d_et, et.size())) ||
         (rc = up(d_et, et.data(), et.size() * sizeof(double))) ||
         (rc = Alloc(&d_vt, vt.size())) ||
         (rc = up(d_vt, vt.data(), vt.size() * sizeof(double))))
       return rc;
     ff.erfc_tab = d_et;
     ff.vir_tab = d_vt;
+    ff.pair_tab = d_pt;
   }
   if ((rc = up(d_ff, &ff, sizeof(FF))))
     return rc;
@@ -1548,11 +1563,12 @@ int Box::SetBox(const double L[3], const double *xyz, const double *com) {
     return rc;
   // force-field constants that depend on the edges (the mixed form's FP32
   // turn length); the erfc table does not
-  const double *etab = ff.erfc_tab, *vtab = ff.vir_tab;
+  const double *etab = ff.erfc_tab, *vtab = ff.vir_tab, *ptab = ff.pair_tab;
   int key0 = ff.etab_key0, nseg = ff.etab_nseg;
   build_ff(s, cfg, &ff);
   ff.erfc_tab = etab;
   ff.vir_tab = vtab;
+  ff.pair_tab = ptab;
   ff.etab_key0 = key0;
   ff.etab_nseg = nseg;
   if ((rc = CudaCheck(cudaMemcpyAsync(d_ff, &ff, sizeof(FF),

@@ -1,12 +1,11 @@
 // Real-space kernels (FP64 plain form):
-//   BoxInter        one CTA per (cell, neighbour) tile, i < j pairs
-//                   (src/CalculateEnergy.cpp:157-266)
+//   BoxInter        pair walk, a warp per atom, each pair once
+//                   (src/CalculateEnergy.cpp:157-266); VirialCalc likewise
 //   MoleculeInter   one CTA per (atom, old/new, neighbour cell)
 //                   (src/CalculateEnergy.cpp:581-686)
 //   ParticleInter   one CTA per (trial, neighbour cell)
 //                   (src/CalculateEnergy.cpp:727-785)
-//   BoxForce        one CTA per (cell, third of the neighbour shell); each
-//                   thread gathers the force on one atom, so no atomics
+//   BoxForce        pair walk from both ends, no atomics
 //                   (src/CalculateEnergy.cpp:268-406)
 //   MolCorrection   per molecule (src/Ewald.cpp:1056-1085)
 //   CalculateTorque per molecule (src/CalculateEnergy.cpp:1365-1406)
@@ -51,276 +50,363 @@ __global__ void k_reduce_partials(const double *__restrict__ part, int n, int w,
   }
 }
 
-// ---------------------------------------------------------------------------
-// BoxInter
-// ---------------------------------------------------------------------------
-// A warp scans its 32 atoms of cell c against the neighbour cell with an
-// FP32 distance pre-filter (its radius padded beyond FP32 position
-// rounding) and queues the candidate pairs (i < j atom ids, other molecule)
-// in shared memory; every 32 queued pairs are evaluated in FP64 by the full
-// warp, with the exact FP64 cutoff test.  The FP64 energy work then scales
-// with the pairs inside the cutoff, not with the pairs scanned.
-constexpr int QW = 64;  // queue slots per warp
-
-// Bulk asynchronous copies (the TMA engine's untiled form) from global to
-// this CTA's shared memory, completed on an mbarrier: the copy engine moves
-// a cell's slots while no thread issues a load.  Addresses and sizes are
-// multiples of 16 bytes (cell slot arrays are padded to multiples of 32).
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src,
-                                         unsigned bytes, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n"
-      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait on phase 0 of the barrier; false (and the box's error word
-// set) when it gives up, after a second bounded wait for the copies.
-__device__ bool mbar_wait_bounded(uint64_t *bar, int *err) {
-  constexpr unsigned LIMIT = 1u << 22;
-  for (unsigned it = 0; it < LIMIT; ++it)
-    if (mbar_try_wait(bar, 0))
-      return true;
-  atomicOr(err, DERR_BARRIER_TIMEOUT);
-  for (unsigned it = 0; it < LIMIT; ++it)
-    if (mbar_try_wait(bar, 0))
-      break;
-  return false;
+// Column blockIdx.x of `n` partials of width gridDim.x, fixed order.
+constexpr int RCT = 512;
+__global__ void __launch_bounds__(RCT) k_reduce_cols(const double *__restrict__ part,
+                                                     int n, int w, double *out) {
+  __shared__ double sh[RCT / 32];
+  double v = 0.0;
+  for (int i = threadIdx.x; i < n; i += RCT)
+    v += part[(size_t)i * w + blockIdx.x];
+  const double r = block_sum<RCT>(v, sh);
+  if (threadIdx.x == 0)
+    out[blockIdx.x] = r;
 }
 
-// One CTA per (cell c, neighbour cell c2) tile.  Thread 0 starts bulk copies
-// of both cells' slots (positions and charges, meta words, atom ids) into
-// shared memory; then every warp scans 32 atoms of c against c2.
-__global__ void __launch_bounds__(RT) k_box_inter(DevBox b, const FF *__restrict__ pff,
-                                                  double *part) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ int2 queue[RT / 32][QW];
-  __shared__ __align__(8) uint64_t bar;
-  const FF &ff = *pff;
-  int tile = blockIdx.x;
-  int c = tile / NB27, n = tile % NB27;
-  int c2 = b.nbr[c * NB27 + n];
-  int n1 = b.cell_count[c], n2 = b.cell_count[c2];
-  if (n1 == 0 || n2 == 0) {  // no pair in this tile
-    if (threadIdx.x == 0) {
-      part[2 * tile] = 0.0;
-      part[2 * tile + 1] = 0.0;
-    }
+// ---------------------------------------------------------------------------
+// The pair walk of BoxInter, VirialCalc and BoxForce.
+//
+// FP64 bounds all three: GB300 retires two FP64 lanes per SM and clock and a
+// warp instruction costs the same with 1 active lane as with 32, so what
+// counts is the number of FP64 warp instructions, and FP32 and integer work
+// is 64 times cheaper.  Hence:
+//   * a warp takes one atom at a time and scans the cells around it on the
+//     32-bit fixed-point turns of the grid (the difference of two turns wraps
+//     by itself), 32 neighbours a step, with an FP32 distance test whose
+//     radius is padded beyond its rounding; survivors are compacted into a
+//     queue of the warp, and FP64 runs on full batches of 32 pairs, with the
+//     exact FP64 cutoff test;
+//   * energies and the virial take each pair once (cells c2 > c, and later
+//     slots of the own cell), the force walk takes a pair from both ends: the
+//     warp's lanes then hold one atom's force, so no atomics are needed and
+//     every sum has a fixed order;
+//   * comparisons of FP64 values are made on their bits, a minimum-image
+//     shift is added only where a lane of the batch needs one, Lennard-Jones
+//     terms are skipped for a batch without any (a hydrogen's whole walk),
+//     1 / r^2 starts from the FP32 reciprocal, and of the Coulomb segment
+//     polynomial only degrees 0-5 are FP64 (degrees 6-8 add less than 1e-9 of
+//     the value, so their FP32 rounding stays below 1e-16 of it).
+// One CTA of four warps takes every (grid.y * 4)-th atom of a cell; grid.y is
+// set so that a warp has one atom in small boxes and up to eight in large
+// ones (pair_split).  Measured on 8,000 waters, Rcut 10 A, against one CTA
+// per cell pair (energies, virial) or per third of a neighbour shell
+// (forces): the calls forces + reciprocal + torque 31.4 -> 24.6 ms, virial
+// 15.9 -> 12.7 ms; SystemTotal of 20,000 waters 72.9 -> 70.6 ms.
+// ---------------------------------------------------------------------------
+constexpr int PW = RT / 32;  // warps per CTA
+constexpr int PQ = 64;       // queue slots per warp: one batch plus a scan step
+
+__device__ __forceinline__ long long bits64(double v) {
+  return __double_as_longlong(v);
+}
+// a > b of two non-negative values (NaN above all), on the integer pipe
+__device__ __forceinline__ bool gt_pos(double a, double b) {
+  return bits64(a) > bits64(b);
+}
+
+// min_image on a full warp (the same result): the shift is an FP64 addition
+// only for a batch in which some lane crosses half a box.
+__device__ __forceinline__ double min_image_warp(double raw, double ax,
+                                                 double half) {
+  const bool far = (bits64(raw) & 0x7fffffffffffffffLL) > bits64(half);
+  if (__any_sync(0xffffffffu, far)) {
+    const double sh = far ? copysign(ax, raw) : 0.0;
+    raw -= sh;
+  }
+  return raw;
+}
+
+// FP32 value of a positive FP64 number in FP32's normal range, truncated, and
+// the exact FP64 value of a normal FP32 one, by moving bits: the conversion
+// instructions run at the FP64 rate.
+__device__ __forceinline__ float trunc_f32(double v) {
+  const long long b = bits64(v);
+  return __int_as_float((int)(b >> 29) - (896 << 23));
+}
+__device__ __forceinline__ double widen_f64(float f) {
+  const int b = __float_as_int(f);
+  const int hi = (b & 0x80000000) | (((b & 0x7fffffff) >> 3) + (896 << 20));
+  return __hiloint2double(hi, b << 29);
+}
+
+// 1 / s to the last bit or two, s positive and well inside FP32's range: the
+// FP32 reciprocal (relative error e below 2^-21), one cubic step (e^3) and a
+// final correction.
+__device__ __forceinline__ double recip_pos(double s) {
+  double y = widen_f64(__frcp_rn(trunc_f32(s)));
+  double e = fma(-s, y, 1.0);
+  y = fma(y, fma(e, e, e), y);
+  return fma(fma(-s, y, 1.0), y, y);
+}
+// recip_pos and the bit conversions hold for 2^-60 < s < 2^60
+__device__ __forceinline__ bool in_fast_range(double s) {
+  const int e = __double2hiint(s) >> 20;
+  return e > 1023 - 60 && e < 1023 + 60;
+}
+
+// Segment polynomial `which` (0 energy, 1 force factor) of ff.pair_tab at
+// s; false outside its range.  The segment and the position u in [-1, 1) in
+// it come from the bits of s, as in seg_poly.
+__device__ __forceinline__ bool pair_poly(const FF &ff, int which, double s,
+                                          double *out) {
+  const long long b = bits64(s);
+  const int seg = (int)(b >> 46) - ff.etab_key0;
+  if (ff.pair_tab == nullptr || (unsigned)seg >= (unsigned)ff.etab_nseg)
+    return false;
+  const double u = fma(
+      2.0, __longlong_as_double(((b << 6) & 0x000fffffffffffffLL) |
+                                0x3ff0000000000000LL), -3.0);
+  const float uf = fmaf(
+      2.0f, __int_as_float(((int)(b >> 23) & 0x007fffff) | 0x3f800000), -3.0f);
+  const double2 *c = (const double2 *)(ff.pair_tab + ((size_t)seg * 2 + which) * 8);
+  const double2 c01 = __ldg(c), c23 = __ldg(c + 1), c45 = __ldg(c + 2);
+  const float4 f = __ldg((const float4 *)(c + 3));  // degrees 6, 7, 8
+  const float t = fmaf(fmaf(f.z, uf, f.y), uf, f.x);
+  double p = fma(widen_f64(t), u, c45.y);
+  p = fma(p, u, c45.x);
+  p = fma(p, u, c23.y);
+  p = fma(p, u, c23.x);
+  p = fma(p, u, c01.y);
+  *out = fma(p, u, c01.x);
+  return true;
+}
+
+// Scan constants of a box: FP32 edge of 2^-23 turns squared, and the padded
+// squared cutoff.  A turn difference is cut to 23 bits (L 2^-23 at most), the
+// turns themselves are within L 2^-32: the pad of 1e-6 of the longest edge
+// and 1e-4 of Rcut^2 covers both.
+struct Scan {
+  float sx, sy, sz, cut;
+};
+__device__ __forceinline__ Scan scan_of(const DevBox &b, const FF &ff) {
+  const float t = 1.1920929e-7f;  // 2^-23
+  const float lx = (float)b.L[0] * t, ly = (float)b.L[1] * t,
+              lz = (float)b.L[2] * t;
+  const float rp = (float)ff.rcut + 1e-6f * fmaxf((float)b.L[0],
+                                                  fmaxf((float)b.L[1],
+                                                        (float)b.L[2]));
+  return {lx * lx, ly * ly, lz * lz, rp * rp * 1.0001f};
+}
+// FP32 of a signed turn difference in units of 2^-23 turns: the top 23 bits
+// placed in the mantissa of 1.5 * 2^23.
+__device__ __forceinline__ float turn_f32(uint32_t a, uint32_t b) {
+  return __int_as_float(0x4B400000 + ((int)(a - b) >> 9)) - 12582912.0f;
+}
+__device__ __forceinline__ bool scan_near(const Scan &s, const uint4 &a,
+                                          const uint4 &b) {
+  const float dx = turn_f32(a.x, b.x), dy = turn_f32(a.y, b.y),
+              dz = turn_f32(a.z, b.z);
+  return fmaf(dx * dx, s.sx, fmaf(dy * dy, s.sy, dz * dz * s.sz)) < s.cut;
+}
+
+// The exact separation of a batch's pairs; true where the pair is inside the
+// cutoff (act lanes only).
+__device__ __forceinline__ bool pair_sep(const DevBox &b, const FF &ff, bool act,
+                                         const double4_32a &pi,
+                                         const double4_32a &pj, double v[3],
+                                         double *distSq) {
+  v[0] = min_image_warp(pi.x - pj.x, b.L[0], b.half[0]);
+  v[1] = min_image_warp(pi.y - pj.y, b.L[1], b.half[1]);
+  v[2] = min_image_warp(pi.z - pj.z, b.L[2], b.half[2]);
+  *distSq = dsq3(v[0], v[1], v[2]);
+  return act && gt_pos(ff.rcutSq, *distSq);
+}
+
+// Whether a pair's Lennard-Jones terms can be other than zero: a zero
+// epsilon gives zero unless (sigma^2 / r^2)^6 overflows.
+__device__ __forceinline__ bool lj_live(const FF &ff, double distSq, int idx) {
+  return ff.eps_cn[idx] != 0.0 || !in_fast_range(distSq);
+}
+
+// lj_energy and lj_virial of one pair (either may be NULL), sharing 1 / r^2.
+__device__ __forceinline__ void lj_terms(const FF &ff, double s, int idx,
+                                         double *en, double *vir) {
+  if (bits64(ff.nexp[idx]) == bits64(12.0) && in_fast_range(s)) {
+    const double y = recip_pos(s);
+    const double rRat2 = y * ff.sigmaSq[idx];
+    const double attract = rRat2 * rRat2 * rRat2;
+    const double repulse = attract * attract;
+    if (en)
+      *en = ff.eps_cn[idx] * (repulse - attract);
+    if (vir)
+      *vir = ff.eps_cn_6[idx] * (ff.nOver6[idx] * repulse - attract) * y;
     return;
   }
-  const int cap = b.cap;
-  double4_32a *sp = (double4_32a *)smem;  // neighbour cell c2
-  float4 *sf = (float4 *)(sp + cap);
-  int *sm = (int *)(sf + cap);
-  int *sa = sm + cap;
-  double4_32a *cp = (double4_32a *)(sa + cap);  // cell c
-  int *cm = (int *)(cp + cap);
-  int *ca = cm + cap;
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar))
-                 : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    const unsigned p1 = (unsigned)n1 * 32, p2 = (unsigned)n2 * 32;
-    const unsigned w1 = (unsigned)((n1 + 3) & ~3) * 4;
-    const unsigned w2 = (unsigned)((n2 + 3) & ~3) * 4;
-    asm volatile(
-        "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-            smem_u32(&bar)),
-        "r"(p1 + p2 + 2 * (w1 + w2))
-        : "memory");
-    const size_t o1 = (size_t)c * cap, o2 = (size_t)c2 * cap;
-    bulk_g2s(sp, b.cell_pos + o2, p2, &bar);
-    bulk_g2s(sm, b.cell_meta + o2, w2, &bar);
-    bulk_g2s(sa, b.cell_atom + o2, w2, &bar);
-    bulk_g2s(cp, b.cell_pos + o1, p1, &bar);
-    bulk_g2s(cm, b.cell_meta + o1, w1, &bar);
-    bulk_g2s(ca, b.cell_atom + o1, w1, &bar);
+  if (en)
+    *en = lj_energy(ff, s, idx);
+  if (vir)
+    *vir = lj_virial(ff, s, idx);
+}
+
+// Energies of one batch added to lj and re (every lane of the warp calls).
+__device__ __forceinline__ void batch_energy(const DevBox &b, const FF &ff,
+                                             bool act, int2 e, double &lj,
+                                             double &re) {
+  double4_32a pi = make_double4_32a(0, 0, 0, 0), pj = pi;
+  int idx = 0;
+  if (act) {
+    pi = b.cell_pos[e.x];
+    pj = b.cell_pos[e.y];
+    idx = meta_kind(b.cell_meta[e.x]) + meta_kind(b.cell_meta[e.y]) * ff.n_kinds;
   }
-  __syncthreads();  // the barrier is initialised before anyone waits on it
-  const bool ok = mbar_wait_bounded(&bar, b.err);
-  if (!ok)
-    return;  // the error word reports it; no partial is read
-  for (int j = threadIdx.x; j < n2; j += RT) {
-    const double4_32a p = sp[j];
-    sf[j] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.0f);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const float Lf[3] = {(float)b.L[0], (float)b.L[1], (float)b.L[2]};
-  const float Hf[3] = {(float)b.half[0], (float)b.half[1], (float)b.half[2]};
-  // FP32 positions are within L 2^-24 of the FP64 ones; the pre-filter
-  // radius covers twice that per axis plus 1e-4 of Rcut^2
-  const double lmax = fmax(b.L[0], fmax(b.L[1], b.L[2]));
-  const double rpad = ff.rcut + 1e-6 * lmax;
-  const float cut_f = (float)(rpad * rpad * 1.0001);
-  int2 *q = queue[warp];
-  double lj = 0.0, re = 0.0;
-  // FP64 energy of queued pair e (slot of cell c, slot of the neighbour cell)
-  auto eval = [&](int2 e) {
-    double4_32a pi = cp[e.x];
-    double4_32a pj = sp[e.y];
-    double dx = min_image(pi.x - pj.x, b.L[0], b.half[0]);
-    double dy = min_image(pi.y - pj.y, b.L[1], b.half[1]);
-    double dz = min_image(pi.z - pj.z, b.L[2], b.half[2]);
-    double distSq = dsq3(dx, dy, dz);
-    if (ff.rcutSq > distSq) {
-      int ki = meta_kind(cm[e.x]);
-      int kj = meta_kind(sm[e.y]);
-      if (ff.electrostatic) {
-        double qq = pi.w * pj.w * QQ_FACT;
-        if (qq != 0.0)
-          re += coulomb_energy(ff, distSq, qq);
-      }
-      lj += lj_energy(ff, distSq, ki + kj * ff.n_kinds);
-    }
-  };
-  int qn = 0;  // warp-uniform queue fill
-  for (int i0 = warp * 32; i0 < n1; i0 += RT) {
-    int i = i0 + lane;
-    bool act = i < n1;
-    int ai = -1, moli = -1;
-    float px = 0.0f, py = 0.0f, pz = 0.0f;
-    if (act) {
-      double4_32a p = cp[i];
-      px = (float)p.x;
-      py = (float)p.y;
-      pz = (float)p.z;
-      ai = ca[i];
-      moli = meta_mol(cm[i]);
-    }
-    for (int j = 0; j < n2; ++j) {
-      bool in = false;
-      if (act && ai < sa[j] && moli != meta_mol(sm[j])) {
-        float4 pj = sf[j];
-        float dx = px - pj.x, dy = py - pj.y, dz = pz - pj.z;
-        dx = dx > Hf[0] ? dx - Lf[0] : dx < -Hf[0] ? dx + Lf[0] : dx;
-        dy = dy > Hf[1] ? dy - Lf[1] : dy < -Hf[1] ? dy + Lf[1] : dy;
-        dz = dz > Hf[2] ? dz - Lf[2] : dz < -Hf[2] ? dz + Lf[2] : dz;
-        in = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut_f;
-      }
-      unsigned m = __ballot_sync(0xffffffffu, in);
-      if (in)
-        q[qn + __popc(m & lt)] = make_int2(i, j);
-      qn += __popc(m);
-      if (qn >= 32) {
-        __syncwarp();
-        eval(q[lane]);
-        int rest = qn - 32;
-        int2 mv = lane < rest ? q[32 + lane] : make_int2(0, 0);
-        __syncwarp();
-        if (lane < rest)
-          q[lane] = mv;
-        __syncwarp();
-        qn = rest;
-      }
+  double v[3], distSq;
+  const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+  if (ff.electrostatic && in) {
+    const double qq = pi.w * pj.w * QQ_FACT;
+    if (qq != 0.0) {
+      double p;
+      if (!gt_pos(distSq, ff.rcutCoulSq) && ff.ewald &&
+          pair_poly(ff, 0, distSq, &p))
+        re = fma(qq, p, re);
+      else
+        re += coulomb_energy(ff, distSq, qq);
     }
   }
-  __syncwarp();
-  if (lane < qn)
-    eval(q[lane]);
-  __shared__ double red[RT / 32];
-  double a = block_sum<RT>(lj, red);
-  double r = block_sum<RT>(re, red);
-  if (threadIdx.x == 0) {
-    part[2 * tile] = a;
-    part[2 * tile + 1] = r;
+  if (in && lj_live(ff, distSq, idx)) {
+    double l;
+    lj_terms(ff, distSq, idx, &l, nullptr);
+    lj += l;
   }
 }
 
-// ---------------------------------------------------------------------------
-// Pair virial (CalculateEnergy::VirialCalc CPU branch,
-// src/CalculateEnergy.cpp:458-519): the BoxInter tiles, each pair's force
-// factor times the product of its atom separation and the molecule-centre
-// separation, diagonal components; partials = LJ xx, yy, zz, then the
-// Coulomb factor (q_i q_j, without qqFact) xx, yy, zz.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(RT) k_box_virial(DevBox b, const FF *__restrict__ pff,
-                                                   double *part) {
-  extern __shared__ __align__(32) unsigned char smem[];
-  const FF &ff = *pff;
-  int tile = blockIdx.x;
-  int c = tile / NB27, n = tile % NB27;
-  int c2 = b.nbr[c * NB27 + n];
-  int n1 = b.cell_count[c], n2 = b.cell_count[c2];
-  double4_32a *sp = (double4_32a *)smem;
-  int *sm = (int *)(sp + b.cap);
-  int *sa = sm + b.cap;
-  for (int j = threadIdx.x; j < n2; j += RT) {
-    size_t s = (size_t)c2 * b.cap + j;
-    sp[j] = b.cell_pos[s];
-    sm[j] = b.cell_meta[s];
-    sa[j] = b.cell_atom[s];
+// Virial terms of one batch (src/CalculateEnergy.cpp:458-519): the force
+// factor times the product of the atom and the molecule-centre separation;
+// v6 = LJ xx, yy, zz, then Coulomb (q_i q_j, without qqFact) xx, yy, zz.
+__device__ __forceinline__ void batch_virial(const DevBox &b, const FF &ff,
+                                             bool act, int2 e, double v6[6]) {
+  double4_32a pi = make_double4_32a(0, 0, 0, 0), pj = pi;
+  int idx = 0, mi = 0, mj = 0;
+  if (act) {
+    pi = b.cell_pos[e.x];
+    pj = b.cell_pos[e.y];
+    mi = b.cell_meta[e.x];
+    mj = b.cell_meta[e.y];
+    idx = meta_kind(mi) + meta_kind(mj) * ff.n_kinds;
+    mi = meta_mol(mi);
+    mj = meta_mol(mj);
   }
-  __syncthreads();
-  double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < n1; i += RT) {
-    size_t si = (size_t)c * b.cap + i;
-    double4_32a pi = b.cell_pos[si];
-    int mi = b.cell_meta[si], ai = b.cell_atom[si];
-    int moli = meta_mol(mi), ki = meta_kind(mi);
-    for (int j = 0; j < n2; ++j) {
-      int aj = sa[j];
-      int mj = sm[j];
-      int molj = meta_mol(mj);
-      if (!(ai < aj && moli != molj))
-        continue;
-      double4_32a pj = sp[j];
-      double vc[3] = {min_image(pi.x - pj.x, b.L[0], b.half[0]),
-                      min_image(pi.y - pj.y, b.L[1], b.half[1]),
-                      min_image(pi.z - pj.z, b.L[2], b.half[2])};
-      double distSq = dsq3(vc[0], vc[1], vc[2]);
-      if (!(ff.rcutSq > distSq))
-        continue;
-      double cc[3] = {min_image(b.cx[moli] - b.cx[molj], b.L[0], b.half[0]),
-                      min_image(b.cy[moli] - b.cy[molj], b.L[1], b.half[1]),
-                      min_image(b.cz[moli] - b.cz[molj], b.L[2], b.half[2])};
-      if (ff.electrostatic) {
-        double qi_qj = pi.w * pj.w;
-        if (qi_qj != 0.0) {
-          double pRF = coulomb_virial(ff, distSq, qi_qj);
-          for (int d = 0; d < 3; ++d)
-            v[3 + d] += pRF * (vc[d] * cc[d]);
-        }
-      }
-      double pVF = lj_virial(ff, distSq, ki + meta_kind(mj) * ff.n_kinds);
+  double v[3], distSq;
+  const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+  double w[3];
+  w[0] = v[0] * min_image_warp(b.cx[mi] - b.cx[mj], b.L[0], b.half[0]);
+  w[1] = v[1] * min_image_warp(b.cy[mi] - b.cy[mj], b.L[1], b.half[1]);
+  w[2] = v[2] * min_image_warp(b.cz[mi] - b.cz[mj], b.L[2], b.half[2]);
+  if (ff.electrostatic && in) {
+    const double qi_qj = pi.w * pj.w;
+    if (qi_qj != 0.0) {
+      double p;
+      if (!gt_pos(distSq, ff.rcutCoulSq) && ff.ewald &&
+          pair_poly(ff, 1, distSq, &p))
+        p = qi_qj * p;
+      else
+        p = coulomb_virial(ff, distSq, qi_qj);
       for (int d = 0; d < 3; ++d)
-        v[d] += pVF * (vc[d] * cc[d]);
+        v6[3 + d] = fma(p, w[d], v6[3 + d]);
     }
   }
-  __shared__ double red[RT / 32];
-  for (int d = 0; d < 6; ++d) {
-    double r = block_sum<RT>(v[d], red);
-    if (threadIdx.x == 0)
-      part[6 * tile + d] = r;
+  if (in && lj_live(ff, distSq, idx)) {
+    double p;
+    lj_terms(ff, distSq, idx, nullptr, &p);
+    for (int d = 0; d < 3; ++d)
+      v6[d] = fma(p, w[d], v6[d]);
   }
+}
+
+// Every in-range pair once: MODE 0 the energies (partials LJ, real), 1 the
+// virial (six partials).
+template <int MODE>
+__global__ void __launch_bounds__(RT) k_box_pairs(DevBox b, const FF *__restrict__ pff,
+                                                  double *part) {
+  __shared__ int2 queue[PW][PQ];
+  const FF &ff = *pff;
+  const int c = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const Scan sc = scan_of(b, ff);
+  const int n1 = b.cell_count[c];
+  constexpr int NV = MODE ? 6 : 2;
+  double v[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    v[k] = 0.0;
+  int2 *q = queue[warp];
+  auto eval = [&](bool act, int2 e) {
+    if constexpr (MODE == 0)
+      batch_energy(b, ff, act, e, v[0], v[1]);
+    else
+      batch_virial(b, ff, act, e, v);
+  };
+  int qn = 0;  // warp-uniform queue fill
+  for (int s = blockIdx.y * PW + warp; s < n1; s += gridDim.y * PW) {
+    const int gi = c * b.cap + s;
+    const uint4 ti = b.cell_fix[gi];
+    const int moli = meta_mol(b.cell_meta[gi]);
+    for (int nn = 0; nn < NB27; ++nn) {
+      const int c2 = b.nbr[c * NB27 + nn];
+      if (c2 < c)
+        continue;
+      const int n2 = b.cell_count[c2];
+      for (int j0 = c2 == c ? s + 1 : 0; j0 < n2; j0 += 32) {
+        const int gj = c2 * b.cap + j0 + lane;
+        bool in = j0 + lane < n2;
+        if (in)
+          in = scan_near(sc, ti, b.cell_fix[gj]) &&
+               meta_mol(b.cell_meta[gj]) != moli;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in)
+          q[qn + __popc(m & lt)] = make_int2(gi, gj);
+        qn += __popc(m);
+        __syncwarp();
+        if (qn >= 32) {
+          const int2 e = q[lane];
+          const int2 mv = q[32 + lane];
+          __syncwarp();
+          qn -= 32;
+          if (lane < qn)
+            q[lane] = mv;
+          __syncwarp();
+          eval(true, e);
+        }
+      }
+    }
+  }
+  if (qn > 0)
+    eval(lane < qn, q[lane]);
+  __shared__ double red[PW];
+  const size_t t = (size_t)c * gridDim.y + blockIdx.y;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const double r = block_sum<RT>(v[k], red);
+    if (threadIdx.x == 0)
+      part[NV * t + k] = r;
+  }
+}
+
+// CTAs per cell: about 32 warps an SM in all, a warp taking one to eight
+// atoms (more atoms per warp fill the last batch of its queue better).
+static int pair_split(const Box &bx, const DevBox &b) {
+  const int avg = (b.n_atoms + b.ncell - 1) / b.ncell;
+  const int per = std::max(1, std::min(8, b.n_atoms / (32 * bx.sm_count)));
+  return std::max(1, (avg + PW * per - 1) / (PW * per));
+}
+
+template <int MODE>
+static int launch_pairs(Box &bx, const DevBox &b, double *d_out,
+                        const char *what) {
+  constexpr int NV = MODE ? 6 : 2;
+  const int split = pair_split(bx, b);
+  const int n = b.ncell * split;
+  int rc = bx.EnsureScratch((size_t)n * NV);
+  if (rc)
+    return rc;
+  k_box_pairs<MODE><<<dim3(b.ncell, split), RT, 0, bx.stream>>>(b, bx.d_ff,
+                                                                bx.d_scratch);
+  k_reduce_cols<<<NV, RCT, 0, bx.stream>>>(bx.d_scratch, n, NV, d_out);
+  return bx.CudaCheck(cudaGetLastError(), what);
 }
 
 int launch_box_virial(Box &bx, double *d_out6) {
-  DevBox &b = bx.dev;
-  int tiles = b.ncell * NB27;
-  int rc = bx.EnsureScratch((size_t)tiles * 6);
-  if (rc)
-    return rc;
-  size_t sh = (size_t)b.cap * (sizeof(double4_32a) + 2 * sizeof(int));
-  raise_smem_limit((const void *)k_box_virial, sh);
-  k_box_virial<<<tiles, RT, sh, bx.stream>>>(b, bx.d_ff, bx.d_scratch);
-  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, tiles, 6, d_out6, 0);
-  return bx.CudaCheck(cudaGetLastError(), "box virial");
+  return launch_pairs<1>(bx, bx.dev, d_out6, "box virial");
 }
 
 int launch_box_inter(Box &bx, double *d_out2) {
@@ -329,18 +415,7 @@ int launch_box_inter(Box &bx, double *d_out2) {
 
 // BoxInter on a view (its coordinates, cell grid and edges).
 int launch_box_inter_view(Box &bx, const DevBox &b, double *d_out2) {
-  int tiles = b.ncell * NB27;
-  int rc = bx.EnsureScratch((size_t)tiles * 2);
-  if (rc)
-    return rc;
-  // neighbour cell: positions, FP32 copies, meta, atom ids; cell c:
-  // positions, meta, atom ids
-  size_t sh = (size_t)b.cap * (2 * sizeof(double4_32a) + sizeof(float4) +
-                                4 * sizeof(int));
-  raise_smem_limit((const void *)k_box_inter, sh);
-  k_box_inter<<<tiles, RT, sh, bx.stream>>>(b, bx.d_ff, bx.d_scratch);
-  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, tiles, 2, d_out2, 0);
-  return bx.CudaCheck(cudaGetLastError(), "box inter");
+  return launch_pairs<0>(bx, b, d_out2, "box inter");
 }
 
 // ---------------------------------------------------------------------------
@@ -605,183 +680,146 @@ int launch_correction(Box &bx, double *d_out) {
 }
 
 // ---------------------------------------------------------------------------
-// BoxForce: CTA (cell c, group g of 9 neighbour cells); thread = atom of c.
-// Energies count each pair once (i < j); forces gather every pair.
+// BoxForce: the pair walk from both ends.  A warp's lanes hold partial forces
+// on its atom, added over the warp in a fixed order; energies count the pairs
+// that k_box_pairs takes.
 // ---------------------------------------------------------------------------
-constexpr int FG = 3;  // neighbour-shell groups
-// Each thread owns one atom of cell c per pass and gathers the force on it
-// from the CTA's third of the neighbour shell.  Per neighbour cell (staged in
-// shared memory with FP32 copies of the positions) a thread first marks the
-// neighbours that pass an FP32 distance pre-filter in a bit mask, then the
-// warp walks the masks together: in each round every thread evaluates its
-// next marked pair in FP64 (exact cutoff test, forces, and the energy of
-// pairs with i < j).  The FP64 work then follows the pairs inside the
-// cutoff, and each atom's sum runs over its pairs in neighbour order.
-constexpr int FMW = 8;  // 64-bit mask words per neighbour-cell chunk (512)
 __global__ void __launch_bounds__(RT) k_box_force(DevBox b, const FF *__restrict__ pff,
-                                                  double *fpart, double *epart) {
-  extern __shared__ __align__(32) unsigned char smem[];
+                                                  double *aF, double *epart) {
+  __shared__ unsigned queue[PW][PQ];
   const FF &ff = *pff;
-  int c = blockIdx.x, g = blockIdx.y;
-  int n1 = b.cell_count[c];
-  double4_32a *sp = (double4_32a *)smem;
-  float4 *sf = (float4 *)(sp + b.cap);
-  int *sm = (int *)(sf + b.cap);
-  int *sa = sm + b.cap;
-  const float Lf[3] = {(float)b.L[0], (float)b.L[1], (float)b.L[2]};
-  const float Hf[3] = {(float)b.half[0], (float)b.half[1], (float)b.half[2]};
-  // FP32 positions are within L 2^-24 of the FP64 ones; the pre-filter
-  // radius covers twice that per axis plus 1e-4 of Rcut^2
-  const double lmax = fmax(b.L[0], fmax(b.L[1], b.L[2]));
-  const double rpad = ff.rcut + 1e-6 * lmax;
-  const float cut_f = (float)(rpad * rpad * 1.0001);
+  const int c = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const Scan sc = scan_of(b, ff);
+  const int n1 = b.cell_count[c];
   double lj = 0.0, re = 0.0;
-  for (int base = 0; base < n1; base += RT) {
-    int i = base + threadIdx.x;
-    bool own = i < n1;
-    double4_32a pi = make_double4_32a(0, 0, 0, 0);
-    int mi = 0, ai = -1;
-    if (own) {
-      size_t si = (size_t)c * b.cap + i;
-      pi = b.cell_pos[si];
-      mi = b.cell_meta[si];
-      ai = b.cell_atom[si];
-    }
-    const float pxf = (float)pi.x, pyf = (float)pi.y, pzf = (float)pi.z;
+  unsigned *q = queue[warp];
+  for (int s = blockIdx.y * PW + warp; s < n1; s += gridDim.y * PW) {
+    const int gi = c * b.cap + s;
+    const uint4 ti = b.cell_fix[gi];
+    const double4_32a pi = b.cell_pos[gi];
+    const int mi = b.cell_meta[gi];
     const int moli = meta_mol(mi), ki = meta_kind(mi);
-    double fx = 0, fy = 0, fz = 0;
-    for (int nn = g * (NB27 / FG); nn < (g + 1) * (NB27 / FG); ++nn) {
-      int c2 = b.nbr[c * NB27 + nn];
-      int n2 = b.cell_count[c2];
-      __syncthreads();
-      for (int j = threadIdx.x; j < n2; j += RT) {
-        size_t s2 = (size_t)c2 * b.cap + j;
-        const double4_32a p = b.cell_pos[s2];
-        sp[j] = p;
-        sf[j] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.0f);
-        sm[j] = b.cell_meta[s2];
-        sa[j] = b.cell_atom[s2];
+    const double qi = pi.w * QQ_FACT;
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    // one batch: entries are slot << 1 | (the pair's energy is counted here)
+    auto eval = [&](bool act, unsigned e) {
+      const int gj = (int)(e >> 1);
+      const bool first = act && (e & 1);
+      double4_32a pj = make_double4_32a(0, 0, 0, 0);
+      int idx = 0;
+      if (act) {
+        pj = b.cell_pos[gj];
+        idx = ki + meta_kind(b.cell_meta[gj]) * ff.n_kinds;
       }
-      __syncthreads();
-      for (int jb = 0; jb < n2; jb += 64 * FMW) {
-        // candidates of this thread's atom among neighbours jb .. jb + 511
-        unsigned long long mk[FMW];
-#pragma unroll
-        for (int w = 0; w < FMW; ++w) {
-          unsigned long long m = 0;
-          const int j0 = jb + 64 * w;
-          if (own)
-            for (int k = 0; k < 64 && j0 + k < n2; ++k) {
-              const int j = j0 + k;
-              const float4 q = sf[j];
-              float dx = pxf - q.x, dy = pyf - q.y, dz = pzf - q.z;
-              dx = dx > Hf[0] ? dx - Lf[0] : dx < -Hf[0] ? dx + Lf[0] : dx;
-              dy = dy > Hf[1] ? dy - Lf[1] : dy < -Hf[1] ? dy + Lf[1] : dy;
-              dz = dz > Hf[2] ? dz - Lf[2] : dz < -Hf[2] ? dz + Lf[2] : dz;
-              if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut_f &&
-                  moli != meta_mol(sm[j]))
-                m |= 1ull << k;
-            }
-          mk[w] = m;
-        }
-        // rounds: every thread takes its next marked neighbour
-        for (;;) {
-          int j = -1;
-#pragma unroll
-          for (int w = 0; w < FMW; ++w)
-            if (j < 0 && mk[w]) {
-              const int k = __ffsll((long long)mk[w]) - 1;
-              mk[w] &= mk[w] - 1;
-              j = jb + 64 * w + k;
-            }
-          if (!__any_sync(0xffffffffu, j >= 0))
-            break;
-          if (j < 0)
-            continue;
-          const int mj = sm[j];
-          const double4_32a pj = sp[j];
-          double dx = min_image(pi.x - pj.x, b.L[0], b.half[0]);
-          double dy = min_image(pi.y - pj.y, b.L[1], b.half[1]);
-          double dz = min_image(pi.z - pj.z, b.L[2], b.half[2]);
-          double distSq = dsq3(dx, dy, dz);
-          if (ff.rcutSq > distSq) {
-            int idx = ki + meta_kind(mj) * ff.n_kinds;
-            double fR = 0.0;
-            bool hasR = false;
-            const bool first = ai < sa[j];
-            if (ff.electrostatic) {
-              double qq = pi.w * pj.w * QQ_FACT;
-              if (qq != 0.0) {
-                if (first)
-                  re += coulomb_energy(ff, distSq, qq);
-                fR = coulomb_virial(ff, distSq, qq);
-                hasR = true;
-              }
-            }
-            if (first)
-              lj += lj_energy(ff, distSq, idx);
-            double fL = lj_virial(ff, distSq, idx);
-            fx += dx * fL + (hasR ? dx * fR : 0.0);
-            fy += dy * fL + (hasR ? dy * fR : 0.0);
-            fz += dz * fL + (hasR ? dz * fR : 0.0);
+      double v[3], distSq;
+      const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+      double f = 0.0;
+      const bool table = in && !gt_pos(distSq, ff.rcutCoulSq) && ff.ewald;
+      if (ff.electrostatic && in) {
+        const double qq = qi * pj.w;
+        if (qq != 0.0) {
+          double p;
+          if (table && pair_poly(ff, 1, distSq, &p))
+            f = qq * p;
+          else
+            f = coulomb_virial(ff, distSq, qq);
+          if (first) {
+            if (table && pair_poly(ff, 0, distSq, &p))
+              re = fma(qq, p, re);
+            else
+              re += coulomb_energy(ff, distSq, qq);
           }
         }
       }
+      if (in && lj_live(ff, distSq, idx)) {
+        double l, p;
+        lj_terms(ff, distSq, idx, &l, &p);
+        if (first)
+          lj += l;
+        f += p;
+      }
+      if (in) {
+        fx = fma(v[0], f, fx);
+        fy = fma(v[1], f, fy);
+        fz = fma(v[2], f, fz);
+      }
+    };
+    int qn = 0;  // warp-uniform queue fill
+    for (int nn = 0; nn < NB27; ++nn) {
+      const int c2 = b.nbr[c * NB27 + nn];
+      const int n2 = b.cell_count[c2];
+      for (int j0 = 0; j0 < n2; j0 += 32) {
+        const int j = j0 + lane, gj = c2 * b.cap + j;
+        bool in = j < n2;
+        if (in)
+          in = scan_near(sc, ti, b.cell_fix[gj]) &&
+               meta_mol(b.cell_meta[gj]) != moli;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in)
+          q[qn + __popc(m & lt)] = (unsigned)gj << 1 | (c2 > c || (c2 == c && j > s) ? 1u : 0u);
+        qn += __popc(m);
+        __syncwarp();
+        if (qn >= 32) {
+          const unsigned e = q[lane], mv = q[32 + lane];
+          __syncwarp();
+          qn -= 32;
+          if (lane < qn)
+            q[lane] = mv;
+          __syncwarp();
+          eval(true, e);
+        }
+      }
     }
-    if (own) {
-      double *f = fpart + ((size_t)g * b.n_atoms + ai) * 3;
+    if (qn > 0)
+      eval(lane < qn, q[lane]);
+    __syncwarp();  // the queue is read before the next atom fills it
+    for (int o = 16; o > 0; o >>= 1) {
+      fx += __shfl_down_sync(0xffffffffu, fx, o);
+      fy += __shfl_down_sync(0xffffffffu, fy, o);
+      fz += __shfl_down_sync(0xffffffffu, fz, o);
+    }
+    if (lane == 0) {
+      double *f = aF + 3 * (size_t)b.cell_atom[gi];
       f[0] = fx;
       f[1] = fy;
       f[2] = fz;
     }
   }
-  __shared__ double red[RT / 32];
-  double A = block_sum<RT>(lj, red);
-  double R = block_sum<RT>(re, red);
+  __shared__ double red[PW];
+  const double A = block_sum<RT>(lj, red);
+  const double R = block_sum<RT>(re, red);
   if (threadIdx.x == 0) {
-    size_t t = (size_t)c * FG + g;
+    const size_t t = (size_t)c * gridDim.y + blockIdx.y;
     epart[2 * t] = A;
     epart[2 * t + 1] = R;
   }
 }
 
-__global__ void k_force_gather(DevBox b, const double *__restrict__ fpart,
-                               double *aF, double *mF) {
+__global__ void k_mol_force(DevBox b, const double *__restrict__ aF, double *mF) {
   int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= b.n_mol)
     return;
-  double mx = 0, my = 0, mz = 0;
-  for (int a = b.mstart[m]; a < b.mstart[m + 1]; ++a) {
-    double f[3] = {0, 0, 0};
-    for (int g = 0; g < FG; ++g)
-      for (int d = 0; d < 3; ++d)
-        f[d] += fpart[((size_t)g * b.n_atoms + a) * 3 + d];
+  double f[3] = {0, 0, 0};
+  for (int a = b.mstart[m]; a < b.mstart[m + 1]; ++a)
     for (int d = 0; d < 3; ++d)
-      aF[3 * (size_t)a + d] = f[d];
-    mx += f[0];
-    my += f[1];
-    mz += f[2];
-  }
-  mF[3 * (size_t)m] = mx;
-  mF[3 * (size_t)m + 1] = my;
-  mF[3 * (size_t)m + 2] = mz;
+      f[d] += aF[3 * (size_t)a + d];
+  for (int d = 0; d < 3; ++d)
+    mF[3 * (size_t)m + d] = f[d];
 }
 
 int launch_box_force(Box &bx, const DevBox &b, double *aF, double *mF,
                      double *d_out2) {
-  size_t need = (size_t)FG * b.n_atoms * 3 + (size_t)b.ncell * FG * 2;
-  int rc = bx.EnsureScratch(need);
+  const int split = pair_split(bx, b);
+  const int n = b.ncell * split;
+  int rc = bx.EnsureScratch((size_t)n * 2);
   if (rc)
     return rc;
-  double *fpart = bx.d_scratch;
-  double *epart = fpart + (size_t)FG * b.n_atoms * 3;
-  size_t sh = (size_t)b.cap * (sizeof(double4_32a) + sizeof(float4) +
-                                2 * sizeof(int));
-  raise_smem_limit((const void *)k_box_force, sh);
-  k_box_force<<<dim3(b.ncell, FG), RT, sh, bx.stream>>>(b, bx.d_ff, fpart, epart);
-  k_force_gather<<<(b.n_mol + 127) / 128, 128, 0, bx.stream>>>(b, fpart, aF,
-                                                              mF);
-  k_reduce_partials<<<1, RT, 0, bx.stream>>>(epart, b.ncell * FG, 2, d_out2, 0);
+  k_box_force<<<dim3(b.ncell, split), RT, 0, bx.stream>>>(b, bx.d_ff, aF,
+                                                          bx.d_scratch);
+  k_mol_force<<<(b.n_mol + 127) / 128, 128, 0, bx.stream>>>(b, aF, mF);
+  k_reduce_cols<<<2, RCT, 0, bx.stream>>>(bx.d_scratch, n, 2, d_out2);
   return bx.CudaCheck(cudaGetLastError(), "box force");
 }
 

@@ -1,0 +1,117 @@
+"""The box-wide walks and sums -- BoxInter, BoxForce, VirialCalc, the
+structure factor and the reciprocal forces -- against the oracle, where their
+tiling can go wrong: boxes of three cells per axis, edges that differ, one
+molecule, atom counts around the warp, batch and tile sizes, molecules of one
+to eight sites, a Coulomb cutoff below Rcut, a Mie exponent other than 12,
+and no Ewald sum.
+
+Bar: 1e-10 of the largest value of each output (of at least 1 K), the bar of
+the other FP64 tests.
+"""
+import numpy as np
+import pytest
+
+from gomc_gb300.config import SimConfig
+from gomc_gb300.systems import AtomKind, MolSystem, MoleculeType
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-10
+
+
+def mixture(counts, box, seed, charged=True):
+    """counts[t] molecules of type t (1, 3 and 8 sites) on a jittered grid of
+    at least 3.3 A, randomly assigned to its points."""
+    rng = np.random.default_rng(seed)
+    box = np.asarray(box, dtype=np.float64)
+    kinds = [AtomKind("A", 70.0, 2.9, 12.0), AtomKind("H", 0.0, 1.0, 12.0),
+             AtomKind("M", 45.0, 2.7, 14.0)]
+    sites = [np.zeros((1, 3)),
+             np.array([[0, 0, 0], [0.8, 0.55, 0], [-0.8, 0.55, 0.1]]),
+             np.array([[x, y, z] for x in (-.4, .4) for y in (-.4, .4)
+                       for z in (-.4, .4)], dtype=np.float64)]
+    akind = [[2], [0, 1, 1], [0, 1, 1, 1, 1, 1, 1, 2]]
+    q = [[0.35], [-0.8, 0.4, 0.4], [-0.7, .1, .1, .1, .1, .1, .1, 0.0]]
+    if not charged:
+        q = [[0.0] * len(c) for c in q]
+    types = [MoleculeType("T%d" % t, ["X%d" % i for i in range(len(s))],
+                          akind[t], q[t]) for t, s in enumerate(sites)]
+    n = np.maximum((box / 3.3).astype(int), 1)
+    grid = np.stack(np.meshgrid(*[np.arange(k) for k in n], indexing="ij"),
+                    -1).reshape(-1, 3)
+    pick = grid[rng.permutation(len(grid))[:sum(counts)]]
+    centre = (pick + 0.5) * (box / n) + rng.uniform(-0.2, 0.2, pick.shape)
+    pos, kind, chg, mol, start, mtype = [], [], [], [], [0], []
+    order = rng.permutation(np.repeat(np.arange(3), counts))
+    for m, t in enumerate(order):
+        a = rng.uniform(0, 2 * np.pi)
+        rot = np.array([[np.cos(a), -np.sin(a), 0], [np.sin(a), np.cos(a), 0],
+                        [0, 0, 1.0]])
+        pos.append(np.mod(centre[m] + sites[t] @ rot.T, box))
+        kind += akind[t]
+        chg += q[t]
+        mol += [m] * len(akind[t])
+        start.append(start[-1] + len(akind[t]))
+        mtype.append(t)
+    return MolSystem(box, kinds, types, np.concatenate(pos),
+                     np.array(kind, np.int32), np.array(chg),
+                     np.array(mol, np.int32), np.array(start, np.int32),
+                     np.array(mtype, np.int32))
+
+
+# molecules by type, edges, configuration
+CASES = {
+    "one_molecule": ((0, 0, 1), (20.0, 20.0, 20.0), {}),
+    "three_cells": ((60, 40, 3), (20.0, 23.1, 26.9), {}),
+    "odd_edges": ((301, 230, 17), (27.3, 31.1, 64.7), {}),
+    "coulomb_cut": ((100, 99, 1), (28.0, 28.0, 29.5),
+                    dict(rcut=9.0, rcut_coulomb=7.5)),
+    "no_ewald": ((128, 64, 5), (30.0, 27.5, 33.0), dict(ewald=False)),
+    "neutral": ((257, 100, 0), (31.0, 30.0, 36.0),
+                dict(ewald=False, electrostatic=False)),
+    "tile_128": ((128, 0, 0), (24.0, 24.0, 24.0), {}),
+    "tile_129": ((129, 0, 0), (24.0, 24.0, 24.0), {}),
+    "many_sites": ((1, 900, 301), (45.0, 47.0, 49.0), {}),
+}
+
+
+@pytest.fixture(scope="module")
+def gb():
+    from gomc_gb300 import engine
+    engine.lib(build_if_missing=True)
+    return engine
+
+
+def near(got, ref):
+    ref = np.asarray(ref, dtype=np.float64)
+    np.testing.assert_allclose(np.asarray(got).reshape(ref.shape), ref, rtol=0,
+                               atol=REL * max(np.abs(ref).max(), 1.0))
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_against_oracle(gb, name):
+    from oracle import oracle as orc
+    counts, edges, opt = CASES[name]
+    cfg = SimConfig(**{**dict(temperature=298.0, rcut=9.0, tolerance=1e-5),
+                       **opt})
+    s = mixture(counts, edges, 5, cfg.electrostatic)
+    box, ref = gb.Box(s, cfg), orc.OracleBox(s, cfg)
+    st, rt = box.system_total(), ref.system_total()
+    for k in ("inter", "real", "recip", "self", "correction", "total"):
+        near(st[k], rt[k])
+    aF, mF, lj, re = box.box_force()
+    rF = ref.box_force()
+    near(aF, rF[0])
+    near(mF, rF[1])
+    near(lj, rF[2])
+    near(re, rF[3])
+    if cfg.ewald:
+        near(box.sums_new(), ref.sum_new())
+        box.copy_recip()
+        ref.copy_recip()
+        aR, mR = box.box_force_reciprocal()
+        rR = ref.box_force_recip()
+        near(aR, rR[0])
+        near(mR, rR[1])
+    near(box.virial(), ref.virial())
+    box.close()
