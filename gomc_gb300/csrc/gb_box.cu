@@ -396,9 +396,8 @@ int Box::GridGeometry(const double L[3], const double *x, const double *y,
 }
 
 // Ewald::RecipInit (src/Ewald.cpp:835-903) for edges L into `ks`: the
-// k-vectors with their prefactors, the integer indices, and runs of up to
-// KRUN consecutive n_x per (n_y, n_z) column for the structure-factor
-// kernels (longest runs first).
+// k-vectors with their prefactors, the integer indices, and the (|n_y|,
+// |n_z|) pairs of the sums over all atoms.
 int Box::BuildKSet(const double L[3], KSet &ks) {
   std::vector<double> kx, ky, kz, hs, pf;
   std::vector<char4> kn;
@@ -409,46 +408,22 @@ int Box::BuildKSet(const double L[3], KSet &ks) {
     return Fail(ERR_UNSUPPORTED, "k-vector index above 127");
   const int K = (int)kx.size();
   std::vector<float> pff(pf.begin(), pf.end());
-  std::map<std::pair<int, int>, std::vector<std::pair<int, int>>> cols;
-  for (int k = 0; k < K; ++k)
-    cols[{kn[k].y, kn[k].z}].push_back({kn[k].x, k});
-  std::vector<int4> runs;
-  std::vector<int> run_k;
-  for (auto &c : cols) {
-    auto &v = c.second;  // n_x ascending (k vectors are listed x outer)
-    size_t i = 0;
-    while (i < v.size()) {
-      size_t j = i + 1;
-      while (j < v.size() && j - i < (size_t)KRUN &&
-             v[j].first == v[j - 1].first + 1)
-        ++j;
-      runs.push_back(make_int4(c.first.first, c.first.second, v[i].first,
-                               (int)(j - i)));
-      for (int g = 0; g < KRUN; ++g)
-        run_k.push_back(i + g < j ? v[i + g].second : -1);
-      i = j;
-    }
+  // largest n_x of every pair, pairs by it (largest first): neighbouring
+  // rows of the product then need about the same columns
+  const int S = kmax + 1;
+  std::vector<int> top((size_t)S * S, -1), pairs, at((size_t)S * S, 0);
+  for (int k = 0; k < K; ++k) {
+    int &t = top[std::abs(kn[k].y) * S + std::abs(kn[k].z)];
+    t = std::max(t, (int)kn[k].x);
   }
-  // longest runs first: neighbouring threads then take runs of equal
-  // length, and a warp skips the members none of its runs has (each run's
-  // sums do not depend on which thread takes it)
-  {
-    std::vector<int> order(runs.size());
-    for (size_t r = 0; r < runs.size(); ++r)
-      order[r] = (int)r;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-      return runs[x].w > runs[y].w;
-    });
-    std::vector<int4> r2(runs.size());
-    std::vector<int> k2(run_k.size());
-    for (size_t r = 0; r < runs.size(); ++r) {
-      r2[r] = runs[order[r]];
-      for (int g = 0; g < KRUN; ++g)
-        k2[r * KRUN + g] = run_k[(size_t)order[r] * KRUN + g];
-    }
-    runs.swap(r2);
-    run_k.swap(k2);
-  }
+  for (int n = kmax; n >= 0; --n)
+    for (int i = 0; i < S * S; ++i)
+      if (top[i] == n) {
+        at[i] = (int)pairs.size();
+        pairs.push_back(i / S | (i % S) << 8 | n << 16);
+      }
+  while (pairs.empty() || pairs.size() % 32)
+    pairs.push_back(0);
   int rc;
   if ((size_t)K > ks.cap) {
     if ((rc = regrow(*this, (void **)&ks.kx, (size_t)K * 8, allocs_)) ||
@@ -461,13 +436,15 @@ int Box::BuildKSet(const double L[3], KSet &ks) {
       return rc;
     ks.cap = K;
   }
-  if (runs.size() > ks.run_cap) {
-    if ((rc = regrow(*this, (void **)&ks.krun, runs.size() * sizeof(int4),
-                     allocs_)) ||
-        (rc = regrow(*this, (void **)&ks.krun_k, run_k.size() * sizeof(int),
-                     allocs_)))
+  if (pairs.size() > ks.pair_cap) {
+    if ((rc = regrow(*this, (void **)&ks.pair, pairs.size() * 4, allocs_)))
       return rc;
-    ks.run_cap = runs.size();
+    ks.pair_cap = pairs.size();
+  }
+  if (at.size() > ks.at_cap) {
+    if ((rc = regrow(*this, (void **)&ks.pair_at, at.size() * 4, allocs_)))
+      return rc;
+    ks.at_cap = at.size();
   }
   auto up = [&](void *dst, const void *src, size_t bytes) {
     return CudaCheck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice,
@@ -480,8 +457,8 @@ int Box::BuildKSet(const double L[3], KSet &ks) {
       (rc = up(ks.prefact, pf.data(), (size_t)K * 8)) ||
       (rc = up(ks.hsqr, hs.data(), (size_t)K * 8)) ||
       (rc = up(ks.kn, kn.data(), (size_t)K * 4)) ||
-      (rc = up(ks.krun, runs.data(), runs.size() * sizeof(int4))) ||
-      (rc = up(ks.krun_k, run_k.data(), run_k.size() * sizeof(int))) ||
+      (rc = up(ks.pair, pairs.data(), pairs.size() * 4)) ||
+      (rc = up(ks.pair_at, at.data(), at.size() * 4)) ||
       (rc = up(ks.prefact_f, pff.data(), (size_t)K * 4)))
     return rc;
   // the host vectors go out of scope: wait for the copies
@@ -489,7 +466,7 @@ int Box::BuildKSet(const double L[3], KSet &ks) {
     return rc;
   ks.K = K;
   ks.kmax = kmax;
-  ks.nrun = (int)runs.size();
+  ks.npair = (int)pairs.size();
   for (int d = 0; d < 3; ++d)
     ks.L[d] = L[d];
   return OK;
@@ -526,7 +503,7 @@ int Box::EnsureSums(size_t K) {
 void Box::MirrorKRef() {
   dev.K = kref.K;
   dev.kmax = kref.kmax;
-  dev.nrun = kref.nrun;
+  dev.npair = kref.npair;
   dev.kx = kref.kx;
   dev.ky = kref.ky;
   dev.kz = kref.kz;
@@ -534,14 +511,16 @@ void Box::MirrorKRef() {
   dev.hsqr = kref.hsqr;
   dev.kn = kref.kn;
   dev.prefact_f = kref.prefact_f;
-  dev.krun = kref.krun;
-  dev.krun_k = kref.krun_k;
+  dev.pair = kref.pair;
+  dev.pair_at = kref.pair_at;
 }
 
 int Box::EnsureScratch(size_t n) {
   if (n <= scratch_len)
     return OK;
-  int rc = Alloc(&d_scratch, n);
+  // the old array is done with once the stream's work is
+  scratch_len = 0;
+  int rc = regrow(*this, (void **)&d_scratch, n * sizeof(double), allocs_);
   if (rc)
     return rc;
   scratch_len = n;
@@ -621,6 +600,13 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
   double half[3] = {s.L[0] * 0.5, s.L[1] * 0.5, s.L[2] * 0.5};
   calc_com(s);
   build_ff(s, c, &ff);
+  double qmax = 0.0, qsum = 0.0;
+  for (int i = 0; i < N; ++i) {
+    qmax = std::max(qmax, std::fabs(s.q[i]));
+    qsum += std::fabs(s.q[i]);
+  }
+  std::frexp(qmax, &q_exp);
+  q_abs = std::ldexp(qsum, -q_exp);
   DevBox &d = dev;
   for (int k = 0; k < 3; ++k) {
     d.L[k] = s.L[k];
@@ -705,36 +691,11 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
     return rc;
 
   // Ewald tables: the k-vector set of the box edges and its structure
-  // factors; exp(2 pi i j / 256) (float-float) for the mixed form's phases
+  // factors
   if (c.ewald) {
     if ((rc = BuildKSet(s.L, kref)) || (rc = EnsureSums(kref.K)))
       return rc;
     MirrorKRef();
-    if ((rc = Alloc(&d.cis256, 256)))
-      return rc;
-    // exp(2 pi i j / 256) from the first octant by symmetry, each value
-    // split into FP32 hi + lo
-    std::vector<float4> cis(256);
-    for (int j = 0; j < 256; ++j) {
-      int o = j & 63;  // angle within its quarter turn, in 1/256 turns
-      bool flip = o > 32;
-      long double a = (flip ? 64 - o : o) * (3.14159265358979323846264338327950L / 128.0L);
-      double c = (double)cosl(a), sn = (double)sinl(a);
-      if (flip)
-        std::swap(c, sn);
-      double re, im;
-      switch (j >> 6) {
-        case 0: re = c; im = sn; break;
-        case 1: re = -sn; im = c; break;
-        case 2: re = -c; im = -sn; break;
-        default: re = sn; im = -c; break;
-      }
-      float rh = (float)re, ih = (float)im;
-      cis[j] = make_float4(rh, (float)(re - (double)rh), ih,
-                           (float)(im - (double)ih));
-    }
-    if ((rc = up(d.cis256, cis.data(), 256 * sizeof(float4))))
-      return rc;
   }
   if ((rc = GridAll()))
     return rc;
@@ -815,8 +776,6 @@ int Box::BoxInter(double *inter, double *real) {
 int Box::RecipSums(const double *x, const double *y, const double *z) {
   if (!cfg.ewald)
     return OK;
-  if (cfg.precision == 1)  // mixed form: float-float structure factor
-    return launch_recip_sums_ff(*this, x, y, z, dev.sumRnew, dev.sumInew);
   return launch_recip_sums(*this, x, y, z, dev.sumRnew, dev.sumInew);
 }
 
@@ -1482,7 +1441,7 @@ int Box::RecipSumsCoords(const double *xyz, bool new_set) {
   DevBox v = trial.v;
   v.K = ks.K;
   v.kmax = ks.kmax;
-  v.nrun = ks.nrun;
+  v.npair = ks.npair;
   v.kx = ks.kx;
   v.ky = ks.ky;
   v.kz = ks.kz;
@@ -1490,8 +1449,8 @@ int Box::RecipSumsCoords(const double *xyz, bool new_set) {
   v.hsqr = ks.hsqr;
   v.kn = ks.kn;
   v.prefact_f = ks.prefact_f;
-  v.krun = ks.krun;
-  v.krun_k = ks.krun_k;
+  v.pair = ks.pair;
+  v.pair_at = ks.pair_at;
   if ((rc = launch_recip_sums_view(*this, v, v.x, v.y, v.z, dev.sumRnew,
                                    dev.sumInew)))
     return rc;

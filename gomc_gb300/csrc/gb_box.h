@@ -17,15 +17,14 @@ struct McState;  // Monte Carlo loop state (gb_mc.cu)
 // current set (Ref) and a second one that RecipInit fills for trial edges
 // (New); UpdateRecipVec swaps them (src/Ewald.cpp:1462-1487).
 struct KSet {
-  int K = 0, kmax = 0, nrun = 0;
-  size_t cap = 0, run_cap = 0;  // allocated k-vectors, runs
+  int K = 0, kmax = 0, npair = 0;
+  size_t cap = 0, pair_cap = 0, at_cap = 0;  // allocated entries
   double L[3] = {0, 0, 0};
   double *kx = nullptr, *ky = nullptr, *kz = nullptr, *prefact = nullptr,
          *hsqr = nullptr;
   char4 *kn = nullptr;
   float *prefact_f = nullptr;
-  int4 *krun = nullptr;
-  int *krun_k = nullptr;
+  int *pair = nullptr, *pair_at = nullptr;
 };
 
 // Coordinates and cell grid of a trial state (other coordinates, other box
@@ -130,6 +129,10 @@ class Box {
   size_t sums_cap = 0;
   TrialState trial;
 
+  // charges: |q| < 2^q_exp, and their sum in units of 2^q_exp
+  int q_exp = 0;
+  double q_abs = 0.0;
+
   // scratch buffers
   double *d_scratch = nullptr;   // reduction partials
   size_t scratch_len = 0;
@@ -181,7 +184,7 @@ void recip_vectors(const double L[3], double volume, double alphaSq,
                    std::vector<double> &prefact, std::vector<char4> &kn,
                    int *kmax);
 
-// kernel launchers (gb_cells.cu / gb_real.cu / gb_recip.cu).  Launchers
+// kernel launchers (gb_cells.cu / gb_real.cu / gb_recip.cu / gb_ewald.cu).  Launchers
 // that take a DevBox run on that view (coordinates and cell grid), which lets
 // the MultiParticle move evaluate its trial state in separate buffers.
 int launch_grid_all(Box &b, const DevBox &d);
@@ -194,8 +197,12 @@ int launch_recip_sums(Box &b, const double *x, const double *y,
 int launch_recip_sums_view(Box &b, const DevBox &d, const double *x,
                            const double *y, const double *z, double *sumR,
                            double *sumI);
-int launch_recip_sums_ff(Box &b, const double *x, const double *y,
-                         const double *z, double *sumR, double *sumI);
+size_t recip_sums_scratch(int n_atoms, int kmax, int npair);
+// reciprocal forces without the intramolecular part as *nfp partials
+// [*nfp][3][n_atoms] in scratch, with `extra` doubles of it for the caller
+int launch_force_split(Box &b, const DevBox &d, const double *sumR,
+                       const double *sumI, size_t extra, double **fpart,
+                       int *nfp, double **extra_out);
 int launch_recip_energy(Box &b, const double *sumR, const double *sumI,
                         double *d_out);
 int launch_recip_energy_view(Box &b, const DevBox &d, const double *sumR,
@@ -212,6 +219,7 @@ int launch_cell_add_mol(Box &b, int m);
 int launch_correction(Box &b, double *d_out);
 int launch_box_force(Box &b, const DevBox &d, double *aF, double *mF,
                      double *d_out2);
+int launch_mol_force(Box &b, const DevBox &d, const double *aF, double *mF);
 int launch_force_recip(Box &b, const DevBox &d, const double *sumR,
                        const double *sumI, double *aR, double *mR);
 int launch_torque(Box &b, const DevBox &d, const double *aF, const double *aR,

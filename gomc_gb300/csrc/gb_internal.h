@@ -24,7 +24,6 @@ constexpr int MAX_KINDS = 8;
 constexpr int ETAB_DEG = 8;  // degree of the erfc(alpha r)/r segments
 constexpr int MAX_MOL_ATOMS = 8;   // rigid molecules handled by the move loop
 constexpr int END_CELL = -1;
-constexpr int KRUN = 8;  // k-vectors per run of the structure-factor kernel
 
 // Status codes of the C ABI (include/gomc_gb300.h).
 enum Status : int {
@@ -136,14 +135,13 @@ struct DevBox {
   int K, kmax;
   double *kx, *ky, *kz, *prefact, *hsqr;  // [K]
   char4 *kn;                              // [K] integer k indices
-  // runs of up to KRUN k-vectors with one (n_y, n_z) and consecutive n_x,
-  // for the full structure factor: (n_y, n_z, first n_x, length) and the
-  // k index of each member (-1 past the length)
-  int nrun;
-  int4 *krun;   // [nrun]
-  int *krun_k;  // [nrun * KRUN]
+  // pairs (|n_y|, |n_z|) of the k-vectors for the sums over all atoms,
+  // largest n_x first: |n_y| | |n_z| << 8 | largest n_x << 16, padded to a
+  // multiple of 32; and the place of a pair in that list
+  int npair;
+  int *pair;     // [npair]
+  int *pair_at;  // [(kmax + 1)^2]
   float *prefact_f;                       // [K]
-  float4 *cis256;  // [256] exp(2 pi i j / 256) as float-float (re, im)
   double *sumRref, *sumIref, *sumRnew, *sumInew;  // [K]
   // running energies: inter, real, recip, self, correction
   double *energy;

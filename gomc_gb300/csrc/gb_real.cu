@@ -50,17 +50,41 @@ __global__ void k_reduce_partials(const double *__restrict__ part, int n, int w,
   }
 }
 
-// Column blockIdx.x of `n` partials of width gridDim.x, fixed order.
-constexpr int RCT = 512;
+// Column blockIdx.x of `n` partials of width w, fixed order.  The threads'
+// sums are added with the rounding errors carried along (the large numbers
+// meet there).
+constexpr int RCT = 128;
+struct Sum2 {
+  double hi, lo;
+};
+__device__ __forceinline__ Sum2 add2(Sum2 a, double v, double lo) {
+  const double s = __dadd_rn(a.hi, v), t = __dadd_rn(s, -a.hi);
+  const double e = __dadd_rn(__dadd_rn(a.hi, -__dadd_rn(s, -t)),
+                             __dadd_rn(v, -t));
+  return {s, a.lo + (lo + e)};
+}
 __global__ void __launch_bounds__(RCT) k_reduce_cols(const double *__restrict__ part,
                                                      int n, int w, double *out) {
-  __shared__ double sh[RCT / 32];
-  double v = 0.0;
+  __shared__ Sum2 sh[RCT / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Sum2 v = {0.0, 0.0};
+#pragma unroll 4
   for (int i = threadIdx.x; i < n; i += RCT)
-    v += part[(size_t)i * w + blockIdx.x];
-  const double r = block_sum<RCT>(v, sh);
-  if (threadIdx.x == 0)
-    out[blockIdx.x] = r;
+    v.hi += part[(size_t)i * w + blockIdx.x];
+  for (int o = 16; o > 0; o >>= 1)
+    v = add2(v, __shfl_down_sync(0xffffffffu, v.hi, o),
+             __shfl_down_sync(0xffffffffu, v.lo, o));
+  if (lane == 0)
+    sh[warp] = v;
+  __syncthreads();
+  if (warp)
+    return;
+  v = lane < RCT / 32 ? sh[lane] : Sum2{0.0, 0.0};
+  for (int o = RCT / 64; o > 0; o >>= 1)
+    v = add2(v, __shfl_down_sync(0xffffffffu, v.hi, o),
+             __shfl_down_sync(0xffffffffu, v.lo, o));
+  if (lane == 0)
+    out[blockIdx.x] = isfinite(v.lo) ? v.hi + v.lo : v.hi;
 }
 
 // ---------------------------------------------------------------------------
@@ -809,6 +833,11 @@ __global__ void k_mol_force(DevBox b, const double *__restrict__ aF, double *mF)
     mF[3 * (size_t)m + d] = f[d];
 }
 
+int launch_mol_force(Box &bx, const DevBox &b, const double *aF, double *mF) {
+  k_mol_force<<<(b.n_mol + 127) / 128, 128, 0, bx.stream>>>(b, aF, mF);
+  return bx.CudaCheck(cudaGetLastError(), "molecule forces");
+}
+
 int launch_box_force(Box &bx, const DevBox &b, double *aF, double *mF,
                      double *d_out2) {
   const int split = pair_split(bx, b);
@@ -818,7 +847,8 @@ int launch_box_force(Box &bx, const DevBox &b, double *aF, double *mF,
     return rc;
   k_box_force<<<dim3(b.ncell, split), RT, 0, bx.stream>>>(b, bx.d_ff, aF,
                                                           bx.d_scratch);
-  k_mol_force<<<(b.n_mol + 127) / 128, 128, 0, bx.stream>>>(b, aF, mF);
+  if ((rc = launch_mol_force(bx, b, aF, mF)))
+    return rc;
   k_reduce_cols<<<2, RCT, 0, bx.stream>>>(bx.d_scratch, n, 2, d_out2);
   return bx.CudaCheck(cudaGetLastError(), "box force");
 }

@@ -208,7 +208,8 @@ size_t job_bytes(const Job &j, int K, int kmax, int csize, size_t moves) {
   if (mixed_smem(K, kmax, csize, true) > MIXED_SMEM_MAX)
     mc += mixed_cold_buffer(K, csize);
   // reduction scratch of the set-up kernels and allocation rounding
-  size_t scratch = (size_t)K * 16 + N * 8 + ((size_t)1 << 20);
+  size_t scratch = 8 * recip_sums_scratch((int)N, kmax, (kmax + 1) * (kmax + 1)) +
+                   ((size_t)1 << 20);
   return box + mc + scratch + 96 * 512;
 }
 
