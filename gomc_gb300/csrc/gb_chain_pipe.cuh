@@ -29,12 +29,13 @@
 //     and the flags of context(t + 1), in one poll -> commit(t - 1) ->
 //     phase A(t + 1);
 //   * decider at move t: CTA 0's flag of context(t) -> header -> every
-//     work CTA's partials(t) -> decision -> release of the word -> partial
-//     slots reset, coordinates written.
-// Contexts rotate over three buffers and partials over three slot sets: a
-// writer overwrites context t - 1's buffer while building context t + 2,
-// after it has seen decision t, which the decider gave only after every
-// work CTA had read context t - 1 and stored partials(t); a work CTA stores
+//     work CTA's partials(t) -> decision -> the word -> partial slots reset,
+//     coordinates written -> fence (it releases them with the next word).
+// Contexts rotate over four buffers and partials over three slot sets: a
+// writer overwrites context t - 2's buffer while building context t + 2 in
+// phase A(t), after it has seen decision t - 2, which the decider gave only
+// after every work CTA had read context t - 2 and stored partials(t - 2) (and
+// had read that context's header itself); a work CTA stores
 // partials(t + 3) after it has seen decision t + 1, behind which the
 // decider reset slot set t.  The decider can run at most one move past a
 // work CTA's read of the word.
@@ -52,6 +53,14 @@ __device__ __forceinline__ unsigned ld_relaxed(const unsigned *p) {
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void st_relaxed(unsigned *p, unsigned v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// integers in the order of finite FP64 values
+__device__ __forceinline__ long long order64(double v) {
+  const long long i = __double_as_longlong(v);
+  return i ^ ((i >> 63) & 0x7fffffffffffffffLL);
+}
 // the outcome of move tt from a word at or past it (at most three moves)
 __device__ __forceinline__ int dec_outcome(unsigned w, int tt) {
   return (int)((w >> ((int)(w >> 4) - (tt + 1))) & 1u);
@@ -64,12 +73,11 @@ __host__ __device__ inline size_t chain_pipe_kvec_doubles(int kc_max) {
   return ((9 * (size_t)kc_max + (kc_max + 1) / 2 + 1) & ~(size_t)1);
 }
 
-// The pair list of a k-chunk CTA: one segment of PSEG entries per warp
-// (its own atoms' pairs, found by a warp-level scan) and one for the
-// previous move's atoms, so that the list needs one CTA barrier and no
-// CTA-wide prefix sum.
+// The pair list of a k-chunk CTA: one segment of PSEG entries per listing
+// warp and one for the previous move's atoms, so that the list needs one CTA
+// barrier and no CTA-wide prefix sum.
 constexpr int PSEG = 64;
-constexpr int PNSEG = CT / 32 + 1;
+constexpr int PNSEG = CT / 32;
 constexpr int ICL_CAP = PSEG * PNSEG;
 
 // Minimum-image wrap of one axis decided on fixed-point turns when a pair
@@ -80,11 +88,9 @@ __device__ __forceinline__ unsigned turn_wrap(const uint32_t *tp, uint4 f) {
   const uint32_t tf[3] = {f.x, f.y, f.z};
   unsigned w = 0;
   for (int d = 0; d < 3; ++d) {
-    const long long dt = (long long)tp[d] - (long long)tf[d];
-    if (dt > 2147483648LL)
-      w |= 1u << (2 * d);
-    else if (dt < -2147483648LL)
-      w |= 2u << (2 * d);
+    const unsigned dt = tp[d] - tf[d];
+    if (tp[d] > tf[d] ? dt > 0x80000000u : -dt > 0x80000000u)
+      w |= (tp[d] > tf[d] ? 1u : 2u) << (2 * d);
   }
   return w;
 }
@@ -93,76 +99,86 @@ __device__ __forceinline__ unsigned turn_wrap(const uint32_t *tp, uint4 f) {
 // instructions (a warp's FP64 instruction holds its SM sub-partition's FP64
 // unit for about 64 cycles on GB300, so their count sets the time of a
 // pass over the pair list): the minimum image from the listed wrap bits
-// (the same FP64 differences: x - L is x + (-L)), the neighbour's charge
-// stored times QQ_FACT, and -- where every kind pair has the 12-6 form --
-// 1 / r^2 by two Newton-Raphson steps from the FP32 reciprocal (relative
-// error below 2^-90 before the final rounding) with sigma^2 / r^2 as a
-// product; the Coulomb cutoff is tested only where it is shorter than the
-// pair cutoff.
+// (the same FP64 differences: x - L is x + (-L)), added only where a lane
+// has one; the neighbour's charge stored times QQ_FACT; comparisons on the
+// bits; degrees 6-8 of the erfc(alpha r)/r segment in FP32 (pair_poly_at);
+// and -- where every kind pair has the 12-6 form -- 1 / r^2 from the FP32
+// reciprocal by one cubic step (relative error below 2^-60 before the final
+// rounding) with sigma^2 / r^2 as a product, for pairs with an epsilon.
 // The force field's pair tables held in shared memory by the chain with two
-// moves in flight: the erfc(alpha r)/r segments (NULL: read from global
-// memory) and the LJ sigma^2 and epsilon C_n of every kind pair.
+// moves in flight: the erfc(alpha r)/r segments in the layout of FF::pair_tab
+// without the force factors (NULL: read from global memory) and the LJ
+// sigma^2 and epsilon C_n of every kind pair.
 struct PairTabs {
   const double *etab;
   const double *sig2, *eps;
 };
 
-// erfc(alpha r) / r as erfc_over_r: the same segment polynomial, its
-// coefficients read from shared memory
+// Terms outside the fast forms (exponents other than 12, r^2 outside the
+// tables), called rather than inlined: the chain's phases stay short enough
+// for the instruction cache.
+__device__ __noinline__ double lj_energy_far(const FF *ff, double s, int idx) {
+  return lj_energy(*ff, s, idx);
+}
+__device__ __noinline__ double erfc_over_r_far(const FF *ff, double s) {
+  return erfc_over_r(*ff, s);
+}
+
+// erfc(alpha r) / r from the segments in shared memory
 __device__ __forceinline__ double erfc_over_r_tab(const FF &ff,
                                                   const double *tab, double s) {
-  const long long bits = __double_as_longlong(s);
+  const long long bits = bits64(s);
   const int seg = (int)(bits >> 46) - ff.etab_key0;
   if (tab == nullptr || (unsigned)seg >= (unsigned)ff.etab_nseg)
-    return erfc_over_r(ff, s);
-  const double a = __longlong_as_double(bits & ~((1LL << 46) - 1));
-  const double scale = __longlong_as_double((2053LL - (bits >> 52)) << 52);
-  const double u = fma(s - a, scale, -1.0);
-  const double *c = tab + (size_t)seg * (ETAB_DEG + 1);
-  double p = c[ETAB_DEG];
-#pragma unroll
-  for (int m = ETAB_DEG - 1; m >= 0; --m)
-    p = fma(p, u, c[m]);
-  return p;
+    return erfc_over_r_far(&ff, s);
+  const double2 *c = (const double2 *)(tab + (size_t)seg * 8);
+  return pair_poly_at(bits, c[0], c[1], c[2], *(const float4 *)(c + 3));
 }
 
 // One pair's terms, signed for the side (new position +, old -): false
-// outside the cutoff.  pzq: the neighbour's z and the pair's charge
-// product q_i q_j QQ_FACT (formed when the pair was listed).
+// outside the cutoff.  a, side: the moved atom and whether its new position;
+// pzq: the neighbour's z and charge times QQ_FACT.
 __device__ __forceinline__ bool pair_energy_pipe(const ChainArgs &A,
-                                                 const double *hdr, int u,
-                                                 double2 pxy, double2 pzq,
-                                                 int mj, unsigned wrap,
+                                                 const double *hdr, int a,
+                                                 int side, double2 pxy,
+                                                 double2 pzq, int mj,
+                                                 unsigned wrap,
                                                  bool lj12, bool coul_cut,
                                                  const PairTabs &pt, double &e,
                                                  double &l, bool &ov) {
   const DevBox &b = A.b;
   const FF &ff = *A.ff;
-  const int a = u / (2 * NB27), side = (u / NB27) % 2;
   const double *pp = hdr + (side ? 48 : 24) + 3 * a;
   double dx = pp[0] - pxy.x, dy = pp[1] - pxy.y, dz = pp[2] - pzq.x;
-  dx += (wrap & 1u) ? -b.L[0] : (wrap & 2u) ? b.L[0] : 0.0;
-  dy += (wrap & 4u) ? -b.L[1] : (wrap & 8u) ? b.L[1] : 0.0;
-  dz += (wrap & 16u) ? -b.L[2] : (wrap & 32u) ? b.L[2] : 0.0;
+  if (wrap & 3u)
+    dx += (wrap & 1u) ? -b.L[0] : b.L[0];
+  if (wrap & 12u)
+    dy += (wrap & 4u) ? -b.L[1] : b.L[1];
+  if (wrap & 48u)
+    dz += (wrap & 16u) ? -b.L[2] : b.L[2];
   const double d2 = dsq3(dx, dy, dz);
-  if (!(ff.rcutSq > d2))
+  if (!gt_pos(ff.rcutSq, d2))
     return false;
-  ov = side && d2 < ff.rcutLowSq;
+  ov = side && gt_pos(ff.rcutLowSq, d2);
   e = 0.0;
-  if (ff.electrostatic && !(coul_cut && ff.rcutCoulSq < d2))
-    e = ff.ewald ? pzq.y * erfc_over_r_tab(ff, pt.etab, d2) : pzq.y / sqrt(d2);
+  if (ff.electrostatic && !(coul_cut && gt_pos(d2, ff.rcutCoulSq))) {
+    const double qq = hdr[108 + a] * pzq.y;
+    e = ff.ewald ? qq * erfc_over_r_tab(ff, pt.etab, d2) : qq / sqrt(d2);
+  }
   const int idx = ((const int *)(hdr + 116))[a] + meta_kind(mj) * ff.n_kinds;
-  if (lj12) {
-    double y = (double)__frcp_rn((float)d2);
-    double r = fma(-d2, y, 1.0);
-    y = fma(y, r, y);
-    r = fma(-d2, y, 1.0);
-    y = fma(y, r, y);
-    const double rRat2 = pt.sig2[idx] * y;
-    const double attract = rRat2 * rRat2 * rRat2;
-    l = pt.eps[idx] * (attract * attract - attract);
+  if (lj12 && in_fast_range(d2)) {
+    l = 0.0;
+    const double eps = pt.eps[idx];
+    if (bits64(eps) != 0) {
+      double y = widen_f64(__frcp_rn(trunc_f32(d2)));
+      const double r = fma(-d2, y, 1.0);
+      y = fma(y, fma(r, r, r), y);
+      const double rRat2 = pt.sig2[idx] * y;
+      const double attract = rRat2 * rRat2 * rRat2;
+      l = eps * fma(attract, attract, -attract);
+    }
   } else {
-    l = lj_energy(ff, d2, idx);
+    l = lj_energy_far(&ff, d2, idx);
   }
   // the old position's terms subtracted: the sign bit flipped (exact)
   const unsigned long long neg = side ? 0ull : 0x8000000000000000ull;
@@ -171,19 +187,43 @@ __device__ __forceinline__ bool pair_energy_pipe(const ChainArgs &A,
   return true;
 }
 
-// pair_energy_pipe added to one set of sums
-__device__ __forceinline__ void pair_term_pipe(const ChainArgs &A,
-                                               const double *hdr, int u,
-                                               double2 pxy, double2 pzq,
-                                               int mj, unsigned wrap,
-                                               bool lj12, bool coul_cut,
-                                               const PairTabs &pt,
-                                               double &lj, double &re,
-                                               double &ovl) {
+// Sums over a warp of four values with six additions a lane instead of
+// twenty: the lanes share the values out as the sums fold.  Lane 0 has v[0],
+// lane 8 v[1], lane 16 v[2], lane 24 v[3].
+__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool h = lane & 16, g = lane & 8;
+  double a = h ? v[2] : v[0], b = h ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, h ? v[1] : v[3], 16);
+  double c = g ? b : a;
+  c += __shfl_xor_sync(0xffffffffu, g ? a : b, 8);
+  for (int o = 4; o > 0; o >>= 1)
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
+// Two values, five additions: lane 0 has x, lane 16 y.
+__device__ __forceinline__ double warp_sum2(double x, double y) {
+  const bool h = threadIdx.x & 16;
+  double a = (h ? y : x) + __shfl_xor_sync(0xffffffffu, h ? x : y, 16);
+  for (int o = 8; o > 0; o >>= 1)
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+
+// pair_energy_pipe added to one set of sums (a pair past a full list)
+__device__ __noinline__ void pair_term_pipe(const ChainArgs &A,
+                                            const double *hdr, int a,
+                                            int side, double2 pxy,
+                                            double2 pzq, int mj,
+                                            unsigned wrap, bool lj12,
+                                            bool coul_cut, const PairTabs &pt,
+                                            double &lj, double &re,
+                                            double &ovl) {
   double e, l;
   bool ov;
-  if (pair_energy_pipe(A, hdr, u, pxy, pzq, mj, wrap, lj12, coul_cut, pt, e, l,
-                       ov)) {
+  if (pair_energy_pipe(A, hdr, a, side, pxy, pzq, mj, wrap, lj12, coul_cut, pt,
+                       e, l, ov)) {
     re += e;
     lj += l;
     if (ov)
@@ -238,7 +278,6 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
     unsigned long long r = x - __umul64hi(x, A.perm_r) * n;
     return (int)(r >= n ? r - n : r);
   };
-  auto perm = [&](int a) { return mod_n((unsigned long long)a * A.perm_m); };
   const int orank = cta - nkb;  // this CTA's rank among the owners
   const int own_per = (b.n_atoms + OWN - 1) / OWN;
   const int on = (!leader && orank >= 0 && orank < b.n_atoms)
@@ -271,10 +310,10 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
                        to_turns(z, b.invL[2]),
                        (unsigned)pack_meta(b.mol[a], b.kind[a]));
   }
-  const bool own_tab = !leader && !kless && ff.erfc_tab != nullptr;
+  const bool own_tab = !leader && !kless && ff.pair_tab != nullptr;
   if (own_tab)
-    for (int i = threadIdx.x; i < ff.etab_nseg * (ETAB_DEG + 1); i += CT)
-      etab_s[i] = ff.erfc_tab[i];
+    for (int i = threadIdx.x; i < ff.etab_nseg * 8; i += CT)
+      etab_s[i] = ff.pair_tab[(i >> 3) * 16 + (i & 7)];
   for (int i = threadIdx.x; i < ff.n_kinds * ff.n_kinds; i += CT) {
     lj_sig2_s[i] = ff.sigmaSq[i];
     lj_eps_s[i] = ff.eps_cn[i];
@@ -367,6 +406,7 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
     bool pend = false;
     int m_prev = -1, acc_prev = 0;
     unsigned hist = 0;  // outcomes of the last moves, newest in bit 0
+    const double nbeta = -ff.beta;
     for (int t = 0; t < A.n; ++t) {
       const int mol_next = nmol;
       nmol = t + 2 < A.n ? A.moves[t + 2].mol : -1;
@@ -381,7 +421,7 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       __syncthreads();
       if (!S.ok)
         return;
-      const double *ctx_t = A.ctx + (size_t)(t % A.nctx) * A.ctx_len;
+      const double *ctx_t = A.ctx + (size_t)(t % PIPE_NCTX) * A.ctx_len;
       for (int i = threadIdx.x; i < HDR; i += CT)
         S.hdr[i] = __ldcg(ctx_t + i);
       __syncthreads();
@@ -392,6 +432,8 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       const bool nspec = t + 1 < A.n && mol_next != m && !bnd &&
                          !(pend && mol_next == m_prev);
       const int var = pend ? acc_prev : 0;  // the partials' outcome set
+      const bool margins = S.hdr[3] > 0.0;
+      const long long hi_o = order64(S.hdr[81]), lo_o = order64(S.hdr[82]);
       double *part_t = A.part + (size_t)(t % 3) * G * 8;
       constexpr int PF = PART_MAX_GRID / 32;
       if (warp < 4) {
@@ -458,10 +500,11 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
           pv[i] = got == 0 ? pp[0][i] : got == 1 ? pp[1][i] : pp[2][i];
         if (ok) {
           if (q < 3) {
-            double v = 0.0;
+            double v = pv[0];
 #pragma unroll
-            for (int i = 0; i < PF; ++i)
-              v += pv[i];
+            for (int i = 1; i < PF; ++i)
+              if (32 * i < W)  // an FP64 addition takes 64 cycles
+                v += pv[i];
             for (int o = 16; o > 0; o >>= 1)
               v += __shfl_down_sync(0xffffffffu, v, o);
             if (lane == 0)
@@ -485,23 +528,27 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
         if (warp == 0 && ok) {
           double dLJ = 0.0, dRe = 0.0, dRc = 0.0;
           if (lane == 0) {
-            bool over = S.tot[3] > 0;
+            const bool over = bits64(S.tot[3]) != 0;
             dLJ = S.tot[0];
             dRe = S.tot[1];
             dRc = (!over && b.K > 0) ? S.tot[2] - S.e_run[2] : 0.0;
-            double ex = __dmul_rn(-ff.beta, __dadd_rn(__dadd_rn(dLJ, dRe), dRc));
+            double ex = __dmul_rn(nbeta, __dadd_rn(__dadd_rn(dLJ, dRe), dRc));
             // pacc < exp(ex), decided on logarithms unless the two sides
-            // are within 1e-9 (or pacc is 0)
+            // are within 1e-9 (or pacc is 0, or ex not finite); compared as
+            // integers of the same order
+            const long long xo = order64(ex);
             int res;
-            if (S.hdr[3] > 0.0 && ex > S.hdr[81])
+            if (margins && xo > hi_o && xo < order64(1.0e300))
               res = 1;
-            else if (S.hdr[3] > 0.0 && ex < S.hdr[82])
+            else if (margins && xo < lo_o && xo > order64(-1.0e300))
               res = 0;
             else
               res = S.hdr[3] < exp(ex);
             acc = res && !over;
             hist = (hist << 1) | (unsigned)acc;
-            st_release(A.seq, dec_word(t, hist));
+            // what the word releases (coordinates, emptied slots) was
+            // fenced at the end of the last move
+            st_relaxed(A.seq, dec_word(t, hist));
           }
           acc = __shfl_sync(0xffffffffu, acc, 0);
           if (prof)
@@ -560,8 +607,12 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       if (!S.ok)
         return;
       const int acc = S.accept;
-      if (threadIdx.x == 0)
+      if (threadIdx.x == 0) {
         settings_update(S.set, (int)S.hdr[1], acc);
+        // releases this CTA's writes with the next word (a release store of
+        // the word itself would wait for them then: 0.45 us of every decision)
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      }
       if (!nspec && t + 1 < A.n) {
         if (!adjust_before(t + 1, bnd))
           return;
@@ -578,48 +629,68 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
     // ---------------- work CTAs ----------------
     // warp 7 gathers the next context's inputs, warp 0 counts its writers
     const bool piper = warp == 7 || warp == 0;
-    CtxPre pipe_a, pipe_b;  // record of t + 2 (a), record and range of t + 1 (b)
-    int pipe_b1 = 0;
-    pipe_a.writer = pipe_b.writer = false;
-    pipe_a.m = pipe_b.m = -1;
+    // records and ranges of moves t + 1 and t + 2, the record of t + 3
+    CtxPre r1, r2, r3;
+    int r1_end = 0, r2_end = 0;
+    r1.writer = r2.writer = r3.writer = false;
+    r1.m = r2.m = r3.m = -1;
+    r1.a0 = r2.a0 = 0;
     if (piper) {
-      ctx_pre_record(A, 1, pipe_b);
-      ctx_pre_range(A, pipe_b, pipe_b1);
-      ctx_pre_record(A, 2, pipe_a);
+      ctx_pre_record(A, 1, r1);
+      ctx_pre_range(A, r1, r1_end);
+      ctx_pre_record(A, 2, r2);
+      ctx_pre_range(A, r2, r2_end);
+      ctx_pre_record(A, 3, r3);
     }
+    int nmol2 = A.n > 2 ? A.moves[2].mol : -1;
+    bool built1 = false;  // this move's successor has its context already
     bool pend = false;  // this move runs before the previous one's decision
-    int m_prev = -1, na_prev = 0, a0_prev = 0;
+    int m_prev = -1, na_prev = 0;
     int mol_cur = A.n > 0 ? A.moves[0].mol : -1;
     bool have_next = false;  // this move's context prefetched into smem
     // three header buffers in turn: this move's (hc), the previous move's
     // while it is undecided (hq), the next move's, prefetched (hn)
-    __shared__ double hbuf[3][HDR];
+    __shared__ __align__(16) double hbuf[3][HDR];
     int hc = 0, hq = 1, hn = 2;
     for (int t = 0; t < A.n; ++t) {
-      const int mol_next = nmol;
-      nmol = t + 2 < A.n ? A.moves[t + 2].mol : -1;
+      const int mol_next = nmol, mol_next2 = nmol2;
+      nmol = nmol2;
+      nmol2 = t + 3 < A.n ? A.moves[t + 3].mol : -1;
       const bool bnd = adj_r == 0;
       adj_r = adj_r + 1 == S.set.adj ? 0 : adj_r + 1;
-      CtxPre pre = pipe_b;
-      pre.na = pipe_b1 - pipe_b.a0;
+      CtxPre pre = r1, pre2 = r2;
+      pre.na = r1_end - r1.a0;
+      pre2.na = r2_end - r2.a0;
       if (piper) {
-        pipe_b = pipe_a;
-        ctx_pre_range(A, pipe_b, pipe_b1);
-        ctx_pre_record(A, t + 3, pipe_a);
+        r1 = r2;
+        r1_end = r2_end;
+        r2 = r3;
+        ctx_pre_range(A, r2, r2_end);
+        ctx_pre_record(A, t + 4, r3);
       }
       // ---------------- phase A ----------------
-      const double *ctx_t = A.ctx + (size_t)(t % A.nctx) * A.ctx_len;
+      const double *ctx_t = A.ctx + (size_t)(t % PIPE_NCTX) * A.ctx_len;
       const int m = mol_cur;
-      // this move's atom range, from the record pipeline of warp 0 (stored
+      // this move's atom count, from the record pipeline of warp 0 (stored
       // during the previous move) but for the first move
-      __shared__ int nx_a0, nx_na;
-      const int a0m = t == 0 ? __ldg(b.mstart + m) : nx_a0;
-      const int na = t == 0 ? __ldg(b.mstart + m + 1) - a0m : nx_na;
+      __shared__ int nx_na;
+      const int na = t == 0 ? __ldg(b.mstart + m + 1) - __ldg(b.mstart + m)
+                            : nx_na;
       // may move t + 1 run before this move's decision
       const bool nspec = t + 1 < A.n && mol_next != m && !bnd &&
                          !(pend && mol_next == m_prev);
-      pre.writer = false;
-      const bool wload = nspec && warp == 7;
+      // A context takes longer to write and reach every CTA than the rest of
+      // a phase (9,200 of 15,900 cycles on 256 waters), so that of move t + 2
+      // is written during this phase where it can be: its molecule is none of
+      // those that move or may have moved meanwhile, and no settings
+      // adjustment precedes it or move t + 1.  Else it is written during
+      // phase A(t + 1), as that of t + 1 is now if it was not yet.
+      const bool early2 = nspec && t + 2 < A.n && adj_r != 0 &&
+                          mol_next2 != m && mol_next2 != mol_next &&
+                          !(pend && mol_next2 == m_prev);
+      const bool late1 = nspec && !built1;
+      pre.writer = pre2.writer = false;
+      const bool wload = late1 && warp == 7, wload2 = early2 && warp == 7;
       const int nbuild = max(1, min(W, b.K > 0 ? 2 * pre.na * 3 : 0));
       double lj = 0.0, re = 0.0, ovl = 0.0, er = 0.0, er2 = 0.0;
       // pair terms of the previous move's atoms this CTA owns, at their
@@ -639,63 +710,70 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       // takes them all.
       __shared__ double2 icl_pos[ICL_CAP][2];
       __shared__ int icl_meta[ICL_CAP];
-      __shared__ short icl_unit[ICL_CAP];
-      // entry class: 0 an own atom that both outcomes of the previous move
-      // share, 1 / 2 an atom of the previous move's molecule at its old
-      // position (that move rejected) / its new one (accepted)
-      __shared__ unsigned char icl_cls[ICL_CAP];
-      __shared__ unsigned char icl_wrap[ICL_CAP];  // turn_wrap of the pair
+      // position (old atoms, then new) | class << 8 | turn_wrap << 16; class 0
+      // an own atom that both outcomes of the previous move share, 1 / 2 an
+      // atom of the previous move's molecule at its old position (that move
+      // rejected) / its new one (accepted)
+      __shared__ int icl_tag[ICL_CAP];
       __shared__ int seg_cnt[PNSEG];  // entries found per segment
       const int npos = 2 * na;
       double *const hd = hbuf[hc];        // this move's header
       const double *const hdrp = hbuf[hq];  // the previous move's
       const uint32_t *pturn = (const uint32_t *)(hd + 84);
-      int n_prev = 0;  // own atoms of the previous molecule (usually 0 or 1)
-      if (pend)
+      // own atoms of the previous molecule (usually 0 or 1)
+      const int2 *const ownp = (const int2 *)(hdrp + 120);
+      int n_prev = 0;
+      if (pend && !kless)
         for (int ap = 0; ap < na_prev; ++ap)
-          n_prev += perm(a0_prev + ap) % OWN == orank;
+          n_prev += ownp[ap].x == orank;
       const int ncomb = n_prev * 2 * npos;
       double *const part_c = A.part + (size_t)(t % 3) * G * 8 + (size_t)cta * 8;
-      // own atom i against this move's positions: bit p set where position
-      // p passes the FP32 pre-test
-      auto pretest = [&](int i, uint4 &f) -> unsigned {
-        unsigned hit = 0;
-        f = ot[i];
-        const int mj = meta_mol((int)f.w);
-        if (mj != m && !(pend && mj == m_prev)) {
-          for (int pp = 0; pp < npos; ++pp) {
-            float dx = (float)(int)(pturn[3 * pp] - f.x) * turn_f[0];
-            float dy = (float)(int)(pturn[3 * pp + 1] - f.y) * turn_f[1];
-            float dz = (float)(int)(pturn[3 * pp + 2] - f.z) * turn_f[2];
-            if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut_f)
-              hit |= 1u << pp;
-          }
+      // Lists, from slot n on and below slot lim, the pairs of 32 own atoms
+      // (one a lane) with this move's positions p0, p0 + step, ...: an FP32
+      // pre-test of them all, then for each position that some lane passes a
+      // ballot that gives the lanes their slots.  Pairs past lim are
+      // evaluated here (not met at liquid densities).  Returns the end of
+      // the entries.
+      auto list_own = [&](int i, bool valid, int p0, int step, int n,
+                          int lim) -> int {
+        uint4 f = make_uint4(0, 0, 0, 0);
+        double2 pxy = make_double2(0.0, 0.0), pzq = pxy;
+        unsigned hit = 0;  // bit p: position p passes the pre-test
+        if (valid) {
+          f = ot[i];
+          pxy = oxy[i];
+          pzq = ozq[i];
+          const int mj = meta_mol((int)f.w);
+          if (mj != m && !(pend && mj == m_prev))
+#pragma unroll 2
+            for (int pp = p0; pp < npos; pp += step) {
+              float dx = (float)(int)(pturn[3 * pp] - f.x) * turn_f[0];
+              float dy = (float)(int)(pturn[3 * pp + 1] - f.y) * turn_f[1];
+              float dz = (float)(int)(pturn[3 * pp + 2] - f.z) * turn_f[2];
+              if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut_f)
+                hit |= 1u << pp;
+            }
         }
-        return hit;
-      };
-      // list own atom i's passing positions from slot pos on, below slot
-      // lim (past it: evaluated here, not met at liquid densities)
-      auto list_hits = [&](int i, unsigned hit, uint4 f, int pos, int lim) {
-        const double2 pxy = oxy[i], oq = ozq[i];
-        for (unsigned h = hit; h; h &= h - 1) {
-          const int pp = __ffs(h) - 1;
-          const int side = pp >= na ? 1 : 0, a = pp - side * na;
-          const int u = (a * 2 + side) * NB27;
-          const double2 pzq = make_double2(oq.x, hd[108 + a] * oq.y);
+        for (unsigned any = __reduce_or_sync(0xffffffffu, hit); any;
+             any &= any - 1) {
+          const int pp = __ffs(any) - 1;
+          const bool mine = hit >> pp & 1;
+          const unsigned mask = __ballot_sync(0xffffffffu, mine);
+          const int pos = n + __popc(mask & ((1u << lane) - 1));
+          n += __popc(mask);
           const unsigned wr = turn_wrap(pturn + 3 * pp, f);
-          if (pos < lim) {
+          if (mine && pos < lim) {
             icl_pos[pos][0] = pxy;
             icl_pos[pos][1] = pzq;
             icl_meta[pos] = (int)f.w;
-            icl_unit[pos] = (short)u;
-            icl_cls[pos] = 0;
-            icl_wrap[pos] = (unsigned char)wr;
-          } else {
-            pair_term_pipe(A, hd, u, pxy, pzq, (int)f.w, wr, lj12, coul_cut, ptab,
-                           lj, re, ovl);
+            icl_tag[pos] = pp | (int)wr << 16;
+          } else if (mine) {
+            const int side = pp >= na;
+            pair_term_pipe(A, hd, pp - side * na, side, pxy, pzq, (int)f.w, wr,
+                           lj12, coul_cut, ptab, lj, re, ovl);
           }
-          ++pos;
         }
+        return n;
       };
       // The previous move's atoms this CTA owns on both outcomes (entries
       // c = (atom, outcome, position)), pre-tested like the others and
@@ -714,10 +792,8 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
             const int r = c - ap * 2 * npos;
             vr = r / npos;
             pp = r - vr * npos;
-            const int ga = a0_prev + ap;
-            const int pg = perm(ga);
-            if (pg % OWN == orank) {
-              i = pg / OWN;
+            if (ownp[ap].x == orank) {
+              i = ownp[ap].y;
               f = ot[i];
               if (vr) {
                 const uint32_t *nt = (const uint32_t *)(hdrp + 84) + (na_prev + ap) * 3;
@@ -735,28 +811,22 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
           if (hit) {
             const int pos = n + __popc(mask & ((1u << lane) - 1));
             const int side = pp >= na ? 1 : 0, a = pp - side * na;
-            const int u = (a * 2 + side) * NB27;
             double2 pxy = oxy[i], pzq = ozq[i];
             if (vr) {
               const double *np = hdrp + 48 + 3 * ap;
               pxy = make_double2(np[0], np[1]);
               pzq.x = np[2];
             }
-            pzq.y *= hd[108 + a];  // q_i q_j QQ_FACT
             const unsigned wr = turn_wrap(pturn + 3 * pp, f);
             if (pos < lim) {
               icl_pos[pos][0] = pxy;
               icl_pos[pos][1] = pzq;
               icl_meta[pos] = (int)f.w;
-              icl_unit[pos] = (short)u;
-              icl_cls[pos] = (unsigned char)(1 + vr);
-              icl_wrap[pos] = (unsigned char)wr;
-            } else if (vr) {
-              pair_term_pipe(A, hd, u, pxy, pzq, (int)f.w, wr, lj12, coul_cut,
-                             ptab, ljA, reA, ovA);
+              icl_tag[pos] = pp | (1 + vr) << 8 | (int)wr << 16;
             } else {
-              pair_term_pipe(A, hd, u, pxy, pzq, (int)f.w, wr, lj12, coul_cut,
-                             ptab, ljR, reR, ovR);
+              pair_term_pipe(A, hd, a, side, pxy, pzq, (int)f.w, wr, lj12,
+                             coul_cut, ptab, vr ? ljA : ljR, vr ? reA : reR,
+                             vr ? ovA : ovR);
             }
           }
           n += __popc(mask);
@@ -764,85 +834,62 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
         return n;
       };
       // the listed pairs, by the lanes of one warp, each added to its
-      // class's sums; the previous move's pairs past a full list directly
-      // (entries first * 32 + lane, stepping step * 32: the passes of 32
-      // entries split between two warps when the list is longer than one)
-      // (entry v of the list: slot v, or with segments the v-th listed
-      // entry counting through the segments in order)
-      auto eval_pairs = [&](int n_eval, int first, int step, bool segs) {
-        for (int v = first * 32 + lane; v < n_eval; v += step * 32) {
-          int i = v;
-          if (segs) {
-            int r = v;
-            for (int sg = 0; sg < PNSEG; ++sg) {
-              const int c = min(seg_cnt[sg], PSEG);
-              if (r < c) {
-                i = sg * PSEG + r;
-                break;
-              }
-              r -= c;
+      // class's sums (the v-th listed entry counting through the segments
+      // in order)
+      double psum[4];  // LJ and real space, previous move rejected, accepted
+      bool ov0, ov1;
+      auto eval_pairs = [&](int n_eval, int nseg) {
+        psum[0] = psum[1] = psum[2] = psum[3] = 0.0;
+        ov0 = ov1 = false;
+        for (int v = lane; v < n_eval; v += 32) {
+          int i = v, before = 0;
+#pragma unroll
+          for (int sg = 0; sg < PNSEG; ++sg)
+            if (sg < nseg) {
+              if (v >= before)
+                i = sg * PSEG + v - before;
+              before += min(seg_cnt[sg], PSEG);
             }
-          }
           double e, l;
           bool o;
-          if (!pair_energy_pipe(A, hd, icl_unit[i], icl_pos[i][0],
-                                icl_pos[i][1], icl_meta[i], icl_wrap[i], lj12,
-                                coul_cut, ptab, e, l, o))
+          const int tag = icl_tag[i], pp = tag & 255, side = pp >= na;
+          if (!pair_energy_pipe(A, hd, pp - side * na, side, icl_pos[i][0],
+                                icl_pos[i][1], icl_meta[i], (unsigned)tag >> 16,
+                                lj12, coul_cut, ptab, e, l, o))
             continue;
-          const int c = icl_cls[i];
-          if (c == 0) {
-            lj += l;
-            re += e;
-            if (o)
-              ovl = 1.0;
-          } else if (c == 1) {
-            ljR += l;
-            reR += e;
-            if (o)
-              ovR = 1.0;
+          const int c = tag >> 8 & 255;
+          const double t4[4] = {c == 2 ? 0.0 : l, c == 2 ? 0.0 : e,
+                                c == 1 ? 0.0 : l, c == 1 ? 0.0 : e};
+          ov0 |= o && c != 2;
+          ov1 |= o && c != 1;
+          if (v == lane) {  // a lane's first pair: no additions
+            for (int j = 0; j < 4; ++j)
+              psum[j] = t4[j];
           } else {
-            ljA += l;
-            reA += e;
-            if (o)
-              ovA = 1.0;
+            for (int j = 0; j < 4; ++j)
+              psum[j] += t4[j];
           }
         }
       };
-      // the pair partials of the warp that evaluated this CTA's pairs (with
-      // the second pair warp's sums from shared memory, when the passes were
-      // split): warp sums (both outcomes), stored by lane 0
-      __shared__ double pair2[4];
-      __shared__ int pair2_ov[2];
-      auto store_pairs_warp = [&](bool split) {
-        double v[4] = {lj + ljR, re + reR, lj + ljA, re + reA};
-        if (ncomb > 0 || split) {  // (the outcomes may differ)
-          for (int o = 16; o > 0; o >>= 1)
-            for (int j = 0; j < 4; ++j)
-              v[j] += __shfl_down_sync(0xffffffffu, v[j], o);
+      // the pair partials of the warp that evaluated this CTA's pairs: warp
+      // sums on both outcomes, into slots 0, 1 and 4, 5
+      auto store_pairs_warp = [&]() {
+        const bool any0 = __any_sync(0xffffffffu, ov0),
+                   any1 = __any_sync(0xffffffffu, ov1);
+        if (ncomb > 0) {
+          const double v = warp_sum4(psum);
+          if ((lane & 7) == 0)
+            __stcg(part_c + (lane >> 3 & 1) + 4 * (lane >> 4), v);
         } else {
           // both outcomes share every pair of this CTA
-          for (int o = 16; o > 0; o >>= 1)
-            for (int j = 0; j < 2; ++j)
-              v[j] += __shfl_down_sync(0xffffffffu, v[j], o);
-          v[2] = v[0];
-          v[3] = v[1];
-        }
-        bool any0 = __any_sync(0xffffffffu, ovl > 0.0 || ovR > 0.0);
-        bool any1 = __any_sync(0xffffffffu, ovl > 0.0 || ovA > 0.0);
-        if (split) {
-          // the second pair warp's sums (named barrier 5: the two warps)
-          asm volatile("bar.sync 5, 64;" ::: "memory");
-          for (int j = 0; j < 4; ++j)
-            v[j] += pair2[j];
-          any0 = any0 || pair2_ov[0];
-          any1 = any1 || pair2_ov[1];
+          const double v = warp_sum2(psum[0], psum[1]);
+          if ((lane & 15) == 0) {
+            __stcg(part_c + (lane >> 4), v);
+            __stcg(part_c + 4 + (lane >> 4), v);
+          }
         }
         if (lane == 0) {
-          __stcg(part_c + 0, v[0]);
-          __stcg(part_c + 1, v[1]);
           __stcg(part_c + 3, any0 ? 1.0 : 0.0);
-          __stcg(part_c + 4, v[2]);
-          __stcg(part_c + 5, v[3]);
           __stcg(part_c + 7, any1 ? 1.0 : 0.0);
         }
       };
@@ -855,109 +902,112 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       // `want`; S.ok false when a wait gave up.
       const int want = nspec ? (pend ? t - 1 : -1) : t;
       auto poll_warp = [&]() {
-        unsigned it = 0, w = 0;
+        unsigned w = 0;
         int ok = 1;
-        // relaxed loads while polling (an acquire load may invalidate the
-        // SM's L1, which the pair terms beside this warp read their tables
-        // through), one acquire fence once everything is seen
-        for (;;) {
-          bool mine = true;
-          if (nspec)
+        // the flags by relaxed loads and one fence once all are seen; the
+        // word, which the CTA waits for, by acquire loads (a fence after it
+        // came would cost about as long as a load)
+        auto wait_for = [&](auto seen) {
+          for (unsigned it = 0; ok;) {
+            if (__all_sync(0xffffffffu, seen()))
+              break;
+            int bad = 0;
+            if (lane == 0) {
+              if (++it > A.spin) {
+                atomicOr(b.err, DERR_BARRIER_TIMEOUT);
+                bad = 1;
+              } else if ((it & 255u) == 0 && *(volatile int *)b.err) {
+                bad = 1;
+              }
+            }
+            if (__shfl_sync(0xffffffffu, bad, 0))
+              ok = 0;
+            __nanosleep(32);
+          }
+        };
+        if (nspec) {
+          wait_for([&]() {
+            bool mine = true;
             for (int c = lane; c < nbuild; c += 32)
               mine &= (int)(ld_relaxed(A.seq + SEQ_CTX + c) - (unsigned)(t + 1)) >= 0;
-          if (lane == 0 && want >= 0) {
-            w = ld_relaxed(A.seq);
-            mine &= (int)(w >> 4) >= want + 1;
-          }
-          if (__all_sync(0xffffffffu, mine)) {
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            break;
-          }
-          int bad = 0;
-          if (lane == 0) {
-            if (++it > A.spin) {
-              atomicOr(b.err, DERR_BARRIER_TIMEOUT);
-              bad = 1;
-            } else if ((it & 255u) == 0 && *(volatile int *)b.err) {
-              bad = 1;
+            return mine;
+          });
+          asm volatile("fence.acq_rel.gpu;" ::: "memory");
+          if (ok && !kless) {
+            // the next context is complete: its header and phase rows into
+            // shared memory now, off the next phase A's path, eight loads in
+            // flight a lane
+            const double2 *src =
+                (const double2 *)(A.ctx + (size_t)((t + 1) % PIPE_NCTX) * A.ctx_len);
+            double2 *tabn = tab == tab0 ? tab1 : tab0;
+            double2 *hn2 = (double2 *)hbuf[hn];
+            const int nh = HDR / 2, n = nh + A.nrows_max * stride;
+            for (int i0 = lane; i0 < n; i0 += 8 * 32) {
+              double2 v[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (i0 + 32 * j < n)
+                  v[j] = __ldcg(src + i0 + 32 * j);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const int i = i0 + 32 * j;
+                if (i < nh)
+                  hn2[i] = v[j];
+                else if (i < n)
+                  tabn[i - nh] = v[j];
+              }
             }
           }
-          if (__shfl_sync(0xffffffffu, bad, 0)) {
-            ok = 0;
-            break;
-          }
-          __nanosleep(32);
         }
+        if (want >= 0)
+          wait_for([&]() {
+            if (lane == 0)
+              w = ld_acquire(A.seq);
+            return lane != 0 || (int)(w >> 4) >= want + 1;
+          });
         if (lane == 0) {
           S.ok = ok && *(volatile int *)b.err == 0;
           S.word = w;
         }
-        if (ok && nspec && !kless) {
-          // the next context is complete (its writers' flags were seen):
-          // its header and phase rows into shared memory now, off the
-          // next phase A's path
-          const double *ctx_n = A.ctx + (size_t)((t + 1) % A.nctx) * A.ctx_len;
-          double2 *tabn = tab == tab0 ? tab1 : tab0;
-          for (int i = lane; i < HDR; i += 32)
-            hbuf[hn][i] = __ldcg(ctx_n + i);
-          for (int i = lane; i < A.nrows_max * stride; i += 32)
-            tabn[i] = __ldcg((const double2 *)(ctx_n + HDR) + i);
-        }
       };
 
       if (kless) {
-        // A context writer without k-vectors.  Warp 0 takes this move's
-        // header, lists its own atoms (a warp-level scan), evaluates the
-        // pairs and stores the partials; warps 1..7 build their part of the
-        // next move's context meanwhile, from the start of the phase (it
-        // does not depend on this move's header).
+        // A context writer without k-vectors and atoms.  Warp 0 takes this
+        // move's header and stores empty partials; warps 1..7 write their
+        // part of a coming move's context meanwhile, from the start of the
+        // phase (it does not depend on this move's header).
         if (warp == 0) {
           for (int i = lane; i < HDR; i += 32)
             hd[i] = __ldcg(ctx_t + i);
           __syncwarp();
           mark(0);
-          int icl_n = 0;
-          for (int base = 0; base < on; base += 32) {
-            const int i = base + lane;
-            uint4 f = make_uint4(0, 0, 0, 0);
-            const unsigned hit = i < on ? pretest(i, f) : 0u;
-            const int cnt = __popc(hit);
-            int incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-              int v = __shfl_up_sync(0xffffffffu, incl, o);
-              if (lane >= o)
-                incl += v;
-            }
-            if (hit)
-              list_hits(i, hit, f, icl_n + incl - cnt, ICL_CAP);
-            icl_n += __shfl_sync(0xffffffffu, incl, 31);
-          }
-          __syncwarp();
-          if (ncomb > 0)
-            icl_n = list_prev(icl_n, ICL_CAP);
-          __syncwarp();
           mark(1);
-          eval_pairs(min(icl_n, ICL_CAP), 0, 1, false);
-          store_pairs_warp(false);
-          if (lane == 0) {
-            __stcg(part_c + 2, 0.0);
-            __stcg(part_c + 6, 0.0);
-          }
+          if (lane < 8)  // no k-vectors and no atoms: nothing to add
+            __stcg(part_c + lane, 0.0);
           poll_warp();
         } else if (nspec) {
-          if (warp == 7) {
-            ctx_pre2(A, S, t + 1, pre);
-            if (pre.writer)
-              ctx_pre_store(S, pre);
-            if (lane == 0)
-              S.b_writer = pre.writer;
-          }
-          group_sync(CT - 32);
-          if (S.b_writer) {
-            build_ctx_rest(A, S, t + 1, (int)threadIdx.x - 32, CT - 32);
+          auto build = [&](int s, CtxPre &c) {
+            if (warp == 7) {
+              ctx_pre2(A, S, s, c);
+              if (c.writer)
+                ctx_pre_store(S, c);
+              if (lane == 0)
+                S.b_writer = c.writer;
+            }
             group_sync(CT - 32);
-            if (threadIdx.x == 32)
-              st_release(A.seq + SEQ_CTX + blockIdx.x, (unsigned)(t + 1));
+            if (S.b_writer) {
+              build_ctx_rest(A, S, s, (int)threadIdx.x - 32, CT - 32);
+              group_sync(CT - 32);
+              if (threadIdx.x == 32)
+                st_release(A.seq + SEQ_CTX + blockIdx.x, (unsigned)s);
+            }
+          };
+          if (late1)
+            build(t + 1, pre);
+          if (early2) {
+            if (late1)
+              group_sync(CT - 32);  // S.b_* read before they change
+            build(t + 2, pre2);
           }
         }
         __syncthreads();
@@ -982,32 +1032,28 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
         mark(0);
         if (wload)
           ctx_pre2(A, S, t + 1, pre);
-        // each warp lists its atoms' pairs into its own segment; warp 0
-        // the previous move's atoms into the last
-        int n_w = 0;
-        for (int base = 0; base < on; base += CT) {
-          const int i = base + threadIdx.x;
-          uint4 f = make_uint4(0, 0, 0, 0);
-          const unsigned hit = i < on ? pretest(i, f) : 0u;
-          const int cnt = __popc(hit);
-          int incl = cnt;
-          for (int o = 1; o < 32; o <<= 1) {
-            int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o)
-              incl += v;
+        else if (wload2)
+          ctx_pre2(A, S, t + 2, pre2);
+        // warps 0-6 list the pairs of 32 own atoms at a time with all
+        // positions (with a share of them where there are fewer such blocks
+        // than warps), each into its own segment; warp 7 forms the x-y
+        // column products and lists the previous move's atoms into the last
+        if (warp < 7) {
+          int n = warp * PSEG;
+          const int nb = (on + 31) / 32;
+          const int share = nb > 3 ? 1 : min(npos, 7 / max(nb, 1));
+          for (int u = warp; u < nb * share; u += 7) {
+            const int p0 = share > 1 ? u / nb : 0, i = (u - p0 * nb) * 32 + lane;
+            n = list_own(i, i < on, p0, share, n, (warp + 1) * PSEG);
           }
-          if (hit)
-            list_hits(i, hit, f, warp * PSEG + n_w + incl - cnt,
-                      (warp + 1) * PSEG);
-          n_w += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0)
-          seg_cnt[warp] = n_w;
-        if (warp == 0) {
-          const int b0 = (PNSEG - 1) * PSEG;
+          if (lane == 0)
+            seg_cnt[warp] = n - warp * PSEG;
+        } else {
+          xy_products(lane, 32, npair, pair_n, tab, stride, na, hd + 72, exy);
+          const int b0 = 7 * PSEG;
           const int n = ncomb > 0 ? list_prev(b0, ICL_CAP) - b0 : 0;
           if (lane == 0)
-            seg_cnt[PNSEG - 1] = n;
+            seg_cnt[7] = n;
         }
         __syncthreads();  // the listed pairs
         mark(1);
@@ -1019,28 +1065,30 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
           n_eval += min(seg_cnt[sg], PSEG);
           all_pairs |= seg_cnt[sg] > PSEG;
         }
-        // A list longer than one warp pass: warp 4 (another sub-partition)
-        // takes every second pass after its k-vectors, instead of warp 3
-        // taking them all in sequence.
-        const bool split = n_eval > 32 && !all_pairs;
         if (warp == pw) {
-          eval_pairs(n_eval, 0, split ? 2 : 1, true);
+          eval_pairs(n_eval, PNSEG);
           if (!all_pairs)
-            store_pairs_warp(split);
+            store_pairs_warp();
         } else if (warp == 7) {
           if (wload && pre.writer) {
             ctx_pre_store(S, pre);
             __syncwarp();
             build_ctx_warp(A, S, t + 1);
           }
+          if (wload2) {
+            if (wload)
+              ctx_pre2(A, S, t + 2, pre2);
+            if (pre2.writer) {
+              __syncwarp();
+              ctx_pre_store(S, pre2);
+              __syncwarp();
+              build_ctx_warp(A, S, t + 2);
+            }
+          }
           if (!all_pairs)
             poll_warp();
         } else {
           const int kw = warp < 3 ? warp : warp - 1;  // 0..5
-          // the x-y column products first (named barrier 4: the six warps)
-          xy_products(kw * 32 + lane, 6 * 32, npair, pair_n, tab, stride, na,
-                      hd + 72, exy);
-          asm volatile("bar.sync 4, 192;" ::: "memory");
           const double *sR = KR(bS), *sI = KI(bS);
           const double *pR = pend ? KR(bP) : nullptr;
           const double *pI = pend ? KI(bP) : nullptr;
@@ -1063,53 +1111,38 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
           }
           // the reciprocal energy of the chunk on both outcomes: warp sums,
           // then the six warps in order (named barrier 4)
-          for (int o = 16; o > 0; o >>= 1) {
-            er += __shfl_down_sync(0xffffffffu, er, o);
-            er2 += __shfl_down_sync(0xffffffffu, er2, o);
-          }
-          if (lane == 0) {
-            red6[2][warp] = er;
-            red6[5][warp] = er2;
-          }
+          const double ew = warp_sum2(er, er2);
+          if ((lane & 15) == 0)
+            red6[lane ? 5 : 2][warp] = ew;
           asm volatile("bar.sync 4, 192;" ::: "memory");
-          if (threadIdx.x == 0) {
-            double r0 = 0.0, r1 = 0.0;
-            for (int w = 0; w < CT / 32; ++w)
-              if (w != 3 && w != 7) {
-                r0 += red6[2][w];
-                r1 += red6[5][w];
-              }
-            __stcg(part_c + 2, r0);
-            __stcg(part_c + 6, pend ? r1 : r0);
-          }
-          if (split && warp == 4) {
-            // the second pair warp: its passes, summed, to warp 3
-            lj = re = ovl = ljR = reR = ovR = ljA = reA = ovA = 0.0;
-            eval_pairs(n_eval, 1, 2, true);
-            double v[4] = {lj + ljR, re + reR, lj + ljA, re + reA};
-            for (int o = 16; o > 0; o >>= 1)
-              for (int j = 0; j < 4; ++j)
-                v[j] += __shfl_down_sync(0xffffffffu, v[j], o);
-            const bool any0 = __any_sync(0xffffffffu, ovl > 0.0 || ovR > 0.0);
-            const bool any1 = __any_sync(0xffffffffu, ovl > 0.0 || ovA > 0.0);
+          if (warp == 0) {
+            // lanes 0-7 the six warps' er, lanes 8-15 their er2
+            const int w = lane & 7;
+            double r = lane < 16 && w != 3 && w != 7 ? red6[lane < 8 ? 2 : 5][w] : 0.0;
+            for (int o = 4; o > 0; o >>= 1)
+              r += __shfl_xor_sync(0xffffffffu, r, o);
             if (lane == 0) {
-              for (int j = 0; j < 4; ++j)
-                pair2[j] = v[j];
-              pair2_ov[0] = any0;
-              pair2_ov[1] = any1;
+              __stcg(part_c + 2, r);
+              if (!pend)
+                __stcg(part_c + 6, r);
+            } else if (lane == 8 && pend) {
+              __stcg(part_c + 6, r);
             }
-            asm volatile("bar.sync 5, 64;" ::: "memory");
           }
         }
         if (all_pairs) {
           // pairs past the list were evaluated by every warp: the CTA's
           // pair sums over all warps, in warp order
           double v[4] = {lj + ljR, re + reR, lj + ljA, re + reA};
+          if (warp == pw)
+            for (int j = 0; j < 4; ++j)
+              v[j] += psum[j];
           for (int o = 16; o > 0; o >>= 1)
             for (int j = 0; j < 4; ++j)
               v[j] += __shfl_down_sync(0xffffffffu, v[j], o);
-          const int any0 = __syncthreads_or(ovl > 0.0 || ovR > 0.0);
-          const int any1 = __syncthreads_or(ovl > 0.0 || ovA > 0.0);
+          const bool mine = warp == pw;
+          const int any0 = __syncthreads_or(ovl > 0.0 || ovR > 0.0 || (mine && ov0));
+          const int any1 = __syncthreads_or(ovl > 0.0 || ovA > 0.0 || (mine && ov1));
           if (lane == 0) {
             red6[0][warp] = v[0];
             red6[1][warp] = v[1];
@@ -1137,7 +1170,7 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       // ---------------- phase B ----------------
       // an accepted move (hd: its header): its new positions for the next
       // contexts, and the moved atoms this CTA owns take them
-      auto commit_atoms = [&](const double *hd, int nn, int a0) {
+      auto commit_atoms = [&](const double *hd, int nn) {
         for (int i = threadIdx.x; i < 3 * nn + 3; i += CT) {
           if (i < 3 * nn)
             S.last_newp[i / 3][i % 3] = hd[48 + i];
@@ -1145,8 +1178,9 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
             S.last_newcom[i - 3 * nn] = hd[4 + i - 3 * nn];
         }
         for (int a = threadIdx.x; a < nn; a += CT) {
-          const int pg = perm(a0 + a), i = pg / OWN;
-          if (pg - i * OWN == orank) {
+          const int2 ow = ((const int2 *)(hd + 120))[a];
+          if (ow.x == orank) {
+            const int i = ow.y;
             const double *np = hd + 48 + 3 * a;
             const uint32_t *pt = (const uint32_t *)(hd + 84) + (nn + a) * 3;
             oxy[i] = make_double2(np[0], np[1]);
@@ -1158,10 +1192,8 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       if (!S.ok)
         return;
       const unsigned word = S.word;
-      if (threadIdx.x == 0) {  // the next move's range (read after a barrier)
-        nx_a0 = pre.a0;
+      if (threadIdx.x == 0)  // the next move's count (read after a barrier)
         nx_na = pre.na;
-      }
       if (pend) {
         const int acc_p = dec_outcome(word, t - 1);
         if (threadIdx.x == 0) {
@@ -1170,7 +1202,7 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
           S.last_acc = acc_p;
         }
         if (acc_p) {
-          commit_atoms(hdrp, na_prev, a0_prev);
+          commit_atoms(hdrp, na_prev);
           bS = bP;  // the previous move's new sums are committed
           bP = bA;  // and this move's new sums on that outcome pend
         } else {
@@ -1184,7 +1216,6 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       if (nspec) {
         m_prev = m;
         na_prev = na;
-        a0_prev = a0m;
         pend = true;
         have_next = !kless;
         __syncthreads();
@@ -1199,7 +1230,7 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
           S.last_acc = acc;
         }
         if (acc) {
-          commit_atoms(hd, na, a0m);
+          commit_atoms(hd, na);
           bS = bP;
         }
         bP = -1;
@@ -1216,6 +1247,7 @@ __global__ void __launch_bounds__(CT, 1) k_chain_fp64_pipe(ChainArgs A) {
       }
       mark(4);
       mol_cur = mol_next;
+      built1 = early2;
       // the headers' roles: this move's becomes the previous one's, the
       // prefetched one (or a free buffer) this move's
       const int hfree = hq;

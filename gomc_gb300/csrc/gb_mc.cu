@@ -376,6 +376,7 @@ __device__ __forceinline__ double2 tab_at(const double2 *row, int n) {
 // The FP64 chain kernel
 // ===========================================================================
 constexpr int CT = 256;
+constexpr int PIPE_NCTX = 4;  // context buffers with two moves in flight
 constexpr int HDR = 128;  // doubles in the move-context header
 constexpr int ICL_MAX = 256;  // in-cutoff pairs a CTA lists per move
 // Words of the chain's flag array: [0] the decision word, alone on its
@@ -407,7 +408,9 @@ __host__ __device__ constexpr size_t chain_ctx_len(int stride) {
 //  0 m, 1 kind, 2 na, 3 pacc, 4..6 newcom, 8..15 cell old, 16..23 cell new,
 //  24..47 old positions [8][3], 48..71 new positions [8][3], 72..79 charges,
 //  80 log(pacc), 81 log(pacc) + 1e-9, 82 log(pacc) - 1e-9,
-//  84..107 fixed-point turns of the positions as uint32 [side][atom][3]
+//  84..107 fixed-point turns of the positions as uint32 [side][atom][3],
+//  108..115 charges, 116..119 kinds (int), 120..127 with atoms spread over
+//  owners (two moves in flight) each atom's owner and index there (int)
 struct ChainArgs {
   DevBox b;
   const FF *ff;
@@ -423,7 +426,8 @@ struct ChainArgs {
                   // written (t)
   double *ctx;    // [nctx][ctx_len], by move modulo nctx: HDR + tables
   size_t ctx_len;
-  int nctx;       // context buffers: 2 (one move in flight) or 3 (two)
+  int nctx;       // context buffers: 2 (one move in flight) or PIPE_NCTX
+  int own;        // owners of the atoms (two moves in flight), else 0
   int nrows_max;  // phase rows of the largest molecule (6 x its atoms)
   int nkless;     // CTAs 0 .. nkless - 1 hold no k-vectors (context writers)
   // permutation of the atom index for the pipelined chain's atom ownership
@@ -470,6 +474,16 @@ __device__ __forceinline__ void group_sync(int count) {
     __syncthreads();
   else
     asm volatile("bar.sync 1, %0;" ::"r"(count) : "memory");
+}
+
+// The owner of atom a and its index there, through the multiplicative
+// permutation of the atom index (x mod n_atoms by Barrett reduction).
+__device__ __forceinline__ int2 chain_owner(const ChainArgs &A, int a) {
+  const unsigned long long n = (unsigned long long)A.b.n_atoms;
+  const unsigned long long x = (unsigned long long)a * A.perm_m;
+  unsigned long long r = x - __umul64hi(x, A.perm_r) * n;
+  const int p = (int)(r >= n ? r - n : r);
+  return make_int2(p % A.own, p / A.own);
 }
 
 // Is this CTA one of the writers of a move's context: CTA 0 (header) and
@@ -544,6 +558,8 @@ __device__ void build_ctx_rest(const ChainArgs &A, ChainShared &S, int t,
         h[72 + a] = fabs(q) < 0.000000001 ? 0.0 : q;
         h[108 + a] = q;  // the charge and kind of the real-space terms
         ((int *)(h + 116))[a] = S.b_ka[a];
+        if (A.own)
+          ((int2 *)(h + 120))[a] = chain_owner(A, S.b_a0 + a);
       }
     } else if (tid >= 128 && tid < 128 + 6 * na) {
       int i = tid - 128, pa = i / 3, d = i % 3;  // pa = side * na + atom
@@ -631,6 +647,8 @@ __device__ void build_ctx_warp(const ChainArgs &A, ChainShared &S, int t) {
         h[72 + a] = fabs(q) < 0.000000001 ? 0.0 : q;
         h[108 + a] = q;  // the charge and kind of the real-space terms
         ((int *)(h + 116))[a] = S.b_ka[a];
+        if (A.own)
+          ((int2 *)(h + 120))[a] = chain_owner(A, S.b_a0 + a);
       }
     }
     for (int i = lane; i < 6 * na; i += 32) {
@@ -1949,8 +1967,7 @@ static size_t chain_smem(const Box &b, int grid, int nrows_max,
          sizeof(unsigned short) * (size_t)kc_max + 64 +
          own_per * (2 * sizeof(double2) + sizeof(uint4)) +
          // (the pipelined chain's copy of the erfc(alpha r)/r segments)
-         (pipe && b.ff.erfc_tab ? sizeof(double) * (size_t)b.ff.etab_nseg *
-                                      (ETAB_DEG + 1)
+         (pipe && b.ff.pair_tab ? sizeof(double) * (size_t)b.ff.etab_nseg * 8
                                 : 0);
 }
 
@@ -2044,7 +2061,7 @@ int mc_init(Box &b, const gb_mc_params &p) {
       (rc = mc_alloc(b, s, &s.d_part, 3 * (size_t)s.grid * 8)) ||
       (rc = mc_alloc(b, s, &s.d_bar, 8)) ||
       (rc = mc_alloc(b, s, &s.d_seq, SEQ_CTX + PART_MAX_GRID)) ||
-      (rc = mc_alloc(b, s, &s.d_ctx, 3 * chain_ctx_len(stride))) ||
+      (rc = mc_alloc(b, s, &s.d_ctx, PIPE_NCTX * chain_ctx_len(stride))) ||
       (rc = mc_alloc(b, s, &s.d_mp, 16)))
     return rc;
   if ((rc = b.CudaCheck(cudaMallocHost(&s.h_moves, s.move_cap * sizeof(MoveRec)),
@@ -2324,7 +2341,8 @@ static int run_chain(Box &b, McState &s, const MoveRec *moves, int64_t first,
   A.nrows_max = b.dev.K > 0 ? 6 * s.na_max : 0;
   A.nkless = chain_kless(A.nrows_max, s.pipe ? s.grid - 1 : s.grid,
                          s.params.writer_kchunk != 0);
-  A.nctx = s.pipe ? 3 : 2;
+  A.nctx = s.pipe ? PIPE_NCTX : 2;
+  A.own = s.pipe ? s.grid - 1 - A.nkless : 0;
   chain_perm(b.dev.n_atoms, &A.perm_m, &A.perm_minv);
   A.perm_r = ~0ULL / (unsigned long long)std::max(b.dev.n_atoms, 1);
   A.tr_i = tr_i;

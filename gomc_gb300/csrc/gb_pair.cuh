@@ -97,6 +97,79 @@ __device__ __forceinline__ double coulomb_virial(const FF &ff, double distSq,
   return qq / (distSq * dist);
 }
 
+// ---- FP64 work moved to the integer and FP32 pipes ----
+// GB300 retires two FP64 lanes per SM and clock, 64 times fewer than FP32 or
+// integer ones; comparisons and conversions are FP64 instructions too.
+__device__ __forceinline__ long long bits64(double v) {
+  return __double_as_longlong(v);
+}
+// a > b of two non-negative values (NaN above all), on the integer pipe
+__device__ __forceinline__ bool gt_pos(double a, double b) {
+  return bits64(a) > bits64(b);
+}
+
+// FP32 value of a positive FP64 number in FP32's normal range, truncated, and
+// the exact FP64 value of a normal FP32 one, by moving bits: the conversion
+// instructions run at the FP64 rate.
+__device__ __forceinline__ float trunc_f32(double v) {
+  const long long b = bits64(v);
+  return __int_as_float((int)(b >> 29) - (896 << 23));
+}
+__device__ __forceinline__ double widen_f64(float f) {
+  const int b = __float_as_int(f);
+  const int hi = (b & 0x80000000) | (((b & 0x7fffffff) >> 3) + (896 << 20));
+  return __hiloint2double(hi, b << 29);
+}
+
+// 1 / s to the last bit or two, s positive and well inside FP32's range: the
+// FP32 reciprocal (relative error e below 2^-21), one cubic step (e^3) and a
+// final correction.
+__device__ __forceinline__ double recip_pos(double s) {
+  double y = widen_f64(__frcp_rn(trunc_f32(s)));
+  double e = fma(-s, y, 1.0);
+  y = fma(y, fma(e, e, e), y);
+  return fma(fma(-s, y, 1.0), y, y);
+}
+// recip_pos and the bit conversions hold for 2^-60 < s < 2^60
+__device__ __forceinline__ bool in_fast_range(double s) {
+  const int e = __double2hiint(s) >> 20;
+  return e > 1023 - 60 && e < 1023 + 60;
+}
+
+// A segment polynomial of ff.pair_tab at the position u in [-1, 1) that the
+// bits b of r^2 give: degrees 0-5 in FP64, 6-8 (f.x, f.y, f.z) in FP32, where
+// they add less than 1e-9 of the value.
+__device__ __forceinline__ double pair_poly_at(long long b, double2 c01,
+                                               double2 c23, double2 c45,
+                                               float4 f) {
+  const double u = fma(
+      2.0, __longlong_as_double(((b << 6) & 0x000fffffffffffffLL) |
+                                0x3ff0000000000000LL), -3.0);
+  const float uf = fmaf(
+      2.0f, __int_as_float(((int)(b >> 23) & 0x007fffff) | 0x3f800000), -3.0f);
+  const float t = fmaf(fmaf(f.z, uf, f.y), uf, f.x);
+  double p = fma(widen_f64(t), u, c45.y);
+  p = fma(p, u, c45.x);
+  p = fma(p, u, c23.y);
+  p = fma(p, u, c23.x);
+  p = fma(p, u, c01.y);
+  return fma(p, u, c01.x);
+}
+
+// Segment polynomial `which` (0 energy, 1 force factor) of ff.pair_tab at
+// s; false outside its range.  The segment and the position u in [-1, 1) in
+// it come from the bits of s, as in seg_poly.
+__device__ __forceinline__ bool pair_poly(const FF &ff, int which, double s,
+                                          double *out) {
+  const long long b = bits64(s);
+  const int seg = (int)(b >> 46) - ff.etab_key0;
+  if (ff.pair_tab == nullptr || (unsigned)seg >= (unsigned)ff.etab_nseg)
+    return false;
+  const double2 *c = (const double2 *)(ff.pair_tab + ((size_t)seg * 2 + which) * 8);
+  *out = pair_poly_at(b, __ldg(c), __ldg(c + 1), __ldg(c + 2),
+                      __ldg((const float4 *)(c + 3)));
+  return true;
+}
 // Soft-core squared distance at coupling lambda (src/FFParticle.cpp:301-308):
 // cbrt(sc_alpha (1 - lambda)^sc_power max(sigma^6, sc_sigma^6) + r^6).
 __device__ __forceinline__ double soft_rsq(const FF &ff, double distSq,
