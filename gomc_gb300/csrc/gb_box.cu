@@ -707,19 +707,21 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
 }
 
 int Box::CheckError() {
-  int herr[4] = {0, 0, 0, 0};
-  int rc = CudaCheck(cudaMemcpyAsync(herr, dev.err, 16, cudaMemcpyDeviceToHost,
+  int word = 0;
+  int rc = CudaCheck(cudaMemcpyAsync(&word, dev.err, 4, cudaMemcpyDeviceToHost,
                                      stream),
                      "error read");
-  if (rc)
+  if (rc || (rc = Sync()))
     return rc;
-  if ((rc = Sync()))
-    return rc;
-  if (herr[0] & DERR_CELL_OVERFLOW)
+  return CheckErrorWord(word);
+}
+
+int Box::CheckErrorWord(int word) {
+  if (word & DERR_CELL_OVERFLOW)
     return Fail(ERR_CAPACITY, "a cell exceeded its slot capacity");
-  if (herr[0] & DERR_BARRIER_TIMEOUT)
+  if (word & DERR_BARRIER_TIMEOUT)
     return Fail(ERR_TIMEOUT, "a device-side wait ran out of iterations");
-  if (herr[0] & DERR_BAD_INPUT)
+  if (word & DERR_BAD_INPUT)
     return Fail(ERR_ARG, "invalid input detected on the device");
   return OK;
 }
@@ -752,7 +754,7 @@ int Box::CellAddMol(int m) {
   if (!cell_out[m])
     return Fail(ERR_STATE, "molecule is already in the cell list");
   int rc = launch_cell_add_mol(*this, m);
-  if (rc || (rc = CheckError()))
+  if (rc || (rc = Sync()) || (rc = CheckErrorWord(*(const int *)h_pinned)))
     return rc;
   cell_out[m] = 0;
   --n_cell_out;
@@ -980,21 +982,13 @@ int Box::MoleculeInter(int m, const double *new_pos, double *lj, double *real,
     return Fail(ERR_UNSUPPORTED, "molecule larger than 64 atoms");
   if (check_newpos(*this, m, new_pos, n))
     return Fail(ERR_ARG, "trial coordinates must lie inside the box");
-  std::memcpy(h_pinned, new_pos, 3 * n * sizeof(double));
-  int rc = CudaCheck(cudaMemcpyAsync(d_small + 1024, h_pinned, 3 * n * 8,
-                                     cudaMemcpyHostToDevice, stream),
-                     "upload");
-  if (rc || (rc = launch_mol_inter(*this, m, d_small + 1024, d_small)))
-    return rc;
-  if ((rc = CudaCheck(cudaMemcpyAsync(h_pinned, d_small, 24,
-                                      cudaMemcpyDeviceToHost, stream),
-                      "download")) ||
-      (rc = Sync()))
+  int rc = launch_mol_inter(*this, m, new_pos);
+  if (rc || (rc = Sync()))
     return rc;
   *lj = h_pinned[0];
   *real = h_pinned[1];
   *overlap = h_pinned[2] != 0.0;
-  return CheckError();
+  return CheckErrorWord(*(const int *)(h_pinned + 3));
 }
 
 // CalculateEnergy::VirialCalc (src/CalculateEnergy.cpp:411-579, LRC off)
@@ -1069,24 +1063,15 @@ int Box::ParticleInter(int m, int part, const double *trials, int ntrials,
   const double charge = host.q[host.mstart[m] + part];
   if (check_newpos(*this, m, trials, ntrials))
     return Fail(ERR_ARG, "trial coordinates must lie inside the box");
-  std::memcpy(h_pinned, trials, 3 * ntrials * sizeof(double));
-  int rc = CudaCheck(cudaMemcpyAsync(d_small + 1024, h_pinned, 3 * ntrials * 8,
-                                     cudaMemcpyHostToDevice, stream),
-                     "upload");
-  if (rc || (rc = launch_particle_inter(*this, kind, charge, d_small + 1024,
-                                        ntrials, d_small)))
-    return rc;
-  if ((rc = CudaCheck(cudaMemcpyAsync(h_pinned, d_small, 3 * ntrials * 8,
-                                      cudaMemcpyDeviceToHost, stream),
-                      "download")) ||
-      (rc = Sync()))
+  int rc = launch_particle_inter(*this, kind, charge, trials, ntrials);
+  if (rc || (rc = Sync()))
     return rc;
   for (int t = 0; t < ntrials; ++t) {
     en[t] = h_pinned[3 * t];
     real[t] = h_pinned[3 * t + 1];
     overlap[t] = h_pinned[3 * t + 2] != 0.0;
   }
-  return CheckError();
+  return CheckErrorWord(*(const int *)(h_pinned + 3 * ntrials));
 }
 
 int Box::MolReciprocal(int m, const double *new_pos, double *de) {
@@ -1099,16 +1084,8 @@ int Box::MolReciprocal(int m, const double *new_pos, double *de) {
   int n = host.mstart[m + 1] - host.mstart[m];
   if (n > 64)
     return Fail(ERR_UNSUPPORTED, "molecule larger than 64 atoms");
-  std::memcpy(h_pinned, new_pos, 3 * n * sizeof(double));
-  int rc = CudaCheck(cudaMemcpyAsync(d_small + 1024, h_pinned, 3 * n * 8,
-                                     cudaMemcpyHostToDevice, stream),
-                     "upload");
-  if (rc || (rc = launch_mol_recip(*this, m, d_small + 1024, 0, d_small)))
-    return rc;
-  if ((rc = CudaCheck(cudaMemcpyAsync(h_pinned, d_small, 8,
-                                      cudaMemcpyDeviceToHost, stream),
-                      "download")) ||
-      (rc = Sync()))
+  int rc = launch_mol_recip(*this, m, new_pos, 0);
+  if (rc || (rc = Sync()))
     return rc;
   *de = h_pinned[0];
   return OK;
@@ -1124,17 +1101,8 @@ int Box::SwapRecip(int m, const double *pos, bool insert, double *de) {
   int n = host.mstart[m + 1] - host.mstart[m];
   if (n > 64)
     return Fail(ERR_UNSUPPORTED, "molecule larger than 64 atoms");
-  std::memcpy(h_pinned, pos, 3 * n * sizeof(double));
-  int rc = CudaCheck(cudaMemcpyAsync(d_small + 1024, h_pinned, 3 * n * 8,
-                                     cudaMemcpyHostToDevice, stream),
-                     "upload");
-  if (rc || (rc = launch_mol_recip(*this, m, d_small + 1024, insert ? 1 : 2,
-                                   d_small)))
-    return rc;
-  if ((rc = CudaCheck(cudaMemcpyAsync(h_pinned, d_small, 8,
-                                      cudaMemcpyDeviceToHost, stream),
-                      "download")) ||
-      (rc = Sync()))
+  int rc = launch_mol_recip(*this, m, pos, insert ? 1 : 2);
+  if (rc || (rc = Sync()))
     return rc;
   *de = h_pinned[0];
   return OK;

@@ -105,6 +105,7 @@ class Box {
   int GetKVectors(double *out7);
   int GetSumNew(double *sr, double *si);
   int CheckError();
+  int CheckErrorWord(int word);
 
   // ---- internals shared with the Monte Carlo loop ----
   DevBox dev{};
@@ -207,13 +208,16 @@ int launch_recip_energy(Box &b, const double *sumR, const double *sumI,
                         double *d_out);
 int launch_recip_energy_view(Box &b, const DevBox &d, const double *sumR,
                              const double *sumI, double *d_out);
-int launch_mol_recip(Box &b, int m, const double *d_newpos, int sign_mode,
-                     double *d_out);
-int launch_mol_inter(Box &b, int m, const double *d_newpos, double *d_out3);
+// one launch each, results in h_pinned once the stream is idle: the energy
+// change
+int launch_mol_recip(Box &b, int m, const double *newpos, int sign_mode);
+// LJ, real space, overlap, device error word
+int launch_mol_inter(Box &b, int m, const double *newpos);
 int launch_single_mol_inter(Box &b, int m, const double *d_lam4,
                             double *d_out4);
+// per trial LJ, real space, overlap; then the device error word
 int launch_particle_inter(Box &b, int kind, double charge,
-                          const double *d_trials, int ntrials, double *d_out);
+                          const double *trials, int ntrials);
 int launch_cell_remove_mol(Box &b, int m);
 int launch_cell_add_mol(Box &b, int m);
 int launch_correction(Box &b, double *d_out);

@@ -94,24 +94,27 @@ __global__ void k_cell_remove_mol(DevBox b, int m) {
 
 // CellList::AddMol (src/CellList.cpp:115-135): put molecule m's atoms, at
 // their current coordinates, into the cells PositionToCell gives.
-__global__ void k_cell_add_mol(DevBox b, int m) {
-  for (int a = b.mstart[m]; a < b.mstart[m + 1]; ++a) {
+// The device error word goes to host memory with it.
+__global__ void k_cell_add_mol(DevBox b, int m, int *word) {
+  int bad = 0;
+  for (int a = b.mstart[m]; a < b.mstart[m + 1] && !bad; ++a) {
     if (b.atom_cell[a] >= 0)
       continue;
     double x = b.x[a], y = b.y[a], z = b.z[a];
     int c = position_to_cell_fast(b, x, y, z);
     if (c < 0 || c >= b.ncell) {
-      atomicOr(b.err, DERR_BAD_INPUT);
-      return;
+      bad = DERR_BAD_INPUT;
+      break;
     }
     int s = b.cell_count[c];
     if (s >= b.cap) {
-      atomicOr(b.err, DERR_CELL_OVERFLOW);
-      return;
+      bad = DERR_CELL_OVERFLOW;
+      break;
     }
     b.cell_count[c] = s + 1;
     cell_write_slot(b, c, s, a, x, y, z);
   }
+  *word = bad ? atomicOr(b.err, bad) | bad : *(volatile int *)b.err;
 }
 
 int launch_cell_remove_mol(Box &bx, int m) {
@@ -120,7 +123,7 @@ int launch_cell_remove_mol(Box &bx, int m) {
 }
 
 int launch_cell_add_mol(Box &bx, int m) {
-  k_cell_add_mol<<<1, 1, 0, bx.stream>>>(bx.dev, m);
+  k_cell_add_mol<<<1, 1, 0, bx.stream>>>(bx.dev, m, (int *)bx.h_pinned);
   return bx.CudaCheck(cudaGetLastError(), "cell add");
 }
 

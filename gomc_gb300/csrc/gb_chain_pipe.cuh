@@ -187,30 +187,6 @@ __device__ __forceinline__ bool pair_energy_pipe(const ChainArgs &A,
   return true;
 }
 
-// Sums over a warp of four values with six additions a lane instead of
-// twenty: the lanes share the values out as the sums fold.  Lane 0 has v[0],
-// lane 8 v[1], lane 16 v[2], lane 24 v[3].
-__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
-  const int lane = threadIdx.x & 31;
-  const bool h = lane & 16, g = lane & 8;
-  double a = h ? v[2] : v[0], b = h ? v[3] : v[1];
-  a += __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
-  b += __shfl_xor_sync(0xffffffffu, h ? v[1] : v[3], 16);
-  double c = g ? b : a;
-  c += __shfl_xor_sync(0xffffffffu, g ? a : b, 8);
-  for (int o = 4; o > 0; o >>= 1)
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-  return c;
-}
-// Two values, five additions: lane 0 has x, lane 16 y.
-__device__ __forceinline__ double warp_sum2(double x, double y) {
-  const bool h = threadIdx.x & 16;
-  double a = (h ? y : x) + __shfl_xor_sync(0xffffffffu, h ? x : y, 16);
-  for (int o = 8; o > 0; o >>= 1)
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-  return a;
-}
-
 // pair_energy_pipe added to one set of sums (a pair past a full list)
 __device__ __noinline__ void pair_term_pipe(const ChainArgs &A,
                                             const double *hdr, int a,

@@ -1,10 +1,9 @@
 // Real-space kernels (FP64 plain form):
 //   BoxInter        pair walk, a warp per atom, each pair once
 //                   (src/CalculateEnergy.cpp:157-266); VirialCalc likewise
-//   MoleculeInter   one CTA per (atom, old/new, neighbour cell)
+//   MoleculeInter   CTAs per (atom, old/new)
 //                   (src/CalculateEnergy.cpp:581-686)
-//   ParticleInter   one CTA per (trial, neighbour cell)
-//                   (src/CalculateEnergy.cpp:727-785)
+//   ParticleInter   CTAs per trial (src/CalculateEnergy.cpp:727-785)
 //   BoxForce        pair walk from both ends, no atomics
 //                   (src/CalculateEnergy.cpp:268-406)
 //   MolCorrection   per molecule (src/Ewald.cpp:1056-1085)
@@ -184,7 +183,10 @@ __device__ __forceinline__ void lj_terms(const FF &ff, double s, int idx,
                                          double *en, double *vir) {
   if (bits64(ff.nexp[idx]) == bits64(12.0) && in_fast_range(s)) {
     const double y = recip_pos(s);
-    const double rRat2 = y * ff.sigmaSq[idx];
+    // sigma^2 / r^2 to the last bit: its sixth power carries the error
+    const double sg = ff.sigmaSq[idx];
+    double rRat2 = y * sg;
+    rRat2 = fma(fma(-rRat2, s, sg), y, rRat2);
     const double attract = rRat2 * rRat2 * rRat2;
     const double repulse = attract * attract;
     if (en)
@@ -380,81 +382,210 @@ int launch_box_inter_view(Box &bx, const DevBox &b, double *d_out2) {
 }
 
 // ---------------------------------------------------------------------------
-// MoleculeInter: unit u = ((atom * 2 + side) * 27 + neighbour)
+// MoleculeInter and ParticleInter: the walk around points.  These calls are
+// bound by latency -- a launch, a few dependent loads and some 25 dependent
+// FP64 instructions of 64 cycles -- so there is one kernel a call: positions
+// come as kernel arguments with their cells and turns (taken on the host),
+// CTAs of four warps (one a sub-partition, each with its FP64 unit to itself)
+// walk the 27 cells around a point with the FP32 scan and FP64 batches of the
+// pair walk, and the last CTA adds the points' sums and writes them to the
+// host's pinned memory.  Up to 64 points a point has seven CTAs, a warp one
+// cell and so one batch (2,400-sphere liquid, 10 trials: one CTA of nine warps
+// a point took 14.7 us, two batches a warp and two warps a sub-partition);
+// beyond, the GPU is full and one CTA a point fills its batches better.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(RT) k_mol_inter(DevBox b, const FF *__restrict__ pff,
-                                                  int m, const double *__restrict__ newpos,
-                                                  double *part) {
+constexpr int PTW = 4;       // warps per CTA
+constexpr int PT_SPLIT = 7;  // CTAs per point of a small call
+template <int N>
+struct Points {
+  double xyz[3 * N];
+  uint32_t turn[3 * N];
+  int cell[N];
+};
+
+// MOL: points 2 a and 2 a + 1 are atom a of molecule m at its own and its new
+// position, the molecule itself left out, sums over all points; else point t
+// is a trial position of an atom of kind ka and charge qa, sums per trial.
+template <bool MOL, int N>
+__global__ void __launch_bounds__(32 * PTW) k_points(DevBox b, const FF *__restrict__ pff,
+                                                     const __grid_constant__ Points<N> P,
+                                                     int parts, int m, int ka,
+                                                     double qa, double *part,
+                                                     double *out) {
+  __shared__ int queue[PTW][PQ];
+  __shared__ double red[2][PTW];
   const FF &ff = *pff;
-  int u = blockIdx.x;
-  int a = u / (2 * NB27), side = (u / NB27) % 2, n = u % NB27;
-  int atom = b.mstart[m] + a;
-  double px, py, pz;
-  if (side == 0) {
-    px = b.x[atom];
-    py = b.y[atom];
-    pz = b.z[atom];
-  } else {
-    px = newpos[3 * a];
-    py = newpos[3 * a + 1];
-    pz = newpos[3 * a + 2];
-  }
-  int cell = position_to_cell_fast(b, px, py, pz);
-  int c2 = b.nbr[cell * NB27 + n];
-  int n2 = b.cell_count[c2];
-  double qa = b.q[atom];
-  int ka = b.kind[atom];
-  double lj = 0.0, re = 0.0, ovl = 0.0;
-  for (int j = threadIdx.x; j < n2; j += RT) {
-    size_t s = (size_t)c2 * b.cap + j;
-    int mj = b.cell_meta[s];
-    if (meta_mol(mj) == m)
-      continue;  // the moving molecule is out of the cell list
-    double4_32a pj = b.cell_pos[s];
-    double dx = min_image(px - pj.x, b.L[0], b.half[0]);
-    double dy = min_image(py - pj.y, b.L[1], b.half[1]);
-    double dz = min_image(pz - pj.z, b.L[2], b.half[2]);
-    double distSq = dsq3(dx, dy, dz);
-    if (ff.rcutSq > distSq) {
-      if (side == 1 && distSq < ff.rcutLowSq)
-        ovl = 1.0;
-      double e = 0.0;
-      if (ff.electrostatic) {
-        double qq = qa * pj.w * QQ_FACT;
-        if (qq != 0.0)
-          e = coulomb_energy(ff, distSq, qq);
-      }
-      double l = lj_energy(ff, distSq, ka + meta_kind(mj) * ff.n_kinds);
-      if (side == 0) {
-        re += -e;
-        lj += -l;
-      } else {
-        re += e;
-        lj += l;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int pt = blockIdx.x / parts, sub = blockIdx.x - pt * parts;
+  const int i = MOL ? pt >> 1 : pt;
+  const bool fresh = !MOL || (pt & 1);
+  double4_32a pi = make_double4_32a(P.xyz[3 * i], P.xyz[3 * i + 1],
+                                    P.xyz[3 * i + 2], qa);
+  uint4 ti = make_uint4(P.turn[3 * i], P.turn[3 * i + 1], P.turn[3 * i + 2], 0);
+  int cell = P.cell[i];
+  if constexpr (MOL) {
+    const int atom = b.mstart[m] + i;
+    pi.w = b.q[atom];
+    ka = b.kind[atom];
+    if (!fresh) {
+      pi.x = b.x[atom];
+      pi.y = b.y[atom];
+      pi.z = b.z[atom];
+      cell = b.atom_cell[atom];
+      if (cell >= 0) {
+        ti = b.cell_fix[(size_t)cell * b.cap + b.atom_slot[atom]];
+      } else {  // out of the grid
+        cell = position_to_cell_fast(b, pi.x, pi.y, pi.z);
+        ti = make_uint4(to_turns(pi.x, b.invL[0]), to_turns(pi.y, b.invL[1]),
+                        to_turns(pi.z, b.invL[2]), 0);
       }
     }
   }
-  __shared__ double red[RT / 32];
-  double A = block_sum<RT>(lj, red);
-  double R = block_sum<RT>(re, red);
-  double O = block_sum<RT>(ovl, red);
-  if (threadIdx.x == 0) {
-    part[3 * u] = A;
-    part[3 * u + 1] = R;
-    part[3 * u + 2] = O > 0 ? 1.0 : 0.0;
+  const Scan sc = scan_of(b, ff);
+  double lj = 0.0, re = 0.0;
+  bool ovl = false;
+  const double qi = pi.w * QQ_FACT;
+  int *q = queue[warp];
+  auto eval = [&](bool act, int gj) {
+    double4_32a pj = make_double4_32a(0, 0, 0, 0);
+    int idx = 0;
+    if (act) {
+      pj = b.cell_pos[gj];
+      idx = ka + meta_kind(b.cell_meta[gj]) * ff.n_kinds;
+    }
+    double v[3], distSq;
+    const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+    ovl |= in && fresh && gt_pos(ff.rcutLowSq, distSq);
+    if (ff.electrostatic && in) {
+      const double qq = qi * pj.w;
+      if (qq != 0.0) {
+        double p;
+        if (!gt_pos(distSq, ff.rcutCoulSq) && ff.ewald &&
+            pair_poly(ff, 0, distSq, &p))
+          re = fma(qq, p, re);
+        else
+          re += coulomb_energy(ff, distSq, qq);
+      }
+    }
+    if (in && lj_live(ff, distSq, idx)) {
+      double l;
+      lj_terms(ff, distSq, idx, &l, nullptr);
+      lj += l;
+    }
+  };
+  int qn = 0;  // warp-uniform queue fill
+  for (int nn = sub * PTW + warp; nn < NB27; nn += parts * PTW) {
+    const int c2 = b.nbr[cell * NB27 + nn];
+    const int n2 = b.cell_count[c2];
+    for (int j0 = 0; j0 < n2; j0 += 32) {
+      const int gj = c2 * b.cap + j0 + lane;
+      bool in = j0 + lane < n2;
+      if (in)
+        in = scan_near(sc, ti, b.cell_fix[gj]) &&
+             !(MOL && meta_mol(b.cell_meta[gj]) == m);
+      const unsigned mask = __ballot_sync(0xffffffffu, in);
+      if (in)
+        q[qn + __popc(mask & lt)] = gj;
+      qn += __popc(mask);
+      __syncwarp();
+      if (qn >= 32) {
+        const int e = q[lane], mv = q[32 + lane];
+        __syncwarp();
+        qn -= 32;
+        if (lane < qn)
+          q[lane] = mv;
+        __syncwarp();
+        eval(true, e);
+      }
+    }
   }
+  if (qn > 0)
+    eval(lane < qn, q[lane]);
+  const double w = warp_sum2(lj, re);
+  if ((lane & 15) == 0)
+    red[lane >> 4][warp] = w;
+  const bool any = __syncthreads_or(ovl);
+  if (warp == 0) {  // lanes 0-3 the warps' LJ, 16-19 their real space
+    const int k = lane & 15;
+    double v = k < PTW ? red[lane >> 4][k] : 0.0;
+    for (int o = 2; o > 0; o >>= 1)
+      v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (k == 0)
+      part[3 * blockIdx.x + (lane >> 4)] = fresh ? v : -v;
+    if (lane == 0)
+      part[3 * blockIdx.x + 2] = any ? 1.0 : 0.0;
+  }
+  if (!last_cta((unsigned *)b.err + 2))
+    return;
+  const int n = gridDim.x;
+  if constexpr (MOL) {
+    if (warp == 0) {
+      double a = 0.0, r = 0.0;
+      bool o = false;
+      for (int k = lane; k < n; k += 32) {
+        a += __ldcg(part + 3 * k);
+        r += __ldcg(part + 3 * k + 1);
+        o |= __ldcg(part + 3 * k + 2) != 0.0;
+      }
+      const double t = warp_sum2(a, r);
+      o = __any_sync(0xffffffffu, o);
+      if ((lane & 15) == 0)
+        out[lane >> 4] = t;
+      if (lane == 0)
+        out[2] = o ? 1.0 : 0.0;
+    }
+  } else {
+    for (int k = threadIdx.x; k < 3 * (n / parts); k += 32 * PTW) {
+      const double *p = part + (size_t)(k / 3) * parts * 3 + k % 3;
+      double v = 0.0;
+      for (int j = 0; j < parts; ++j)
+        v += __ldcg(p + 3 * j);
+      out[k] = v;
+    }
+  }
+  if (threadIdx.x == 0)
+    *(int *)(out + 3 * (MOL ? 1 : n / parts)) = *(volatile int *)b.err;
 }
 
-int launch_mol_inter(Box &bx, int m, const double *d_newpos, double *d_out3) {
-  int na = bx.host.mstart[m + 1] - bx.host.mstart[m];
-  int units = na * 2 * NB27;
-  int rc = bx.EnsureScratch((size_t)units * 3);
+template <bool MOL, int N>
+static int launch_points(Box &bx, const double *xyz, int n, int m, int kind,
+                         double charge, const char *what) {
+  const DevBox &b = bx.dev;
+  const int pts = MOL ? 2 * n : n, parts = pts <= 64 ? PT_SPLIT : 1;
+  int rc = bx.EnsureScratch((size_t)3 * pts * parts);
   if (rc)
     return rc;
-  k_mol_inter<<<units, RT, 0, bx.stream>>>(bx.dev, bx.d_ff, m, d_newpos,
-                                           bx.d_scratch);
-  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, units, 3, d_out3, 1);
-  return bx.CudaCheck(cudaGetLastError(), "molecule inter");
+  Points<N> P;
+  for (int i = 0; i < n; ++i) {
+    for (int d = 0; d < 3; ++d) {
+      P.xyz[3 * i + d] = xyz[3 * i + d];
+      P.turn[3 * i + d] = to_turns(xyz[3 * i + d], b.invL[d]);
+    }
+    P.cell[i] = position_to_cell(b, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]);
+  }
+  k_points<MOL, N><<<pts * parts, 32 * PTW, 0, bx.stream>>>(
+      b, bx.d_ff, P, parts, m, kind, charge, bx.d_scratch, bx.h_pinned);
+  return bx.CudaCheck(cudaGetLastError(), what);
+}
+
+// Arguments of up to 16 positions in the small form (0.7 KB of kernel
+// arguments instead of 10 KB).
+int launch_mol_inter(Box &bx, int m, const double *newpos) {
+  const int n = bx.host.mstart[m + 1] - bx.host.mstart[m];
+  return n <= 16 ? launch_points<true, 16>(bx, newpos, n, m, 0, 0.0, "molecule inter")
+                 : launch_points<true, 64>(bx, newpos, n, m, 0, 0.0, "molecule inter");
+}
+
+// ParticleInter: against every atom the cell grid holds (a molecule being
+// grown by CBMC is taken out of the grid first, as in the reference).
+int launch_particle_inter(Box &bx, int kind, double charge,
+                          const double *trials, int ntrials) {
+  return ntrials <= 16
+             ? launch_points<false, 16>(bx, trials, ntrials, 0, kind, charge,
+                                        "particle inter")
+             : launch_points<false, 256>(bx, trials, ntrials, 0, kind, charge,
+                                         "particle inter");
 }
 
 // ---------------------------------------------------------------------------
@@ -521,83 +652,6 @@ int launch_single_mol_inter(Box &bx, int m, const double *d_lam4,
                                                   bx.d_scratch);
   k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, units, 4, d_out4, 0);
   return bx.CudaCheck(cudaGetLastError(), "single molecule inter");
-}
-
-// ---------------------------------------------------------------------------
-// ParticleInter: unit u = trial * 27 + neighbour, against every atom the
-// cell grid holds (a molecule being grown by CBMC is taken out of the grid
-// first, as in the reference).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(RT) k_particle_inter(DevBox b, const FF *__restrict__ pff,
-                                                       int ka, double qa,
-                                                       const double *__restrict__ trials,
-                                                       double *part) {
-  const FF &ff = *pff;
-  int u = blockIdx.x;
-  int t = u / NB27, n = u % NB27;
-  double px = trials[3 * t], py = trials[3 * t + 1], pz = trials[3 * t + 2];
-  int cell = position_to_cell_fast(b, px, py, pz);
-  int c2 = b.nbr[cell * NB27 + n];
-  int n2 = b.cell_count[c2];
-  double lj = 0.0, re = 0.0, ovl = 0.0;
-  for (int j = threadIdx.x; j < n2; j += RT) {
-    size_t s = (size_t)c2 * b.cap + j;
-    int mj = b.cell_meta[s];
-    double4_32a pj = b.cell_pos[s];
-    double dx = min_image(px - pj.x, b.L[0], b.half[0]);
-    double dy = min_image(py - pj.y, b.L[1], b.half[1]);
-    double dz = min_image(pz - pj.z, b.L[2], b.half[2]);
-    double distSq = dsq3(dx, dy, dz);
-    if (ff.rcutSq > distSq) {
-      if (distSq < ff.rcutLowSq)
-        ovl = 1.0;
-      lj += lj_energy(ff, distSq, ka + meta_kind(mj) * ff.n_kinds);
-      if (ff.electrostatic) {
-        double qq = pj.w * qa * QQ_FACT;
-        if (qq != 0.0)
-          re += coulomb_energy(ff, distSq, qq);
-      }
-    }
-  }
-  __shared__ double red[RT / 32];
-  double A = block_sum<RT>(lj, red);
-  double R = block_sum<RT>(re, red);
-  double O = block_sum<RT>(ovl, red);
-  if (threadIdx.x == 0) {
-    part[3 * u] = A;
-    part[3 * u + 1] = R;
-    part[3 * u + 2] = O > 0 ? 1.0 : 0.0;
-  }
-}
-
-__global__ void k_reduce_trials(const double *__restrict__ part, int ntrials,
-                                double *out) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntrials)
-    return;
-  double a = 0, r = 0, o = 0;
-  for (int n = 0; n < NB27; ++n) {
-    const double *p = part + 3 * ((size_t)t * NB27 + n);
-    a += p[0];
-    r += p[1];
-    o = fmax(o, p[2]);
-  }
-  out[3 * t] = a;
-  out[3 * t + 1] = r;
-  out[3 * t + 2] = o;
-}
-
-int launch_particle_inter(Box &bx, int kind, double charge,
-                          const double *d_trials, int ntrials, double *d_out) {
-  int units = ntrials * NB27;
-  int rc = bx.EnsureScratch((size_t)units * 3);
-  if (rc)
-    return rc;
-  k_particle_inter<<<units, RT, 0, bx.stream>>>(bx.dev, bx.d_ff, kind, charge,
-                                                d_trials, bx.d_scratch);
-  k_reduce_trials<<<(ntrials + 127) / 128, 128, 0, bx.stream>>>(bx.d_scratch,
-                                                               ntrials, d_out);
-  return bx.CudaCheck(cudaGetLastError(), "particle inter");
 }
 
 // ---------------------------------------------------------------------------

@@ -10,6 +10,7 @@
 //
 // The sums over all atoms and k-vectors are in gb_ewald.cu.
 #include "gb_box.h"
+#include "gb_fixed.cuh"
 #include "gb_pair.cuh"
 
 namespace gb {
@@ -61,67 +62,145 @@ int launch_recip_energy_view(Box &bx, const DevBox &b, const double *sumR,
 
 // ---------------------------------------------------------------------------
 // One-molecule delta.  mode 0: displacement/rotation (new - old),
-// 1: insertion (+ new), 2: deletion (- given positions).  One thread per k,
-// with the reference's dot-product phases.
+// 1: insertion (+ new), 2: deletion (- given positions).  One launch: every
+// CTA forms the phase rows exp(i n 2 pi r_d / L_d) of up to eight positions at
+// a time in fixed point (integer work; the sine and cosine of every k . r in
+// FP64 cost about 100 instructions of 64 cycles each), a thread then sums its
+// k-vector's products, and the last CTA adds the energies.
 // ---------------------------------------------------------------------------
-__global__ void k_mol_recip(DevBox b, int m, const double *__restrict__ newpos,
-                            int mode, double *part) {
-  int k = blockIdx.x * ET + threadIdx.x;
-  double e = 0.0;
-  if (k < b.K) {
-    int a0 = b.mstart[m], n = b.mstart[m + 1] - a0;
-    double kx = b.kx[k], ky = b.ky[k], kz = b.kz[k];
-    double rN = 0, iN = 0, rO = 0, iO = 0;
-    for (int p = 0; p < n; ++p) {
-      int a = a0 + p;
-      double q = b.q[a];
-      if (fabs(q) < 0.000000001)
-        continue;
-      double dn = (newpos[3 * p] * kx + newpos[3 * p + 1] * ky +
-                   newpos[3 * p + 2] * kz);
-      double s, c;
-      sincos(dn, &s, &c);
-      rN += q * c;
-      iN += q * s;
-      if (mode == 0) {
-        double dold = (b.x[a] * kx + b.y[a] * ky + b.z[a] * kz);
-        sincos(dold, &s, &c);
-        rO += q * c;
-        iO += q * s;
+constexpr int MRT = 128;  // threads (k-vectors) per CTA
+constexpr int MRP = 8;    // positions per pass
+template <int N>
+struct NewPos {
+  double xyz[3 * N];
+};
+
+template <int N>
+__global__ void __launch_bounds__(MRT) k_mol_recip(DevBox b, int m,
+                                                   const __grid_constant__ NewPos<N> P,
+                                                   int mode, double *part,
+                                                   double *out) {
+  extern __shared__ double2 rows[];  // [MRP][3][kmax + 1]
+  __shared__ unsigned long long us[3 * MRP];
+  __shared__ double qs[MRP];
+  __shared__ int bad;  // a coordinate that is not finite
+  const int k = blockIdx.x * MRT + threadIdx.x;
+  const int stride = b.kmax + 1;
+  const int a0 = b.mstart[m], n = b.mstart[m + 1] - a0;
+  const int np = mode == 0 ? 2 * n : n;  // new positions, then the old ones
+  char4 kn = make_char4(0, 0, 0, 0);
+  if (k < b.K)
+    kn = b.kn[k];
+  if (threadIdx.x == 0)
+    bad = 0;
+  double dR = 0.0, dI = 0.0;
+  for (int p0 = 0; p0 < np; p0 += MRP) {
+    const int cnt = min(MRP, np - p0);
+    __syncthreads();
+    if (threadIdx.x < 3 * cnt) {
+      const int p = p0 + threadIdx.x / 3, d = threadIdx.x % 3;
+      const int a = a0 + (p < n ? p : p - n);
+      const double x = p < n ? P.xyz[3 * p + d]
+                             : (d == 0 ? b.x : d == 1 ? b.y : b.z)[a];
+      us[threadIdx.x] = turn64(x, b.L[d]);
+      if (!isfinite(x))
+        bad = 1;
+      if (d == 0) {
+        const double q = b.q[a];
+        // - for the old positions and for a deletion
+        qs[threadIdx.x / 3] = fabs(q) < 0.000000001      ? 0.0
+                              : (p >= n || mode == 2) ? -q
+                                                      : q;
       }
     }
-    double sr, si;
-    if (mode == 0) {
-      sr = b.sumRref[k] + 1.0 * (rN - rO);
-      si = b.sumIref[k] + 1.0 * (iN - iO);
-    } else if (mode == 1) {
-      sr = b.sumRref[k] + rN;
-      si = b.sumIref[k] + iN;
-    } else {
-      sr = b.sumRref[k] - rN;
-      si = b.sumIref[k] - iN;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 3 * cnt * stride; e += MRT) {
+      const int r = e / stride, j = e - r * stride;
+      const Cis c = cis_q62(us[r] * (unsigned long long)j);
+      const double f = (r % 3 ? 1.0 : qs[r / 3]) / 4611686018427387904.0;  // 2^62
+      rows[e] = make_double2((double)c.c * f, (double)c.s * f);
     }
+    __syncthreads();
+    for (int p = 0; p < cnt; ++p) {
+      const double2 *r = rows + (size_t)(3 * p) * stride;
+      const double2 x = r[kn.x];
+      double2 y = r[stride + abs(kn.y)], z = r[2 * stride + abs(kn.z)];
+      if (kn.y < 0)
+        y.y = -y.y;
+      if (kn.z < 0)
+        z.y = -z.y;
+      const double2 v = make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
+      dR = fma(v.x, z.x, fma(-v.y, z.y, dR));
+      dI = fma(v.x, z.y, fma(v.y, z.x, dI));
+    }
+  }
+  double e = 0.0;
+  if (k < b.K) {
+    if (bad)
+      dR = dI = nan("");
+    const double sr = b.sumRref[k] + dR, si = b.sumIref[k] + dI;
     b.sumRnew[k] = sr;
     b.sumInew[k] = si;
     e = (sr * sr + si * si) * b.prefact[k];
   }
+  // The energy in the order of k_recip_energy and k_sum_in_order (the sums of
+  // 256 k-vectors as eight warp sums in turn, these over 256 threads), so
+  // that the rounding of the new and the stored energy cancels in their
+  // difference.
+  for (int o = 16; o > 0; o >>= 1)
+    e += __shfl_down_sync(0xffffffffu, e, o);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0)
+    part[blockIdx.x * (MRT / 32) + warp] = e;
+  if (!last_cta((unsigned *)b.err + 2))
+    return;
   __shared__ double red[ET / 32];
-  double s = block_sum<ET>(e, red);
-  if (threadIdx.x == 0)
-    part[blockIdx.x] = s;
+  const int nw = gridDim.x * (MRT / 32), nb = (b.K + ET - 1) / ET;
+  for (int vw = warp; vw < ET / 32; vw += MRT / 32) {
+    double v = 0.0;
+    for (int i = vw * 32 + lane; i < nb; i += ET) {
+      double c = 0.0;
+      for (int w = 0; w < ET / 32; ++w)
+        if (i * (ET / 32) + w < nw)
+          c += __ldcg(part + i * (ET / 32) + w);
+      v += c;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+      v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0)
+      red[vw] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = 0.0;
+    for (int w = 0; w < ET / 32; ++w)
+      v += red[w];
+    out[0] = v - b.energy[2];  // - sysPotRef.boxEnergy[box].recip
+  }
 }
 
-int launch_mol_recip(Box &bx, int m, const double *d_newpos, int mode,
-                     double *d_out) {
-  DevBox &b = bx.dev;
-  int nb = (b.K + ET - 1) / ET;
-  int rc = bx.EnsureScratch(nb);
+template <int N>
+static int launch_mol_recip_n(Box &bx, int m, const double *newpos, int n,
+                              int mode) {
+  const DevBox &b = bx.dev;
+  const int nb = (b.K + MRT - 1) / MRT;
+  int rc = bx.EnsureScratch((size_t)nb * (MRT / 32));
   if (rc)
     return rc;
-  k_mol_recip<<<nb, ET, 0, bx.stream>>>(b, m, d_newpos, mode, bx.d_scratch);
-  // energyRecipNew - sysPotRef.boxEnergy[box].recip
-  k_sum_in_order<<<1, ET, 0, bx.stream>>>(bx.d_scratch, nb, b.energy + 2, d_out);
+  NewPos<N> P;
+  for (int i = 0; i < 3 * n; ++i)
+    P.xyz[i] = newpos[i];
+  const size_t sh = (size_t)3 * MRP * (b.kmax + 1) * sizeof(double2);
+  raise_smem_limit((const void *)k_mol_recip<N>, sh);
+  k_mol_recip<N><<<nb, MRT, sh, bx.stream>>>(b, m, P, mode, bx.d_scratch,
+                                             bx.h_pinned);
   return bx.CudaCheck(cudaGetLastError(), "mol recip");
+}
+
+int launch_mol_recip(Box &bx, int m, const double *newpos, int mode) {
+  const int n = bx.host.mstart[m + 1] - bx.host.mstart[m];
+  return n <= 16 ? launch_mol_recip_n<16>(bx, m, newpos, n, mode)
+                 : launch_mol_recip_n<64>(bx, m, newpos, n, mode);
 }
 
 // ---------------------------------------------------------------------------
