@@ -103,6 +103,9 @@ __device__ __forceinline__ double coulomb_virial(const FF &ff, double distSq,
 __device__ __forceinline__ long long bits64(double v) {
   return __double_as_longlong(v);
 }
+__device__ __forceinline__ bool nonzero(double v) {
+  return (bits64(v) << 1) != 0;
+}
 // a > b of two non-negative values (NaN above all), on the integer pipe
 __device__ __forceinline__ bool gt_pos(double a, double b) {
   return bits64(a) > bits64(b);

@@ -99,10 +99,11 @@ __global__ void __launch_bounds__(RCT) k_reduce_cols(const double *__restrict__ 
 //     radius is padded beyond its rounding; survivors are compacted into a
 //     queue of the warp, and FP64 runs on full batches of 32 pairs, with the
 //     exact FP64 cutoff test;
-//   * energies and the virial take each pair once (cells c2 > c, and later
-//     slots of the own cell), the force walk takes a pair from both ends: the
-//     warp's lanes then hold one atom's force, so no atomics are needed and
-//     every sum has a fixed order;
+//   * energies and the virial take each pair once (the 13 neighbour cells
+//     after the own one in the table, which are the other 13 seen from there,
+//     and later slots of the own cell: the same work for every cell), the
+//     force walk takes a pair from both ends: the warp's lanes then hold one
+//     atom's force, so no atomics are needed and every sum has a fixed order;
 //   * comparisons of FP64 values are made on their bits, a minimum-image
 //     shift is added only where a lane of the batch needs one, Lennard-Jones
 //     terms are skipped for a batch without any (a hydrogen's whole walk),
@@ -175,7 +176,7 @@ __device__ __forceinline__ bool pair_sep(const DevBox &b, const FF &ff, bool act
 // Whether a pair's Lennard-Jones terms can be other than zero: a zero
 // epsilon gives zero unless (sigma^2 / r^2)^6 overflows.
 __device__ __forceinline__ bool lj_live(const FF &ff, double distSq, int idx) {
-  return ff.eps_cn[idx] != 0.0 || !in_fast_range(distSq);
+  return nonzero(ff.eps_cn[idx]) || !in_fast_range(distSq);
 }
 
 // lj_energy and lj_virial of one pair (either may be NULL), sharing 1 / r^2.
@@ -201,7 +202,8 @@ __device__ __forceinline__ void lj_terms(const FF &ff, double s, int idx,
     *vir = lj_virial(ff, s, idx);
 }
 
-// Energies of one batch added to lj and re (every lane of the warp calls).
+// Energies of one batch added to lj and re (every lane of the warp calls; re
+// without QQ_FACT).
 __device__ __forceinline__ void batch_energy(const DevBox &b, const FF &ff,
                                              bool act, int2 e, double &lj,
                                              double &re) {
@@ -215,8 +217,8 @@ __device__ __forceinline__ void batch_energy(const DevBox &b, const FF &ff,
   double v[3], distSq;
   const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
   if (ff.electrostatic && in) {
-    const double qq = pi.w * pj.w * QQ_FACT;
-    if (qq != 0.0) {
+    const double qq = pi.w * pj.w;
+    if (nonzero(qq)) {
       double p;
       if (!gt_pos(distSq, ff.rcutCoulSq) && ff.ewald &&
           pair_poly(ff, 0, distSq, &p))
@@ -256,7 +258,7 @@ __device__ __forceinline__ void batch_virial(const DevBox &b, const FF &ff,
   w[2] = v[2] * min_image_warp(b.cz[mi] - b.cz[mj], b.L[2], b.half[2]);
   if (ff.electrostatic && in) {
     const double qi_qj = pi.w * pj.w;
-    if (qi_qj != 0.0) {
+    if (nonzero(qi_qj)) {
       double p;
       if (!gt_pos(distSq, ff.rcutCoulSq) && ff.ewald &&
           pair_poly(ff, 1, distSq, &p))
@@ -304,12 +306,10 @@ __global__ void __launch_bounds__(RT) k_box_pairs(DevBox b, const FF *__restrict
     const int gi = c * b.cap + s;
     const uint4 ti = b.cell_fix[gi];
     const int moli = meta_mol(b.cell_meta[gi]);
-    for (int nn = 0; nn < NB27; ++nn) {
+    for (int nn = NB27 / 2; nn < NB27; ++nn) {
       const int c2 = b.nbr[c * NB27 + nn];
-      if (c2 < c)
-        continue;
       const int n2 = b.cell_count[c2];
-      for (int j0 = c2 == c ? s + 1 : 0; j0 < n2; j0 += 32) {
+      for (int j0 = nn == NB27 / 2 ? s + 1 : 0; j0 < n2; j0 += 32) {
         const int gj = c2 * b.cap + j0 + lane;
         bool in = j0 + lane < n2;
         if (in)
@@ -341,15 +341,16 @@ __global__ void __launch_bounds__(RT) k_box_pairs(DevBox b, const FF *__restrict
   for (int k = 0; k < NV; ++k) {
     const double r = block_sum<RT>(v[k], red);
     if (threadIdx.x == 0)
-      part[NV * t + k] = r;
+      part[NV * t + k] = MODE == 0 && k == 1 ? r * QQ_FACT : r;
   }
 }
 
-// CTAs per cell: about 32 warps an SM in all, a warp taking one to eight
-// atoms (more atoms per warp fill the last batch of its queue better).
+// CTAs per cell: about 64 warps an SM in all, a warp taking one to eight
+// atoms (12 to 128 warps an SM measured within 8 % of each other on 2,001 to
+// 20,000 waters, 64 the best or next to it).
 static int pair_split(const Box &bx, const DevBox &b) {
   const int avg = (b.n_atoms + b.ncell - 1) / b.ncell;
-  const int per = std::max(1, std::min(8, b.n_atoms / (32 * bx.sm_count)));
+  const int per = std::max(1, std::min(8, b.n_atoms / (64 * bx.sm_count)));
   return std::max(1, (avg + PW * per - 1) / (PW * per));
 }
 
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(32 * PTW) k_points(DevBox b, const FF *__restr
     ovl |= in && fresh && gt_pos(ff.rcutLowSq, distSq);
     if (ff.electrostatic && in) {
       const double qq = qi * pj.w;
-      if (qq != 0.0) {
+      if (nonzero(qq)) {
         double p;
         if (!gt_pos(distSq, ff.rcutCoulSq) && ff.ewald &&
             pair_poly(ff, 0, distSq, &p))
@@ -734,16 +735,15 @@ __global__ void __launch_bounds__(RT) k_box_force(DevBox b, const FF *__restrict
       const bool table = in && !gt_pos(distSq, ff.rcutCoulSq) && ff.ewald;
       if (ff.electrostatic && in) {
         const double qq = qi * pj.w;
-        if (qq != 0.0) {
-          double p;
-          if (table && pair_poly(ff, 1, distSq, &p))
+        if (nonzero(qq)) {
+          double p, e = 0.0;
+          if (table && pair_poly(ff, 1, distSq, &p)) {
             f = qq * p;
-          else
+            if (first && pair_poly(ff, 0, distSq, &e))
+              re = fma(qq, e, re);
+          } else {
             f = coulomb_virial(ff, distSq, qq);
-          if (first) {
-            if (table && pair_poly(ff, 0, distSq, &p))
-              re = fma(qq, p, re);
-            else
+            if (first)
               re += coulomb_energy(ff, distSq, qq);
           }
         }
@@ -773,7 +773,8 @@ __global__ void __launch_bounds__(RT) k_box_force(DevBox b, const FF *__restrict
                meta_mol(b.cell_meta[gj]) != moli;
         const unsigned m = __ballot_sync(0xffffffffu, in);
         if (in)
-          q[qn + __popc(m & lt)] = (unsigned)gj << 1 | (c2 > c || (c2 == c && j > s) ? 1u : 0u);
+          q[qn + __popc(m & lt)] =
+              (unsigned)gj << 1 | (nn > NB27 / 2 || (nn == NB27 / 2 && j > s) ? 1u : 0u);
         qn += __popc(m);
         __syncwarp();
         if (qn >= 32) {
