@@ -74,7 +74,8 @@ struct Move {
   float nlt[2][3];         // volume: FP32 turn lengths at the new edges
   double d[4];             // values reported in the trace
   double tot[PMAX];        // cluster sums of the partials
-  unsigned words[6 * GEMC_NTMAX + 2];  // raw words of a transfer's build
+  // raw words of a transfer's build; then its running weight sums
+  __align__(8) unsigned words[6 * GEMC_NTMAX + 2];
   double wts[2 * GEMC_NTMAX];      // trial weights
 };
 
@@ -108,11 +109,10 @@ __device__ __forceinline__ double unwrapd(double v, double ref, double ax,
   }
   return v;
 }
+// (compared on the bits: an FP64 comparison costs as much as an addition)
 __device__ __forceinline__ double mimg(double raw, double ax, double half) {
-  if (raw > half)
-    raw -= ax;
-  else if (raw < -half)
-    raw += ax;
+  if ((bits64(raw) & 0x7fffffffffffffffLL) > bits64(half))
+    raw -= copysign(ax, raw);
   return raw;
 }
 __device__ __forceinline__ float mimgf(float raw, float ax, float half) {
@@ -124,12 +124,39 @@ __device__ __forceinline__ float mimgf(float raw, float ax, float half) {
 }
 // FFParticle::CalcEn, lambda = 1 (src/FFParticle.cpp:295-325), inside Rcut
 __device__ __forceinline__ double lj64(const GemcParams &p, double d2) {
-  double rRat2 = p.sigmaSq / d2;
+  double rRat2;
+  if (in_fast_range(d2)) {
+    // sigma^2 / r^2 from the FP32 reciprocal: one cubic step, the product
+    // and its correction, six FP64 instructions for the division's dozen
+    double y = widen_f64(__frcp_rn(trunc_f32(d2)));
+    const double e = fma(-d2, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    rRat2 = p.sigmaSq * y;
+    rRat2 = fma(fma(-rRat2, d2, p.sigmaSq), y, rRat2);
+  } else {
+    rRat2 = p.sigmaSq / d2;
+  }
   double rRat4 = rRat2 * rRat2;
   double attract = rRat4 * rRat2;
-  double repulse = p.nexp == 12.0 ? attract * attract
-                                  : pow(rRat2, p.nexp * 0.5);
+  double repulse = bits64(p.nexp) == bits64(12.0) ? attract * attract
+                                                  : pow(rRat2, p.nexp * 0.5);
   return p.eps_cn * (repulse - attract);
+}
+// u < exp(x): decided on FP32 values unless they are within 1e-3 of one
+// another (the FP32 exponential's argument and result are good to 2e-5 for
+// |x| < 80), else in FP64, whose exponential takes about 30 dependent
+// instructions of 64 cycles.
+__device__ __forceinline__ int below_exp(double u, double x) {
+  const double ax = __longlong_as_double(bits64(x) & 0x7fffffffffffffffLL);
+  if (gt_pos(80.0, ax) && in_fast_range(ax) && in_fast_range(u)) {
+    const float e = __expf(bits64(x) < 0 ? -trunc_f32(ax) : trunc_f32(ax));
+    const float uf = trunc_f32(u);
+    if (uf > e * 1.001f)
+      return 0;
+    if (uf < e * 0.999f)
+      return 1;
+  }
+  return u < exp(x);
 }
 __device__ __forceinline__ float lj32(const GemcParams &p, float d2) {
   float s = __fdividef(p.sigmaSq_f, d2);
@@ -668,10 +695,10 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           double d2 = r2_f64(nw ? npx : opx, nw ? npy : opy, nw ? npz : opz,
                              A.px[e.x], A.py[e.x], A.pz[e.x], c.ax[b],
                              c.half[b]);
-          if (d2 < p.rcutSq) {
+          if (gt_pos(p.rcutSq, d2)) {
             double en = lj64(p, d2);
             acc += nw ? en : -en;
-            if (nw && d2 < p.rcutLowSq)
+            if (nw && gt_pos(p.rcutLowSq, d2))
               ++ovl;
           }
         };
@@ -746,9 +773,9 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           const int bb = k < nt ? b1 : b;
           double d2 = r2_f64(M.tr[k][0], M.tr[k][1], M.tr[k][2], A.px[e.x],
                              A.py[e.x], A.pz[e.x], c.ax[bb], c.half[bb]);
-          if (d2 < p.rcutSq) {
+          if (gt_pos(p.rcutSq, d2)) {
             double en = lj64(p, d2);
-            bool lowr = d2 < p.rcutLowSq;
+            bool lowr = gt_pos(p.rcutLowSq, d2);
 #pragma unroll
             for (int u = 0; u < 4; ++u)
               if (u == e.y) {
@@ -900,7 +927,7 @@ __global__ void __launch_bounds__(GEMC_THREADS)
         auto eval = [&](int2 e) {  // e = (molecule, molecule)
           double d2 = r2_f64(A.qx[e.x], A.qy[e.x], A.qz[e.x], A.qx[e.y],
                              A.qy[e.y], A.qz[e.y], M.nax[bb], M.nhalf[bb]);
-          if (d2 < p.rcutSq)
+          if (gt_pos(p.rcutSq, d2))
             acc += lj64(p, d2);
         };
         for (int tl = gw; tl < ntile; tl += GW) {
@@ -961,28 +988,36 @@ __global__ void __launch_bounds__(GEMC_THREADS)
     }
     __syncthreads();
     mark(pslot, 1);
-    // this CTA's partials, warps in order (a transfer's trials went straight
-    // to their slots)
-    if (tid < nval && kind != GEMC_TRANSFER) {
-      double v = 0.0;
-      for (int w = 0; w < NW; ++w)
-        v += S.wred[w][tid];
-      S.part[par][tid] = v;
+    // this CTA's partials (a transfer's trials went straight to their
+    // slots): lanes 0-7 the warps' first value, 16-23 their second
+    if (warp == 0 && nval == 2) {
+      double v = (lane & 15) < NW ? S.wred[lane & 15][lane >> 4] : 0.0;
+      for (int o = NW / 2; o > 0; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((lane & 15) == 0)
+        S.part[par][lane >> 4] = v;
     }
     // ---------------- exchange: one cluster barrier ----------------
     cluster_barrier();
-    if (tid < nval) {
-      // the ranks' partials loaded together, added in rank order
-      double pr[16];
-#pragma unroll
-      for (int r = 0; r < 16; ++r)
-        pr[r] = r < C ? cluster.map_shared_rank(&S.part[par][0],
-                                                (unsigned)r)[tid]
-                      : 0.0;
-      double v = 0.0;
-      for (int r = 0; r < C; ++r)
-        v += pr[r];
-      M.tot[tid] = v;
+    // the ranks' partials, eight lanes a value: two ranks each, then folded
+    // (an FP64 addition takes 64 cycles: sixteen in a row were a third of
+    // this phase)
+    for (int k0 = 0; k0 < nval; k0 += GEMC_THREADS / 8) {
+      const int k = k0 + (tid >> 3), r = tid & 7;
+      if (k0 + (warp << 2) < nval) {  // a whole warp at a time
+        double v = 0.0, v2 = 0.0;
+        if (k < nval) {
+          if (r < C)
+            v = cluster.map_shared_rank(&S.part[par][0], (unsigned)r)[k];
+          if (r + 8 < C)
+            v2 = cluster.map_shared_rank(&S.part[par][0], (unsigned)(r + 8))[k];
+        }
+        v += v2;
+        for (int o = 4; o > 0; o >>= 1)
+          v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (r == 0 && k < nval)
+          M.tot[k] = v;
+      }
     }
     __syncthreads();
     mark(pslot, 2);
@@ -994,7 +1029,7 @@ __global__ void __launch_bounds__(GEMC_THREADS)
         if (M.ok) {
           double dLJ = M.tot[0];
           bool ovl = M.tot[1] > 0.0;
-          int res = M.u_acc < exp(-p.beta * (dLJ + 0.0 + 0.0));
+          int res = below_exp(M.u_acc, -p.beta * (dLJ + 0.0 + 0.0));
           acc = res && !ovl;
           if (lane == 0) {
             if (acc)
@@ -1016,20 +1051,28 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           for (int k = lane; k < 2 * nt; k += 32)
             wv[k] = exp(-1 * p.beta * ((0.0 + M.tot[k]) + 0.0));
           __syncwarp();
-          double stepWeight = 0.0;
-          for (int k = 0; k < nt; ++k)
-            stepWeight += wv[k];
-          // PRNG::PickWeighted (src/PRNG.h:167-200)
+          // running sums in trial order: lane 0 the new trials' (kept where
+          // the raw words were), lane 1 the old ones'
+          double *run = (double *)M.words;
+          const double *ws = wv + (lane == 1 ? nt : 0);
+          double sum = 0.0;
+          for (int k = 0; k < nt; ++k) {
+            sum += ws[k];
+            if (lane == 0)
+              run[k] = sum;
+          }
+          __syncwarp();
+          const double stepWeight = __shfl_sync(0xffffffffu, sum, 0);
+          // PRNG::PickWeighted (src/PRNG.h:167-200): the first running sum
+          // that reaches the draw
           double draw = ((double)M.pick_word * (1.0 / 4294967295.0)) *
                         stepWeight;
-          double s = 0.0;
           int winner = -1;
-          for (int k = 0; k < nt; ++k) {
-            s += wv[k];
-            if (s >= draw) {
-              winner = k;
-              break;
-            }
+          for (int k0 = 0; k0 < nt && winner < 0; k0 += 32) {
+            const unsigned hit = __ballot_sync(
+                0xffffffffu, k0 + lane < nt && run[k0 + lane] >= draw);
+            if (hit)
+              winner = k0 + __ffs(hit) - 1;
           }
           if (winner < 0) {
             int lastZero = nt;
@@ -1038,14 +1081,15 @@ __global__ void __launch_bounds__(GEMC_THREADS)
             winner = lastZero - 1;  // |draw - total| < 0.001 in practice
           }
           bool overlap = M.tot[2 * nt + winner] > 0.0;
-          double Wn = 1.0 * (stepWeight / nt);
-          double sumOld = 0.0;
-          for (int k = 0; k < nt; ++k)
-            sumOld += wv[nt + k];
-          double Wo = 1.0 * (sumOld / nt);
           double eNew = 0.0 + M.tot[winner], eOld = 0.0 + M.tot[nt];
           int nsrc = count_of(c, n, b), ndest = count_of(c, n, b1);
-          double coeff = (double)(nsrc) / (double)(ndest + 1) * c.vol[b1] *
+          // three divisions at once: lane 0 and 1 the mean weights, lane 2
+          // the ratio of the molecule counts
+          const double quo = (lane < 2 ? sum : (double)nsrc) /
+                             (lane < 2 ? (double)nt : (double)(ndest + 1));
+          const double Wn = __shfl_sync(0xffffffffu, quo, 0),
+                       Wo = __shfl_sync(0xffffffffu, quo, 1);
+          double coeff = __shfl_sync(0xffffffffu, quo, 2) * c.vol[b1] *
                          c.volInv[b];
           double Wrat = Wn / Wo * 1.0 * 1.0;
           if (Wn > SMALL_WEIGHT && !overlap)
