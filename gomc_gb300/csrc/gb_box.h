@@ -189,6 +189,9 @@ void recip_vectors(const double L[3], double volume, double alphaSq,
 // that take a DevBox run on that view (coordinates and cell grid), which lets
 // the MultiParticle move evaluate its trial state in separate buffers.
 int launch_grid_all(Box &b, const DevBox &d);
+// out[3 i + d] = (x, y, z)[d][i]
+int launch_interleave3(Box &b, const double *x, const double *y,
+                       const double *z, int n, double *out);
 int launch_box_inter(Box &b, double *d_out2);
 int launch_box_inter_view(Box &b, const DevBox &d, double *d_out2);
 int launch_box_virial(Box &b, double *d_out6);

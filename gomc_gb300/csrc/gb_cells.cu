@@ -6,6 +6,7 @@
 #include "gb_box.h"
 #include "gb_cells.cuh"
 
+#include <algorithm>
 #include <climits>
 
 namespace gb {
@@ -125,6 +126,23 @@ int launch_cell_remove_mol(Box &bx, int m) {
 int launch_cell_add_mol(Box &bx, int m) {
   k_cell_add_mol<<<1, 1, 0, bx.stream>>>(bx.dev, m, (int *)bx.h_pinned);
   return bx.CudaCheck(cudaGetLastError(), "cell add");
+}
+
+__global__ void k_interleave3(const double *__restrict__ x,
+                              const double *__restrict__ y,
+                              const double *__restrict__ z, int n, double *out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n;
+       i += gridDim.x * blockDim.x) {
+    const int a = i / 3, d = i - 3 * a;
+    out[i] = (d == 0 ? x : d == 1 ? y : z)[a];
+  }
+}
+
+int launch_interleave3(Box &bx, const double *x, const double *y,
+                       const double *z, int n, double *out) {
+  const int nb = std::min((int)((3LL * n + 255) / 256), 4 * bx.sm_count);
+  k_interleave3<<<nb, 256, 0, bx.stream>>>(x, y, z, n, out);
+  return bx.CudaCheck(cudaGetLastError(), "interleave");
 }
 
 int launch_grid_all(Box &bx, const DevBox &b) {
