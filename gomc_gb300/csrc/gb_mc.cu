@@ -344,21 +344,6 @@ __device__ __forceinline__ double2 cis_turns64(uint64_t phase) {
   }
 }
 
-// Neighbour nn of a cell (offsets dx, dy, dz in -1..1, dz fastest, each
-// axis wrapped): the entry of the 27-neighbour table Box::Init builds
-// (CellList::RebuildNeighbors order), computed instead of loaded.
-__device__ __forceinline__ int nbr_cell(const int *e, int cell, int nn) {
-  int z = cell % e[2], xy = cell / e[2];
-  int y = xy % e[1], x = xy / e[1];
-  x += nn / 9 - 1;
-  y += (nn / 3) % 3 - 1;
-  z += nn % 3 - 1;
-  x += x < 0 ? e[0] : (x >= e[0] ? -e[0] : 0);
-  y += y < 0 ? e[1] : (y >= e[1] ? -e[1] : 0);
-  z += z < 0 ? e[2] : (z >= e[2] ? -e[2] : 0);
-  return (x * e[1] + y) * e[2] + z;
-}
-
 __device__ __forceinline__ double2 cmul2(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }

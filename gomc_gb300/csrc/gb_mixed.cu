@@ -6,8 +6,8 @@
 //     32-bit fixed-point turns, the midpoint p = (r + r')/2 and the half step
 //     h = (r' - r)/2 of every atom) and per-axis phase rows exp(2 pi i n p/L)
 //     from the exact fixed-point phase;
-//   * evaluates its share of the real-space (atom, old/new, neighbour cell)
-//     units in FP32 from fixed-point coordinates -- the minimum image is the
+//   * evaluates its share of the real-space pairs, by neighbour cell of the
+//     moved atoms, in FP32 from fixed-point coordinates -- the minimum image is the
 //     wrapped 32-bit difference -- with an exact FP64 decision for pairs whose
 //     r^2 lies within 1e-5 of the cutoff;
 //   * evaluates its chunk of k-vectors with
@@ -82,20 +82,26 @@ struct MShared {
 // offsets.  Every array starts on a 16-byte boundary whatever the chunk
 // length.
 struct MixedLayout {
-  size_t kcs;   // padded chunk length (multiple of 4)
+  size_t kcs;   // padded chunk length (mixed_kcs)
   size_t cold;  // offset of the remainders (in shared memory or the buffer)
   size_t tab;   // offset of the phase rows in shared memory
 };
+// Padded chunk length; at least 512, since the changes dR/dI also hold the
+// real-space pair lists of a move (before that move's changes are formed).
+__host__ __device__ __forceinline__ size_t mixed_kcs(int kc_max) {
+  const size_t n = ((size_t)kc_max + 3) & ~(size_t)3;
+  return n > 512 ? n : 512;
+}
 __host__ __device__ __forceinline__ MixedLayout mixed_layout(int kc_max,
                                                              bool cold_smem) {
   MixedLayout L;
-  L.kcs = ((size_t)kc_max + 3) & ~(size_t)3;
+  L.kcs = mixed_kcs(kc_max);
   L.cold = 24 * L.kcs;
   L.tab = cold_smem ? L.cold + 8 * L.kcs : L.cold;
   return L;
 }
 __host__ __device__ __forceinline__ size_t mixed_cold_bytes(int kc_max) {
-  return 8 * (((size_t)kc_max + 3) & ~(size_t)3);
+  return 8 * mixed_kcs(kc_max);
 }
 
 // Whether cells c1 and c2 are in one another's 27-cell neighbourhood (every
@@ -142,6 +148,15 @@ __device__ __forceinline__ float fp32_bracket(float r2o, float r2n, float dr2,
     dal = -coul_da * (expf(-thi * thi) - expf(-tlo * tlo));
   }
   return fmaf(erfc_f32(thi), dinv, derfc * inv_o) + dal;
+}
+
+// the FP64 value of an FP32 sum without a conversion (an FP64 instruction)
+__device__ __forceinline__ double f64_of(float v) {
+  if (v == 0.0f)
+    return 0.0;
+  if (!(fabsf(v) > 1e-30f && fabsf(v) < 1e30f))
+    return (double)v;  // tiny, infinite or not a number
+  return widen_f64(v);
 }
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
@@ -191,39 +206,37 @@ __device__ void mixed_header(const MixedChain &C, MShared &S, int t,
                        : __ldcg(xs[d] + a0 + a);
   }
   __syncthreads();
-  if (threadIdx.x < na) {
-    int a = threadIdx.x;
-    double w[3];
-    if (rkind == 0) {
-      for (int d = 0; d < 3; ++d)
-        w[d] = wrap1(__dadd_rn(oldp[a][d], S.prop[d]), b.L[d]);
+  // FP64 work costs a warp 64 cycles an instruction however many lanes take
+  // part, so a lane has one coordinate and the parts are on warps of different
+  // sub-partitions: warp 0 the new positions with their turns and cells, warp
+  // 1 the old ones' (one thread per atom took three times the instructions)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ int axis_cell[2][MAXA][3];
+  if (warp < 2 && lane < 3 * na) {
+    const int a = lane / 3, d = lane % 3;
+    double w = oldp[a][d];
+    if (warp == 0) {
+      if (rkind == 0) {
+        w = wrap1(__dadd_rn(w, S.prop[d]), b.L[d]);
+      } else {
+        const unsigned act = __activemask();
+        const double v = __dadd_rn(unwrap1(w, com[d], b.L[d], b.half[d]), -com[d]);
+        const double v0 = __shfl_sync(act, v, 3 * a), v1 = __shfl_sync(act, v, 3 * a + 1),
+                     v2 = __shfl_sync(act, v, 3 * a + 2);
+        const double u = __dadd_rn(__dadd_rn(__dmul_rn(S.prop[3 * d], v0),
+                                             __dmul_rn(S.prop[3 * d + 1], v1)),
+                                   __dmul_rn(S.prop[3 * d + 2], v2));
+        w = wrap1(__dadd_rn(u, com[d]), b.L[d]);
+      }
+      h.newp[a][d] = w;
+      h.un[a][d] = to_turns(w, b.invL[d]);
     } else {
-      double v[3];
-      for (int d = 0; d < 3; ++d) {
-        v[d] = unwrap1(oldp[a][d], com[d], b.L[d], b.half[d]);
-        v[d] = __dadd_rn(v[d], -com[d]);
-      }
-      for (int i = 0; i < 3; ++i) {
-        double u = __dadd_rn(__dadd_rn(__dmul_rn(S.prop[3 * i], v[0]),
-                                       __dmul_rn(S.prop[3 * i + 1], v[1])),
-                             __dmul_rn(S.prop[3 * i + 2], v[2]));
-        w[i] = wrap1(__dadd_rn(u, com[i]), b.L[i]);
-      }
+      h.oldp[a][d] = w;
+      h.uo[a][d] = to_turns(w, b.invL[d]);
     }
-    for (int d = 0; d < 3; ++d) {
-      h.oldp[a][d] = oldp[a][d];
-      h.newp[a][d] = w[d];
-      uint32_t uo = to_turns(oldp[a][d], b.invL[d]);
-      uint32_t un = to_turns(w[d], b.invL[d]);
-      int32_t D = (int32_t)(un - uo);
-      h.uo[a][d] = uo;
-      h.un[a][d] = un;
-      h.P[a][d] = uo + (uint32_t)(D >> 1);
-      float Df = (float)D;  // pi / 2^32 as FP32 hi + lo
-      h.hf[a][d] = fmaf(Df, -2.03547013e-17f, Df * 7.31459060e-10f);
-    }
-    h.cell_old[a] = position_to_cell_fast(b, oldp[a][0], oldp[a][1], oldp[a][2]);
-    h.cell_new[a] = position_to_cell_fast(b, w[0], w[1], w[2]);
+    axis_cell[warp][a][d] = cell_axis(w, b.cellSize[d], b.invCell[d], b.edge[d]);
+  } else if (warp == 3 && lane < na) {
+    const int a = lane;
     double q = pre ? P.q[a] : b.q[a0 + a];
     bool q0 = fabs(q) < 0.000000001;
     h.qf[a] = q0 ? 0.0f : (float)q;
@@ -232,16 +245,30 @@ __device__ void mixed_header(const MixedChain &C, MShared &S, int t,
     h.qs[a] = q0 ? 0.0f : (float)qs;
     h.qslo[a] = q0 ? 0.0f : (float)(qs - (double)(float)qs);
     h.ka[a] = pre ? P.ka[a] : b.kind[a0 + a];
+  } else if (warp == 2 && lane < 3) {
+    if (lane == 0) {
+      h.m = m;
+      h.kind = rkind;
+      h.na = na;
+      h.a0 = a0;
+      h.lpacc = rlpacc;
+    }
+    h.newcom[lane] = rkind == 0
+                         ? wrap1(__dadd_rn(com[lane], S.prop[lane]), b.L[lane])
+                         : com[lane];
   }
-  if (threadIdx.x == 64) {
-    h.m = m;
-    h.kind = rkind;
-    h.na = na;
-    h.a0 = a0;
-    h.lpacc = rlpacc;
-    for (int d = 0; d < 3; ++d)
-      h.newcom[d] = rkind == 0 ? wrap1(__dadd_rn(com[d], S.prop[d]), b.L[d])
-                               : com[d];
+  __syncthreads();
+  if (threadIdx.x < 3 * na) {
+    const int a = threadIdx.x / 3, d = threadIdx.x % 3;
+    const uint32_t uo = h.uo[a][d], un = h.un[a][d];
+    int32_t D = (int32_t)(un - uo);
+    h.P[a][d] = uo + (uint32_t)(D >> 1);
+    float Df = (float)D;  // pi / 2^32 as FP32 hi + lo
+    h.hf[a][d] = fmaf(Df, -2.03547013e-17f, Df * 7.31459060e-10f);
+  } else if (threadIdx.x >= 32 && threadIdx.x < 32 + 2 * na) {
+    const int a = (threadIdx.x - 32) >> 1, side = (threadIdx.x - 32) & 1;
+    const int *x = axis_cell[side ? 0 : 1][a];
+    (side ? h.cell_new : h.cell_old)[a] = (x[0] * b.edge[1] + x[1]) * b.edge[2] + x[2];
   }
   __syncthreads();
 }
@@ -334,10 +361,6 @@ __global__ void __launch_bounds__(MT_THREADS)
   const float sy = (float)(b.L[1] * 2.3283064365386963e-10);
   const float sz = (float)(b.L[2] * 2.3283064365386963e-10);
   const bool coul_cut = ff.rcutCoulSq < ff.rcutSq;
-  const bool narrow = b.cellSize[0] * b.cellSize[0] < ff.rcutSq ||
-                      b.cellSize[1] * b.cellSize[1] < ff.rcutSq ||
-                      b.cellSize[2] * b.cellSize[2] < ff.rcutSq;
-
   // Warp 7 gathers the next move's header inputs one move ahead: the move
   // record two moves ahead, its atom range a move later, and at the start
   // of a move the proposal, centre, positions and charges of the next one,
@@ -412,32 +435,60 @@ __global__ void __launch_bounds__(MT_THREADS)
       cur_slot = __ldcg(b.atom_slot + h.a0 + threadIdx.x);
     }
     // ---------------- real space ----------------
-    // Each neighbour j is taken once: from the new position's cells when it
-    // is inside the cutoff there (then as the difference u(r') - u(r) if it
-    // was also inside before), from the old position's cells when it was
-    // inside only before.  Differences use r'^2 - r^2 = delta . (d + d').
+    // Each neighbour j of an atom is taken once: inside the cutoff at both
+    // positions as the difference u(r') - u(r), which uses r'^2 - r^2 =
+    // delta . (d + d').
     float lj_h = 0.f, lj_l = 0.f, re_h = 0.f, re_l = 0.f, ovl = 0.f;
-    const int units = na * 2 * NB27;
+    // The moved atoms' positions lie in one or two cells, whose neighbourhoods
+    // together hold every pair inside the cutoff (cells at least the cutoff
+    // wide, or three of them on an axis, which all are neighbours): units are
+    // the 27 neighbours of each distinct cell, less those of an earlier one,
+    // and each of their slots is loaded once and tested against every atom's
+    // two positions (a unit per atom, position and neighbour loaded and
+    // tested every slot six times for a water: 13,000 cycles a move).
+    int my_cell = -1 - (int)(threadIdx.x & 31);
+    if ((int)(threadIdx.x & 31) < 2 * na)
+      my_cell = (threadIdx.x & 1) ? h.cell_new[(threadIdx.x & 31) >> 1]
+                                  : h.cell_old[(threadIdx.x & 31) >> 1];
+    const unsigned alike = __match_any_sync(0xffffffffu, my_cell);
+    const unsigned lead = __ballot_sync(
+        0xffffffffu, my_cell >= 0 && __ffs(alike) - 1 == (int)(threadIdx.x & 31));
+    const int units = __popc(lead) * NB27;
     // a unit's neighbour-cell slots are tiled over ul threads: slot lu,
     // lu + ul, ... of unit usub of this CTA's upc units per pass
     const int ul = 1 << C.ulog, upc = MT_THREADS >> C.ulog;
     const int lu = threadIdx.x & (ul - 1), usub = threadIdx.x >> C.ulog;
     // the units' neighbour cells and slot counts, all at once
     __shared__ int mu_c2[2 * MAXA * NB27], mu_n2[2 * MAXA * NB27];
-    for (int u = threadIdx.x; u < units; u += MT_THREADS) {
-      int a = u / (2 * NB27), side = (u / NB27) % 2, nn = u % NB27;
-      int cell = side ? h.cell_new[a] : h.cell_old[a];
-      int c2 = b.nbr[cell * NB27 + nn];
-      mu_c2[u] = c2;
-      mu_n2[u] = __ldcg(b.cell_count + c2);
+    for (int u0 = 0; u0 < units; u0 += MT_THREADS) {
+      const int u = u0 + threadIdx.x, d = min(u / NB27, 2 * MAXA - 1);
+      unsigned rest = lead;
+      int cell = -1;
+      bool seen = false;
+      int c2 = 0;
+      // this unit's cell is the d-th leader's; the earlier ones' are compared
+      for (int e = 0; rest; ++e, rest &= rest - 1) {
+        const int ce = __shfl_sync(0xffffffffu, my_cell, __ffs(rest) - 1);
+        if (e == d) {
+          cell = ce;
+          if (u < units)
+            c2 = b.nbr[cell * NB27 + (u - d * NB27)];
+        }
+      }
+      rest = lead;
+      for (int e = 0; rest; ++e, rest &= rest - 1) {
+        const int ce = __shfl_sync(0xffffffffu, my_cell, __ffs(rest) - 1);
+        if (e < d && u < units)
+          seen = seen || cells_adjacent(b, ce, c2);
+      }
+      if (u < units) {
+        mu_c2[u] = c2;
+        mu_n2[u] = seen ? 0 : __ldcg(b.cell_count + c2);
+      }
     }
     __syncthreads();
-    // one candidate: unit u against cell slot s (meta mj, fixed-point slot f)
-    auto pair = [&](int u, size_t s, int mj, uint4 f) {
-      if (meta_mol(mj) == m)
-        return;
-      const int a = u / (2 * NB27), side = (u / NB27) % 2;
-      const int c2 = mu_c2[u];
+    // one candidate: atom a against cell slot s (meta mj, fixed-point slot f)
+    auto pair = [&](int a, size_t s, int mj, uint4 f) {
       const uint32_t *uo = h.uo[a], *un = h.un[a];
       const float ddx = (float)(int32_t)(un[0] - uo[0]) * sx;
       const float ddy = (float)(int32_t)(un[1] - uo[1]) * sy;
@@ -456,9 +507,7 @@ __global__ void __launch_bounds__(MT_THREADS)
       bool in_o = r2o < rc2, in_n = r2n < rc2;
       bool amb_o = fabsf(r2o - rc2) <= rc2 * 1e-5f;
       bool amb_n = fabsf(r2n - rc2) <= rc2 * 1e-5f;
-      bool amb_l = side && r2n < rl2 * 1.00001f;
-      if (side ? (!in_n && !amb_n) : (!in_o && !amb_o))
-        return;
+      bool amb_l = r2n < rl2 * 1.00001f;
       if (amb_o || amb_n || amb_l) {
         const double *pp = (const double *)(b.cell_pos + s);
         double px = __ldcg(pp), py = __ldcg(pp + 1), pz = __ldcg(pp + 2);
@@ -475,19 +524,12 @@ __global__ void __launch_bounds__(MT_THREADS)
                            min_image(mp[1] - py, b.L[1], b.half[1]),
                            min_image(mp[2] - pz, b.L[2], b.half[2]));
           in_n = ff.rcutSq > d2;
-          if (side && in_n && d2 < ff.rcutLowSq)
+          if (in_n && d2 < ff.rcutLowSq)
             ovl = 1.f;
         }
       }
-      // With cells narrower than the cutoff a pair inside it may lie
-      // outside the other position's neighbourhood, where it is not summed.
-      if (narrow && in_o && in_n &&
-          !cells_adjacent(b, c2, side ? h.cell_old[a] : h.cell_new[a])) {
-        if (side)
-          in_o = false;
-        else
-          in_n = false;
-      }
+      if (!in_o && !in_n)
+        return;
       int kj = meta_kind(mj);
       int idx = ka + kj * ff.n_kinds;
       // q_i q_j QQ_FACT / (1 + eta) = qq + qc up to FP32 rounding of the
@@ -506,9 +548,7 @@ __global__ void __launch_bounds__(MT_THREADS)
       bool cin_n = coul_cut ? r2n <= rcc2 : true;
       float sg2 = ff.sigmaSq_f[idx], ecn = ff.eps_cn_f[idx];
       float k6 = ff.lj_k6_f[idx], k3 = ff.lj_k3_f[idx];
-      if (side) {
-        if (!in_n)
-          return;
+      if (in_n) {
         if (in_o) {
           const int32_t o3[3] = {ox, oy, oz}, n3[3] = {nx_, ny_, nz_};
           if (r2o < ff.close_r2_f && r2n < ff.close_r2_f) {
@@ -576,8 +616,6 @@ __global__ void __launch_bounds__(MT_THREADS)
           }
         }
       } else {
-        if (!in_o || in_n)
-          return;  // counted from the new position's cells
         float rr2 = sg2 / r2o, r6 = rr2 * rr2 * rr2, r12 = r6 * r6;
         two_sum_add(lj_h, lj_l,
                     -ecn * ((r12 - r6) + fmaf(r12, k6, -r6 * k3)));
@@ -589,38 +627,173 @@ __global__ void __launch_bounds__(MT_THREADS)
       }
     };
     // This CTA takes units rank upc + usub, stepping upc csize; a thread
-    // takes slot lu of its unit (and lu + ul, ... in fuller cells).  The
-    // next unit's slot data are loaded while this one is evaluated.
+    // takes slots lu, lu + ul, ... of its unit.  One candidate in seven is
+    // inside the cutoff, and the pair terms are four branches of one to four
+    // hundred instructions each, which a warp of mixed pairs runs one after
+    // another (a batch took 10,000 cycles).  So the warps only test distances
+    // here and list the survivors (slot, and atom and class in a byte);
+    // the CTA's lists are then sorted by class, in warp and list order, and
+    // dealt to the warps in batches of one class, in rounds where the lists
+    // (they are where this move's dR/dI will be) fill up.  The pair terms
+    // stand in the code once: inlined also for the overflow of a list they
+    // cost more in instruction fetches than they saved.
+    constexpr int W8 = MT_THREADS / 32;
+    // per warp, at least 43; the sorted list has room for each class's padding
+    const int lcap = (int)((8 * L.kcs - 640) / (10 * W8));
+    unsigned *const wl = (unsigned *)dR + wid * lcap;
+    unsigned *const sorted = (unsigned *)dR + W8 * lcap;
+    unsigned char *const wtag =
+        (unsigned char *)(sorted + W8 * lcap + 128) + wid * lcap;
+    unsigned char *const stag =
+        (unsigned char *)(sorted + W8 * lcap + 128) + W8 * lcap;
+    __shared__ int lcnt[4][W8];
+    const unsigned lt = (1u << lid) - 1u;
+    // margins: the pairs decided in FP64 (1e-5), and turn differences cut to
+    // 23 bits here
+    const float marg = 2e-5f + 1e-6f * fmaxf(sx, fmaxf(sy, sz)) * 4294967296.0f *
+                                   rsqrtf(rc2);
+    const float rc2p = rc2 * (1.0f + marg), rc2m = rc2 * (1.0f - marg);
+    const float close_r2 = ff.close_r2_f, far_r2 = ff.far_r2_f;
+    const float qx = sx * 512.0f, qy = sy * 512.0f, qz = sz * 512.0f;
+    auto cut = [](uint32_t d) {  // a turn difference in units of 2^-23
+      return __int_as_float(0x4B400000 + ((int32_t)d >> 9)) - 12582912.0f;
+    };
     const int ustep = upc * csize;
-    int pu = -1, pmj = 0;
-    size_t ps = 0;
-    uint4 pfix = make_uint4(0, 0, 0, 0);
-    auto fetch = [&](int ub) {
-      int u = ub + usub;
-      pu = -1;
-      if (u < units && lu < mu_n2[u]) {
-        ps = (size_t)mu_c2[u] * b.cap + lu;
-        pmj = __ldcg(b.cell_meta + ps);
-        pfix = __ldcg(b.cell_fix + ps);
-        pu = u;
+    auto slots = [&](int v) { return v + usub < units ? mu_n2[v + usub] : 0; };
+    int ub = rank * upc, j = lu, mj = 0;
+    int n2 = ub < units ? slots(ub) : 0;
+    uint4 f = make_uint4(0, 0, 0, 0);
+    auto load = [&](int v, int jj, int cnt, int &meta, uint4 &fix) {
+      if (jj < cnt) {
+        const size_t s = (size_t)mu_c2[v + usub] * b.cap + jj;
+        meta = __ldcg(b.cell_meta + s);
+        fix = __ldcg(b.cell_fix + s);
       }
     };
-    fetch(rank * upc);
-    for (int ub = rank * upc; ub < units; ub += ustep) {
-      const int u = pu, mj = pmj;
-      const size_t s = ps;
-      const uint4 f = pfix;
-      if (ub + ustep < units)
-        fetch(ub + ustep);
-      if (u >= 0)
-        pair(u, s, mj, f);
-      const int uu = ub + usub;
-      if (uu < units)
-        for (int j = lu + ul; j < mu_n2[uu]; j += ul) {
-          size_t s2 = (size_t)mu_c2[uu] * b.cap + j;
-          pair(uu, s2, __ldcg(b.cell_meta + s2), __ldcg(b.cell_fix + s2));
+    load(ub, j, n2, mj, f);
+    // the next slots' data, loaded while these are tested
+    int vmj = 0, at = 0;
+    uint4 vf = make_uint4(0, 0, 0, 0);
+    auto ahead = [&]() {
+      int vb = ub, vj = j + ul, vn = n2;
+      if (!__any_sync(0xffffffffu, vj < vn)) {
+        vb = ub + ustep;
+        vj = lu;
+        vn = vb < units ? slots(vb) : 0;
+      }
+      load(vb, vj, vn, vmj, vf);
+    };
+    ahead();
+    do {
+      int ln = 0;  // warp-uniform list length
+      while (ub < units && ln + 32 <= lcap) {
+        bool in = false;
+        unsigned tag = 0;
+        if (j < n2 && meta_mol(mj) != m) {
+          const uint32_t *uo = h.uo[at], *un = h.un[at];
+          float x = cut(uo[0] - f.x) * qx, y = cut(uo[1] - f.y) * qy,
+                z = cut(uo[2] - f.z) * qz;
+          const float ro = fmaf(x, x, fmaf(y, y, z * z));
+          x = cut(un[0] - f.x) * qx;
+          y = cut(un[1] - f.y) * qy;
+          z = cut(un[2] - f.z) * qz;
+          const float rn = fmaf(x, x, fmaf(y, y, z * z));
+          in = rn < rc2p || ro < rc2p;
+          const unsigned cls = ro > rc2m || rn > rc2m                 ? 3u
+                               : fmaxf(ro, rn) < close_r2             ? 1u
+                               : fminf(ro, rn) < far_r2 || !ff.ewald  ? 0u
+                                                                      : 2u;
+          tag = cls | (unsigned)at << 2;
         }
-    }
+        const unsigned mask = __ballot_sync(0xffffffffu, in);
+        if (in) {
+          const int pos = ln + __popc(mask & lt);
+          wl[pos] = (unsigned)mu_c2[ub + usub] * b.cap + j;
+          wtag[pos] = (unsigned char)tag;
+        }
+        ln += __popc(mask);
+        if (++at == na) {  // the next slot
+          at = 0;
+          j += ul;
+          if (!__any_sync(0xffffffffu, j < n2)) {
+            ub += ustep;
+            j = lu;
+            n2 = ub < units ? slots(ub) : 0;
+          }
+          mj = vmj;
+          f = vf;
+          ahead();
+        }
+      }
+      __syncwarp();
+      // entries per class of this warp, then the place of each class and warp
+      int c4 = 0;  // lane c < 4: entries of class c
+      for (int i0 = 0; i0 < ln; i0 += 32) {
+        const unsigned cls = i0 + lid < ln ? wtag[i0 + lid] & 3u : 4u;
+#pragma unroll
+        for (unsigned c = 0; c < 4; ++c) {
+          const int k = __popc(__ballot_sync(0xffffffffu, cls == c));
+          if (lid == (int)c)
+            c4 += k;
+        }
+      }
+      if (lid < 4)
+        lcnt[lid][wid] = c4;
+      __syncthreads();
+      // lane 8 c + w holds warp w's count of class c
+      const int mine = lcnt[lid >> 3][lid & 7];
+      int incl = mine;
+      for (int o = 1; o < 8; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((lid & 7) >= o)
+          incl += v;
+      }
+      int start = 0, first = 0;
+      int cend[4];  // ends of the classes' entries
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int tot = __shfl_sync(0xffffffffu, incl, 8 * c + 7);
+        if (lid >> 3 == c)
+          first = start;
+        cend[c] = start + tot;
+        start += (tot + 31) & ~31;
+      }
+      const int nbatch = start / 32;
+      const int base = first + incl - mine;  // of class lid >> 3, warp lid & 7
+      int next[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        next[c] = __shfl_sync(0xffffffffu, base, 8 * c + wid);
+      for (int i0 = 0; i0 < ln; i0 += 32) {
+        const unsigned e = i0 + lid < ln ? wl[i0 + lid] : 0u;
+        const unsigned tag = i0 + lid < ln ? wtag[i0 + lid] : 255u;
+        const unsigned cls = i0 + lid < ln ? tag & 3u : 4u;
+#pragma unroll
+        for (unsigned c = 0; c < 4; ++c) {
+          const unsigned mask = __ballot_sync(0xffffffffu, cls == c);
+          if (cls == c) {
+            const int pos = next[c] + __popc(mask & lt);
+            sorted[pos] = e;
+            stag[pos] = (unsigned char)tag;
+          }
+          next[c] += __popc(mask);
+        }
+      }
+      __syncthreads();
+      for (int bt = wid; bt < nbatch; bt += W8) {
+        int end = cend[3];  // of the class this batch is of
+#pragma unroll
+        for (int c = 2; c >= 0; --c)
+          if (32 * bt < cend[c])
+            end = cend[c];
+        if (32 * bt + lid < end) {
+          const size_t s = sorted[32 * bt + lid];
+          const int tag = stag[32 * bt + lid];
+          pair(tag >> 2, s, __ldcg(b.cell_meta + s), __ldcg(b.cell_fix + s));
+        }
+      }
+      // the lists are free for another round, or for dR/dI
+    } while (__syncthreads_or(ub < units));
     // ---------------- reciprocal space ----------------
     float de_h = 0.f, de_l = 0.f;
     for (int i = threadIdx.x; i < kc; i += MT_THREADS) {
@@ -632,7 +805,18 @@ __global__ void __launch_bounds__(MT_THREADS)
         if (q == 0.f)
           continue;
         float arg = fmaf(fx, h.hf[a][0], fmaf(fy, h.hf[a][1], fz * h.hf[a][2]));
-        float sa = sin_f32(arg);
+        // mostly |k.h| < pi/4: the same polynomial without the reduction
+        float sa;
+        if (fabsf(arg) < 0.785f) {
+          const float x2 = arg * arg;
+          float ps = fmaf(x2, -2.5052108385e-8f, 2.7557319224e-6f);
+          ps = fmaf(x2, ps, -1.9841269841e-4f);
+          ps = fmaf(x2, ps, 8.3333333333e-3f);
+          ps = fmaf(x2, ps, -1.6666666667e-1f);
+          sa = fmaf(arg * x2, ps, arg);
+        } else {
+          sa = sin_f32(arg);
+        }
         float w = 2.0f * fmaf(h.qflo[a], sa, q * sa);
         const float2 *rx = tab + (size_t)(3 * a) * stride;
         float2 e = cmulf(cmulf(rx[n.x], tabf(rx + stride, n.y)),
@@ -660,16 +844,18 @@ __global__ void __launch_bounds__(MT_THREADS)
     int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
       for (int c = 0; c < 3; ++c)
-        S.wred[w][c] = (double)vh[c] + (double)vl[c];
-      S.wred[w][3] = v3;
+        S.wred[w][c] = f64_of(vh[c]) + f64_of(vl[c]);
+      S.wred[w][3] = v3 > 0.0f ? 1.0 : 0.0;
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
-      int c = threadIdx.x;
-      double acc = 0.0;
-      for (int i = 0; i < MT_THREADS / 32; ++i)
-        acc = c == 3 ? fmax(acc, S.wred[i][3]) : acc + S.wred[i][c];
-      S.part[c] = acc;
+    if (threadIdx.x < 32) {
+      // lane 8 c + w: warp w's value c, folded over the warps (three FP64
+      // additions of 64 cycles instead of eight); the overlaps just count
+      double v = S.wred[lid & 7][lid >> 3];
+      for (int o = 4; o > 0; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((lid & 7) == 0)
+        S.part[lid >> 3] = v;
     }
     // split cluster barrier: arrive with this CTA's partial, build the next
     // header meanwhile, wait before reading the other CTAs' partials
@@ -702,21 +888,22 @@ __global__ void __launch_bounds__(MT_THREADS)
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     // ---------------- decision (identical in every CTA) ----------------
     if (threadIdx.x < 32) {
-      double p[4] = {0, 0, 0, 0};
-      if ((int)threadIdx.x < csize) {
-        const double *rp = cluster.map_shared_rank(S.part, (unsigned)threadIdx.x);
-        for (int c = 0; c < 4; ++c)
-          p[c] = rp[c];
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        p[0] += __shfl_down_sync(0xffffffffu, p[0], o);
-        p[1] += __shfl_down_sync(0xffffffffu, p[1], o);
-        p[2] += __shfl_down_sync(0xffffffffu, p[2], o);
-        p[3] = fmax(p[3], __shfl_down_sync(0xffffffffu, p[3], o));
-      }
+      // lane 8 c + r: value c of ranks r and r + 8, folded over the ranks
+      const int c = lid >> 3, r = lid & 7;
+      double v = 0.0;
+      if (r < csize)
+        v = cluster.map_shared_rank(S.part, (unsigned)r)[c];
+      if (r + 8 < csize)
+        v += cluster.map_shared_rank(S.part, (unsigned)(r + 8))[c];
+      for (int o = 4; o > 0; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+      const double p0 = __shfl_sync(0xffffffffu, v, 0),
+                   p1 = __shfl_sync(0xffffffffu, v, 8),
+                   p2 = __shfl_sync(0xffffffffu, v, 16),
+                   p3 = __shfl_sync(0xffffffffu, v, 24);
       if (threadIdx.x == 0) {
-        bool over = p[3] > 0;
-        double dLJ = p[0], dRe = p[1], dRc = over ? 0.0 : p[2];
+        const bool over = nonzero(p3);
+        double dLJ = p0, dRe = p1, dRc = over ? 0.0 : p2;
         double ex = -ff.beta * ((dLJ + dRe) + dRc);
         int acc = !over && (ex > h.lpacc);
         if (acc) {
