@@ -1,9 +1,9 @@
 """The box-wide walks and sums -- BoxInter, BoxForce, VirialCalc, the
 structure factor and the reciprocal forces -- against the oracle, where their
-tiling can go wrong: boxes of three cells per axis, edges that differ, one
-molecule, atom counts around the warp, batch and tile sizes, molecules of one
-to eight sites, a Coulomb cutoff below Rcut, a Mie exponent other than 12,
-and no Ewald sum.
+tiling can go wrong: boxes of three cells per axis, edges that differ (one
+five times the others), one molecule, atom counts around the warp, batch and
+tile sizes, molecules of one to eight sites, a Coulomb cutoff below Rcut, a
+Mie exponent other than 12, and no Ewald sum.
 
 Bar: 1e-10 of the largest value of each output (of at least 1 K), the bar of
 the other FP64 tests.
@@ -72,6 +72,12 @@ CASES = {
     "tile_128": ((128, 0, 0), (24.0, 24.0, 24.0), {}),
     "tile_129": ((129, 0, 0), (24.0, 24.0, 24.0), {}),
     "many_sites": ((1, 900, 301), (45.0, 47.0, 49.0), {}),
+    # |n_z| and |n_x| to 41: more columns than one tile of the product has
+    "long_z": ((0, 60, 1), (20.0, 20.5, 101.0), {}),
+    "long_x": ((0, 60, 1), (101.0, 20.5, 20.0), {}),
+    # 33,024 atoms: more than one batch of the product, a molecule across it
+    "two_batches": ((32700, 100, 3), (109.0, 109.0, 110.0),
+                    dict(rcut=12.0, tolerance=1e-2)),
 }
 
 

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 from gomc_gb300.config import SimConfig
+from gomc_gb300.systems import AtomKind, MolSystem, MoleculeType
 from tests.test_gpu_box_sums import CASES, mixture
 
 pytestmark = pytest.mark.gpu
@@ -74,4 +75,48 @@ def test_points_against_oracle(gb, name):
             near(lj[i], l, "inter")
             near(re[i], r, "real")
     box.cell_add_mol(m)
+    box.close()
+
+
+def chains(length, n, edge, seed):
+    """n zigzag chains of `length` charged sites, 6 A apart."""
+    rng = np.random.default_rng(seed)
+    per = int(edge / 6.0)
+    i = np.arange(length)
+    one = np.stack([1.1 * (i % 16), 0.9 * (i // 16), 0.4 * (i % 2)], -1)
+    q = np.where(i % 2, 0.3, -0.3)
+    at = np.arange(n)
+    origin = np.stack([0 * at, at % per, at // per], -1) * 6.0
+    pos = origin[:, None] + one + rng.uniform(-.05, .05, (n, length, 3))
+    kinds = [AtomKind("A", 40.0, 2.6, 12.0), AtomKind("B", 0.0, 1.0, 12.0)]
+    kind = (i % 2).astype(np.int32)
+    t = MoleculeType("CH", ["X%d" % j for j in i], kind.tolist(), q.tolist())
+    return MolSystem(np.full(3, edge), kinds, [t],
+                     np.mod(pos.reshape(-1, 3), edge), np.tile(kind, n),
+                     np.tile(q, n), np.repeat(at, length).astype(np.int32),
+                     (np.arange(n + 1) * length).astype(np.int32),
+                     np.zeros(n, np.int32))
+
+
+# sites: the last of the 16-position call, the first beyond it, the first
+# whose positions need one CTA each, the largest molecule
+@pytest.mark.parametrize("length", [16, 17, 32, 33, 64])
+def test_long_molecules_against_oracle(gb, length):
+    from oracle import oracle as orc
+    edge = 36.0
+    cfg = SimConfig(temperature=298.0, rcut=9.0, tolerance=1e-5)
+    s = chains(length, 12, edge, 2)
+    box, ref = gb.Box(s, cfg), orc.OracleBox(s, cfg)
+    box.system_total()
+    tot = ref.system_total()
+    rng = np.random.default_rng(4)
+    for m in (0, 11):
+        old = ref.coords()[s.mol_start[m]:s.mol_start[m + 1]]
+        for shift in (rng.uniform(-0.3, 0.3, 3), np.array([3.0, 18.0, 15.0])):
+            new = np.mod(old + shift, edge)
+            got = box.molecule_inter(m, new) + (box.mol_reciprocal(m, new),)
+            want = ref.molecule_inter(m, new) + (ref.mol_reciprocal(m, new),)
+            assert got[0] == want[0]
+            for g, w, k in zip(got[1:], want[1:], ("inter", "real", "recip")):
+                assert abs(g - w) <= REL * max(abs(tot[k]), abs(w), 1.0), (k, g, w)
     box.close()
