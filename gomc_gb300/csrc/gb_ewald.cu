@@ -66,9 +66,9 @@ constexpr int ET = 512;      // threads that form the left operand
 constexpr int CW = 3;        // warps that copy the right operand
 constexpr int CTA = ET + 32 + 32 * CW;
 constexpr int NT_MAX = 64;   // columns per CTA: 7 x 64 of 512 TMEM columns
-constexpr int A_SLICE = TM * TK * 2;            // bytes
+constexpr int A_KO = TM * 16 + 32;              // bytes between 8-term groups
+constexpr int A_SLICE = TK / 8 * A_KO;          // bytes
 constexpr int A_STAGE = NSL * A_SLICE;
-constexpr int A_KO = TM * 16;                   // bytes between 8-term groups
 constexpr int BATCH = 32768;                    // atoms per pass (bounds scratch)
 constexpr unsigned WAIT_LIMIT = 1u << 22;       // polls of a barrier
 
@@ -475,15 +475,20 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
     // ---- the left operand, and the accumulators ----
-    const int a_row = FORCE ? tid & 127 : (warp & 3) * 32 + (warp >> 2) * 8 + (lane & 7);
-    const int a_ko = FORCE ? tid >> 7 : lane >> 3;
+    // sums: four lanes take the four term groups of a row, whose factors are
+    // 64 consecutive bytes: eight lanes then touch two lines (one row a lane
+    // touched eight and kept the L1 tags 84 % busy); the 32 bytes beyond a
+    // group's rows put the eight stores in different banks
+    const int a_sub = (warp >> 2) * 8 + (lane >> 2);
+    const int a_row = FORCE ? tid & 127 : (warp & 3) * 32 + a_sub;
+    const int a_ko = FORCE ? tid >> 7 : lane & 3;
     const int a_off = a_ko * A_KO + (a_row >> 3) * 128 + (a_row & 7) * 16;
     const int2 *yrow = A.yz, *zrow = A.yz + (size_t)2 * (A.kmax + 1) * A.nap;
     if constexpr (FORCE) {
       yrow += blockIdx.x * TM + a_row;
       zrow += blockIdx.x * TM + a_row;
     } else {
-      const int pr = A.pair[blockIdx.x * 32 + (warp >> 2) * 8 + (lane & 7)];
+      const int pr = A.pair[blockIdx.x * 32 + a_sub];
       const int comb = warp & 3;
       yrow += ((size_t)(pr & 255) * 2 + (comb >> 1)) * A.nap + 2 * a_ko + s0 * TK;
       zrow += ((size_t)((pr >> 8) & 255) * 2 + (comb & 1)) * A.nap + 2 * a_ko +
