@@ -115,7 +115,9 @@ __global__ void __launch_bounds__(RCT) k_reduce_cols(const double *__restrict__ 
 // ones (pair_split).  Measured on 8,000 waters, Rcut 10 A, against one CTA
 // per cell pair (energies, virial) or per third of a neighbour shell
 // (forces): the calls forces + reciprocal + torque 31.4 -> 24.6 ms, virial
-// 15.9 -> 12.7 ms; SystemTotal of 20,000 waters 72.9 -> 70.6 ms.
+// 15.9 -> 12.7 ms; SystemTotal of 20,000 waters 72.9 -> 70.6 ms.  Per launch
+// now: forces 774 us and virial 515 us (8,000 waters), energies 815 us
+// (20,000), the FP64 pipe 83 % busy (72-76 % with the last wave).
 // ---------------------------------------------------------------------------
 constexpr int PW = RT / 32;  // warps per CTA
 constexpr int PQ = 64;       // queue slots per warp: one batch plus a scan step
@@ -160,8 +162,18 @@ __device__ __forceinline__ bool scan_near(const Scan &s, const uint4 &a,
   return fmaf(dx * dx, s.sx, fmaf(dy * dy, s.sy, dz * dz * s.sz)) < s.cut;
 }
 
-// The exact separation of a batch's pairs; true where the pair is inside the
-// cutoff (act lanes only).
+// Whether r^2 from multiply-adds (within two units of the last place of
+// dsq3's) may fall on the other side of a cutoff than dsq3's.
+__device__ __forceinline__ bool beside(double distSq, double cut) {
+  return (unsigned long long)(bits64(distSq) - bits64(cut) + 8) <= 16;
+}
+
+// The separation of a batch's pairs; true where the pair is inside the
+// cutoff (act lanes only).  FAST: r^2 is three FP64 instructions instead of
+// dsq3's five, but every cutoff is decided as by dsq3 (the walks over a box,
+// which the FP64 pipe bounds: force walk of 8,000 waters 825 -> 774 us,
+// energies of 20,000 862 -> 815 us; with warp_sum4 at an atom's end).
+template <bool FAST>
 __device__ __forceinline__ bool pair_sep(const DevBox &b, const FF &ff, bool act,
                                          const double4_32a &pi,
                                          const double4_32a &pj, double v[3],
@@ -169,8 +181,13 @@ __device__ __forceinline__ bool pair_sep(const DevBox &b, const FF &ff, bool act
   v[0] = min_image_warp(pi.x - pj.x, b.L[0], b.half[0]);
   v[1] = min_image_warp(pi.y - pj.y, b.L[1], b.half[1]);
   v[2] = min_image_warp(pi.z - pj.z, b.L[2], b.half[2]);
-  *distSq = dsq3(v[0], v[1], v[2]);
-  return act && gt_pos(ff.rcutSq, *distSq);
+  double s;
+  if constexpr (FAST)
+    s = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2]));
+  if (!FAST || beside(s, ff.rcutSq) || beside(s, ff.rcutCoulSq))
+    s = dsq3(v[0], v[1], v[2]);
+  *distSq = s;
+  return act && gt_pos(ff.rcutSq, s);
 }
 
 // Whether a pair's Lennard-Jones terms can be other than zero: a zero
@@ -215,7 +232,7 @@ __device__ __forceinline__ void batch_energy(const DevBox &b, const FF &ff,
     idx = meta_kind(b.cell_meta[e.x]) + meta_kind(b.cell_meta[e.y]) * ff.n_kinds;
   }
   double v[3], distSq;
-  const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+  const bool in = pair_sep<true>(b, ff, act, pi, pj, v, &distSq);
   if (ff.electrostatic && in) {
     const double qq = pi.w * pj.w;
     if (nonzero(qq)) {
@@ -251,7 +268,7 @@ __device__ __forceinline__ void batch_virial(const DevBox &b, const FF &ff,
     mj = meta_mol(mj);
   }
   double v[3], distSq;
-  const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+  const bool in = pair_sep<true>(b, ff, act, pi, pj, v, &distSq);
   double w[3];
   w[0] = v[0] * min_image_warp(b.cx[mi] - b.cx[mj], b.L[0], b.half[0]);
   w[1] = v[1] * min_image_warp(b.cy[mi] - b.cy[mj], b.L[1], b.half[1]);
@@ -456,7 +473,7 @@ __global__ void __launch_bounds__(32 * PTW) k_points(DevBox b, const FF *__restr
       idx = ka + meta_kind(b.cell_meta[gj]) * ff.n_kinds;
     }
     double v[3], distSq;
-    const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+    const bool in = pair_sep<false>(b, ff, act, pi, pj, v, &distSq);
     ovl |= in && fresh && gt_pos(ff.rcutLowSq, distSq);
     if (ff.electrostatic && in) {
       const double qq = qi * pj.w;
@@ -730,7 +747,7 @@ __global__ void __launch_bounds__(RT) k_box_force(DevBox b, const FF *__restrict
         idx = ki + meta_kind(b.cell_meta[gj]) * ff.n_kinds;
       }
       double v[3], distSq;
-      const bool in = pair_sep(b, ff, act, pi, pj, v, &distSq);
+      const bool in = pair_sep<true>(b, ff, act, pi, pj, v, &distSq);
       double f = 0.0;
       const bool table = in && !gt_pos(distSq, ff.rcutCoulSq) && ff.ewald;
       if (ff.electrostatic && in) {
@@ -791,17 +808,10 @@ __global__ void __launch_bounds__(RT) k_box_force(DevBox b, const FF *__restrict
     if (qn > 0)
       eval(lane < qn, q[lane]);
     __syncwarp();  // the queue is read before the next atom fills it
-    for (int o = 16; o > 0; o >>= 1) {
-      fx += __shfl_down_sync(0xffffffffu, fx, o);
-      fy += __shfl_down_sync(0xffffffffu, fy, o);
-      fz += __shfl_down_sync(0xffffffffu, fz, o);
-    }
-    if (lane == 0) {
-      double *f = aF + 3 * (size_t)b.cell_atom[gi];
-      f[0] = fx;
-      f[1] = fy;
-      f[2] = fz;
-    }
+    const double v4[4] = {fx, fy, fz, 0.0};
+    const double f = warp_sum4(v4);
+    if ((lane & 7) == 0 && lane < 24)
+      aF[3 * (size_t)b.cell_atom[gi] + (lane >> 3)] = f;
   }
   __shared__ double red[PW];
   const double A = block_sum<RT>(lj, red);

@@ -121,3 +121,36 @@ def test_against_oracle(gb, name):
         near(mR, rR[1])
     near(box.virial(), ref.virial())
     box.close()
+
+
+def test_cutoff_to_the_last_bit(gb):
+    """216 isolated pairs whose r^2 is within a few units of the last place of
+    Rcut^2: each is inside or outside as the oracle's unfused r^2 has it (one
+    pair's terms are 1e-3 of the sums)."""
+    from oracle import oracle as orc
+    rng = np.random.default_rng(8)
+    edge, rc = 180.0, 9.0
+    g = np.arange(6) * 30.0 + 8.0
+    a = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    v = rng.normal(size=a.shape)
+    v *= rc / np.linalg.norm(v, axis=1)[:, None]
+    pos = np.mod(np.concatenate([a, a + v]), edge)
+    n = len(pos)
+    s = MolSystem(np.full(3, edge), [AtomKind("A", 70.0, 2.9, 12.0)],
+                  [MoleculeType("T", ["X"], [0], [0.0])], pos,
+                  np.zeros(n, np.int32), np.zeros(n),
+                  np.arange(n, dtype=np.int32),
+                  np.arange(n + 1, dtype=np.int32), np.zeros(n, np.int32))
+    cfg = SimConfig(temperature=298.0, rcut=rc, ewald=False,
+                    electrostatic=False)
+    box, ref = gb.Box(s, cfg), orc.OracleBox(s, cfg)
+    want = ref.system_total()["inter"]
+    one = abs(4 * 70.0 * (2.9 / rc) ** 6)
+    assert 20 * one < abs(want) < 196 * one  # some pairs on each side
+    near(box.system_total()["inter"], want)
+    aF, mF, lj, _ = box.box_force()
+    rF = ref.box_force()
+    near(aF, rF[0])
+    near(lj, rF[2])
+    near(box.virial(), ref.virial())
+    box.close()
