@@ -57,21 +57,28 @@ constexpr double TURN = 4294967296.0;
 
 constexpr int WQ = 96;  // per-warp queue of FP64 pair candidates
 
-// One move as warp 0 drew it, with what every warp needs of it in the
-// number formats its pair loop uses.
-struct Move {
+// One move as it was drawn, with what every warp needs of it in the number
+// formats its pair loop uses.  The head is kept twice, by move parity: a
+// displacement's can be drawn while the move before it is decided.
+struct MoveHead {
   int kind, b, b1, m, ok;
   double u_acc;            // acceptance uniform (displacement, volume)
-  unsigned pick_word;      // raw word of PickWeighted (transfer)
   double np[3], sh[3];     // displacement: new position; shift
   float nf[3];             // its FP32 copy
   unsigned nt[3];          // its fixed-point turns (mixed form)
+};
+struct Move {
+  unsigned pick_word;      // raw word of PickWeighted (transfer)
   double tr[2 * GEMC_NTMAX][3];     // transfer: new trials, then old trials
   float trf[2 * GEMC_NTMAX][3];
-  unsigned trt[2 * GEMC_NTMAX][3];
-  double nax[2][3], nhalf[2][3], nvol[2], nvolInv[2], sc[2][3];  // volume
-  float vcut[2];           // volume: FP32 pre-filter of the old distances
-  float nlt[2][3];         // volume: FP32 turn lengths at the new edges
+  union {                  // (the second head takes no more than this saves)
+    unsigned trt[2 * GEMC_NTMAX][3];
+    struct {
+      double nax[2][3], nhalf[2][3], nvol[2], nvolInv[2], sc[2][3];  // volume
+      float vcut[2];       // volume: FP32 pre-filter of the old distances
+      float nlt[2][3];     // volume: FP32 turn lengths at the new edges
+    };
+  };
   double d[4];             // values reported in the trace
   double tot[PMAX];        // cluster sums of the partials
   // raw words of a transfer's build; then its running weight sums
@@ -81,6 +88,7 @@ struct Move {
 
 struct GemcShared {
   GemcCtl c;
+  MoveHead head[2];           // by move parity
   Move mv;
   float axf[2][3], halff[2][3], ltf[2][3];  // FP32 edges, half edges, turns
   float pcut[2];  // FP32 distance pre-filter (FP64 form): Rcut with room
@@ -89,6 +97,7 @@ struct GemcShared {
   double wred[NW][2];         // per-warp sums (displacement, volume)
   int2 wq[NW][WQ];            // per-warp FP64 candidate queues
   int accept;
+  int pre_ok, pre_left, pre_next;  // a head drawn ahead; its MT19937 cursor
   int slot;                   // a transferred molecule's slot in the lookup
 };
 
@@ -270,10 +279,9 @@ __device__ void settings_update(GemcCtl &c, int k, int acc, int b) {
   }
 }
 
-// MoveSettings::AdjustMoves / Adjust (src/MoveSettings.cpp:147-238)
-__device__ void settings_adjust(GemcCtl &c, long long step, int adj) {
-  if ((step + 1) % adj != 0)
-    return;
+// MoveSettings::AdjustMoves / Adjust (src/MoveSettings.cpp:147-238), at the
+// last step of each AdjSteps
+__device__ void settings_adjust(GemcCtl &c) {
   for (int b = 0; b < 2; ++b)
     for (int k = 0; k < 3; ++k) {
       // slots: displacement (counter 0), rotation (no tries), volume (2)
@@ -442,9 +450,104 @@ __device__ __forceinline__ void qflush(int2 *q, int &qn, bool all, int lane,
   }
 }
 
-__device__ __forceinline__ void cluster_barrier() {
+__device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
+}
+
+// The next move, if it is a displacement or a transfer: the same words and
+// arithmetic as the drawing code of k_gemc, its first words one a lane.  Sets
+// S.pre_ok and, where that is 1, the head, a transfer's trials (in S.mv, which
+// a displacement does not use) and the generator's cursor after the move;
+// returns a displaced molecule's centre in lanes 0-2 of CTA 0.
+template <bool MIXED>
+__device__ double draw_ahead(const GemcParams &p, GemcShared &S,
+                             const Arrays<MIXED> &A, MoveHead &D, int n,
+                             int lane, int rank) {
+  const GemcCtl &c = S.c;
+  const int left = c.mt_left, next = c.mt_next;
+  int ok = 0, b = 0, m = -1, used = 0, kind = -1;
+  const int nt = p.nt;
+  double centre = 0.0;
+  if (left >= 32) {
+    const unsigned w = MtCursor::temper(c.mt[next + lane]);
+    const double r01 = (double)w * (1.0 / 4294967295.0);
+    const double draw = __shfl_sync(0xffffffffu, r01, 0) * 1.0;
+    const unsigned bal = __ballot_sync(0xffffffffu, lane < GEMC_KINDS &&
+                                                        p.cum[lane] >= draw);
+    kind = bal ? __ffs(bal) - 1 : GEMC_KINDS - 1;
+    if (kind == GEMC_DISPLACE || kind == GEMC_TRANSFER) {
+      const double subDraw = draw - (kind > 0 ? p.cum[kind - 1] : 0.0);
+      b = subDraw >= p.boxdiv[kind] ? 1 : 0;
+      const int nb = count_of(c, n, b);
+      if (nb > 0) {
+        // randInt(nb - 1): the first word whose masked value is in range
+        const unsigned top = (unsigned)nb - 1u;
+        const unsigned mask = top ? 0xffffffffu >> __clz(top) : 0u;
+        const unsigned hit =
+            __ballot_sync(0xffffffffu, lane > 0 && (w & mask) <= top);
+        const int at = hit ? __ffs(hit) - 1 : 32;
+        used = at + (kind == GEMC_DISPLACE ? 5 : 6 * nt + 3);
+        ok = kind == GEMC_DISPLACE ? used <= 32 : at < 32 && used <= left;
+        if (ok)
+          m = A.lookup[first_of(c, b) + (__shfl_sync(0xffffffffu, w, at) & mask)];
+        if (ok && kind == GEMC_DISPLACE) {
+          const double u = __shfl_sync(0xffffffffu, r01, (at + 1 + lane) & 31);
+          if (lane < 3) {
+            const double bound = c.scale[b][0], bound2 = 2.0 * bound;
+            const double sh = u * bound2 - bound;
+            const double pv = lane == 0 ? A.px[m] : lane == 1 ? A.py[m] : A.pz[m];
+            const double nv = wrapd(pv + sh, c.ax[b][lane]);
+            D.np[lane] = nv;
+            D.sh[lane] = sh;
+            D.nf[lane] = (float)nv;
+            if (MIXED)
+              D.nt[lane] = turns(nv, 1.0 / c.ax[b][lane]);
+            if (rank == 0)
+              centre = lane == 0 ? p.cx[m] : lane == 1 ? p.cy[m] : p.cz[m];
+          } else if (lane == 3) {
+            D.u_acc = u;
+          }
+        } else if (ok) {
+          // after the direction's word: 3 nt words, PickWeighted's, 3 nt
+          Move &M = S.mv;
+          const unsigned *src = c.mt + next + at + 2;
+          for (int q = lane; q < 6 * nt; q += 32) {
+            const int k = q / 3, d = q - 3 * k;
+            const int bb = k < nt ? 1 - b : b;
+            const unsigned wq = MtCursor::temper(src[q < 3 * nt ? q : q + 1]);
+            double v = (double)wq * (1.0 / 4294967296.0) * c.ax[bb][d];
+            if (k == nt)
+              v = wrapd(d == 0 ? A.px[m] : d == 1 ? A.py[m] : A.pz[m],
+                        c.ax[b][d]);
+            M.tr[k][d] = v;
+            M.trf[k][d] = (float)v;
+            if (MIXED)
+              M.trt[k][d] = turns(v, 1.0 / c.ax[bb][d]);
+          }
+          if (lane == 0)
+            M.pick_word = MtCursor::temper(src[3 * nt]);
+        }
+      }
+    }
+  }
+  if (lane == 0) {
+    S.pre_ok = ok;
+    S.pre_left = left - used;
+    S.pre_next = next + used;
+    D.kind = kind;
+    D.b = b;
+    D.b1 = 1 - b;
+    D.m = m;
+    D.ok = 1;
+  }
+  return centre;
 }
 
 // The Gibbs-ensemble loop (src/moves/*.h of the GEMC build; the move
@@ -514,14 +617,24 @@ __global__ void __launch_bounds__(GEMC_THREADS)
   };
   Move &M = S.mv;
 
-  double cpend = 0.0;  // CTA 0, warp 0, lanes 0-2: a displaced centre
-  for (int t = 0; t < p.nsteps; ++t) {
-    const long long step = p.first + t;
+  // CTA 0, lanes 0-2 of the drawing warp: a displaced centre; and that of
+  // the move drawn ahead
+  double cpend = 0.0, cnext = 0.0;
+  bool drawn = false;  // this move's head was drawn ahead (the last warp)
+  // steps to the next settings adjustment (0: before this move)
+  int to_adj = (int)(p.adj - 1 - p.first % p.adj);
+  for (int t = 0; t < p.nsteps; ++t, to_adj = to_adj ? to_adj - 1 : p.adj - 1) {
     const int par = t & 1;
+    MoveHead &D = S.head[par];
     // ---------------- draw the move (warp 0) ----------------
-    if (warp == 0) {
-      if (lane == 0)
-        settings_adjust(c, step, p.adj);
+    if (drawn) {
+      if (tid == 0) {
+        c.mt_left = S.pre_left;
+        c.mt_next = S.pre_next;
+      }
+    } else if (warp == 0) {
+      if (lane == 0 && to_adj == 0)
+        settings_adjust(c);
       __syncwarp();
       MtCursor R{c.mt, c.mt_left, c.mt_next};
       // System::PickMove: PRNG::PickArbDist (Wt = 1) walks the running sums
@@ -564,16 +677,16 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           const double sh = (double)w * (1.0 / 4294967295.0) * bound2 - bound;
           const double pv = lane == 0 ? A.px[m] : lane == 1 ? A.py[m] : A.pz[m];
           const double nv = wrapd(pv + sh, c.ax[b][lane]);
-          M.np[lane] = nv;
-          M.sh[lane] = sh;
-          M.nf[lane] = (float)nv;
+          D.np[lane] = nv;
+          D.sh[lane] = sh;
+          D.nf[lane] = (float)nv;
           if (MIXED)
-            M.nt[lane] = turns(nv, 1.0 / c.ax[b][lane]);
+            D.nt[lane] = turns(nv, 1.0 / c.ax[b][lane]);
           if (rank == 0)  // the centres are CTA 0's (global memory): the
                           // load is consumed at the commit
             cpend = lane == 0 ? p.cx[m] : lane == 1 ? p.cy[m] : p.cz[m];
         } else if (lane == 3) {
-          M.u_acc = (double)w3 * (1.0 / 4294967295.0);
+          D.u_acc = (double)w3 * (1.0 / 4294967295.0);
         }
       } else if (kind == GEMC_TRANSFER && ok) {
         // DCLinear::Build: direction, DCSingle::BuildNew (trials in the
@@ -650,31 +763,33 @@ __global__ void __launch_bounds__(GEMC_THREADS)
         if (!c.err) {
           double u = R.rand01();
           if (lane == 0)
-            M.u_acc = u;
+            D.u_acc = u;
         }
       }
       if (lane == 0) {
-        M.kind = kind;
-        M.b = b;
-        M.b1 = b1;
-        M.m = m;
-        M.ok = ok;
+        D.kind = kind;
+        D.b = b;
+        D.b1 = b1;
+        D.m = m;
+        D.ok = ok;
         M.pick_word = pick_word;
         c.mt_left = R.left;
         c.mt_next = R.next;
       }
     }
-    __syncthreads();
-    if (c.err)
-      break;  // every CTA drew the same volume change
-    const int kind = M.kind, b = M.b, b1 = M.b1, m = M.m;
+    if (!drawn) {
+      __syncthreads();
+      if (c.err)
+        break;  // every CTA drew the same volume change
+    }
+    const int kind = D.kind, b = D.b, b1 = D.b1, m = D.m;
     const int pslot = kind == GEMC_DISPLACE ? 0 : kind == GEMC_TRANSFER ? 1
                       : kind == GEMC_VOLUME ? 2 : -1;
     mark(pslot, 0);
     int nval = 0;
     int2 *q = S.wq[warp];
     // ---------------- energy phase (all CTAs) ----------------
-    if (kind == GEMC_DISPLACE && M.ok) {
+    if (kind == GEMC_DISPLACE && D.ok) {
       // Translate::CalcEn -> MoleculeInter (the molecule out of the cell
       // list): this CTA's slice of the box's molecules
       nval = 2;
@@ -684,9 +799,9 @@ __global__ void __launch_bounds__(GEMC_THREADS)
       if (!MIXED) {
         const float *L = S.axf[b], *H = S.halff[b];
         const float ofx = A.fx[m], ofy = A.fy[m], ofz = A.fz[m];
-        const float nfx = M.nf[0], nfy = M.nf[1], nfz = M.nf[2];
+        const float nfx = D.nf[0], nfy = D.nf[1], nfz = D.nf[2];
         const double opx = A.px[m], opy = A.py[m], opz = A.pz[m];
-        const double npx = M.np[0], npy = M.np[1], npz = M.np[2];
+        const double npx = D.np[0], npy = D.np[1], npz = D.np[2];
         double acc = 0.0;
         int ovl = 0, qn = 0;
         const float pc = S.pcut[b];
@@ -731,7 +846,7 @@ __global__ void __launch_bounds__(GEMC_THREADS)
       } else {
         const float *lt = S.ltf[b];
         const unsigned otx = A.tx[m], oty = A.ty[m], otz = A.tz[m];
-        const unsigned ntx = M.nt[0], nty = M.nt[1], ntz = M.nt[2];
+        const unsigned ntx = D.nt[0], nty = D.nt[1], ntz = D.nt[2];
         float sh = 0.0f, sl = 0.0f;
         int ovl = 0;
         for (int i = lo + tid; i < hi; i += GEMC_THREADS) {
@@ -758,7 +873,7 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           S.wred[warp][1] = (double)ovl;
         }
       }
-    } else if (kind == GEMC_TRANSFER && M.ok) {
+    } else if (kind == GEMC_TRANSFER && D.ok) {
       // CalculateEnergy::ParticleInter of each trial (the molecule is out of
       // its box's cell list): new trials in the destination box, old trials
       // in the source box; warp w takes trials w, w + 8, ... over this
@@ -998,7 +1113,20 @@ __global__ void __launch_bounds__(GEMC_THREADS)
         S.part[par][lane >> 4] = v;
     }
     // ---------------- exchange: one cluster barrier ----------------
-    cluster_barrier();
+    cluster_arrive();
+    // A displacement draws no more words, so the next move can be drawn
+    // while this one's sums meet and are decided: by the last warp, which has
+    // no part in either (drawing takes 2.1 us of some 30 dependent FP64
+    // instructions; 2,400 + 300 spheres, 1,000 moves: 9.0 -> 7.9 ms with
+    // displacements drawn ahead).  Not a volume exchange, and not
+    // across a settings adjustment or the end of the generator's block; the
+    // draw is thrown away if this move turns out to have moved the same
+    // molecule.
+    const bool ahead = kind == GEMC_DISPLACE && t + 1 < p.nsteps && to_adj != 1 &&
+                       p.adj > 1;
+    if (ahead && warp == NW - 1)
+      cnext = draw_ahead<MIXED>(p, S, A, S.head[par ^ 1], n, lane, rank);
+    cluster_wait();
     // the ranks' partials, eight lanes a value: two ranks each, then folded
     // (an FP64 addition takes 64 cycles: sixteen in a row were a third of
     // this phase)
@@ -1019,17 +1147,20 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           M.tot[k] = v;
       }
     }
-    __syncthreads();
+    if (kind == GEMC_DISPLACE)
+      __syncwarp();  // its two sums are warp 0's, which decides
+    else
+      __syncthreads();
     mark(pslot, 2);
     // ---------------- decision (identical in every CTA) ----------------
     if (warp == 0) {
       MtCursor R{c.mt, c.mt_left, c.mt_next};
       int acc = 0;
       if (kind == GEMC_DISPLACE) {
-        if (M.ok) {
+        if (D.ok) {
           double dLJ = M.tot[0];
           bool ovl = M.tot[1] > 0.0;
-          int res = below_exp(M.u_acc, -p.beta * (dLJ + 0.0 + 0.0));
+          int res = below_exp(D.u_acc, -p.beta * (dLJ + 0.0 + 0.0));
           acc = res && !ovl;
           if (lane == 0) {
             if (acc)
@@ -1044,7 +1175,7 @@ __global__ void __launch_bounds__(GEMC_THREADS)
           M.d[0] = M.d[1] = M.d[2] = M.d[3] = 0.0;
         }
       } else if (kind == GEMC_TRANSFER) {
-        if (M.ok) {
+        if (D.ok) {
           // the Boltzmann weights of all trials, one lane each, then added
           // in trial order
           double *wv = M.wts;
@@ -1103,9 +1234,9 @@ __global__ void __launch_bounds__(GEMC_THREADS)
               c.e[b] -= eOld;
               c.e[b1] += eNew;
               for (int d = 0; d < 3; ++d) {
-                M.np[d] = M.tr[winner][d];
-                M.nf[d] = M.trf[winner][d];
-                M.nt[d] = M.trt[winner][d];
+                D.np[d] = M.tr[winner][d];
+                D.nf[d] = M.trf[winner][d];
+                D.nt[d] = M.trt[winner][d];
               }
             }
             settings_update(c, 1, acc, b1);
@@ -1125,7 +1256,7 @@ __global__ void __launch_bounds__(GEMC_THREADS)
         double tNew = (0.0 + en0) + en1;
         double tRef = (0.0 + c.e[0]) + c.e[1];
         double uBoltz = exp(-p.beta * (tNew - tRef));
-        acc = M.u_acc < coeff * uBoltz;
+        acc = D.u_acc < coeff * uBoltz;
         if (lane == 0) {
           M.d[0] = en0;
           M.d[1] = en1;
@@ -1136,8 +1267,10 @@ __global__ void __launch_bounds__(GEMC_THREADS)
       }
       if (lane == 0) {
         S.accept = acc;
-        c.mt_left = R.left;
-        c.mt_next = R.next;
+        if (kind != GEMC_DISPLACE) {  // drew nothing, and is being read
+          c.mt_left = R.left;
+          c.mt_next = R.next;
+        }
       }
     }
     __syncthreads();
@@ -1156,26 +1289,26 @@ __global__ void __launch_bounds__(GEMC_THREADS)
     }
     if (acc && (kind == GEMC_DISPLACE || kind == GEMC_TRANSFER)) {
       if (tid == 0) {
-        A.px[m] = M.np[0];
-        A.py[m] = M.np[1];
-        A.pz[m] = M.np[2];
+        A.px[m] = D.np[0];
+        A.py[m] = D.np[1];
+        A.pz[m] = D.np[2];
         if (!MIXED) {
-          A.fx[m] = M.nf[0];
-          A.fy[m] = M.nf[1];
-          A.fz[m] = M.nf[2];
+          A.fx[m] = D.nf[0];
+          A.fy[m] = D.nf[1];
+          A.fz[m] = D.nf[2];
         } else {
-          A.tx[m] = M.nt[0];
-          A.ty[m] = M.nt[1];
-          A.tz[m] = M.nt[2];
+          A.tx[m] = D.nt[0];
+          A.ty[m] = D.nt[1];
+          A.tz[m] = D.nt[2];
         }
         if (kind == GEMC_DISPLACE) {
           // the centre: below, by the lanes that loaded it
         } else {
           // COM::SetNew of one atom; MoleculeLookup::Shift
           if (rank == 0) {
-            p.cx[m] = wrapd(M.np[0] * (1.0 / 1.0), c.ax[b1][0]);
-            p.cy[m] = wrapd(M.np[1] * (1.0 / 1.0), c.ax[b1][1]);
-            p.cz[m] = wrapd(M.np[2] * (1.0 / 1.0), c.ax[b1][2]);
+            p.cx[m] = wrapd(D.np[0] * (1.0 / 1.0), c.ax[b1][0]);
+            p.cy[m] = wrapd(D.np[1] * (1.0 / 1.0), c.ax[b1][1]);
+            p.cz[m] = wrapd(D.np[2] * (1.0 / 1.0), c.ax[b1][2]);
           }
           const int idx = S.slot;
           int ni = b == 0 ? --c.start1 : c.start1++;
@@ -1188,9 +1321,10 @@ __global__ void __launch_bounds__(GEMC_THREADS)
         }
       }
     }
-    if (acc && kind == GEMC_DISPLACE && rank == 0 && warp == 0 && lane < 3) {
+    if (acc && kind == GEMC_DISPLACE && rank == 0 &&
+        warp == (drawn ? NW - 1 : 0) && lane < 3) {
       double *cc = lane == 0 ? p.cx : lane == 1 ? p.cy : p.cz;
-      cc[m] = wrapd(cpend + M.sh[lane], c.ax[b][lane]);
+      cc[m] = wrapd(cpend + D.sh[lane], c.ax[b][lane]);
     }
     if (acc && kind == GEMC_VOLUME) {
       // new positions, centres and axes
@@ -1245,6 +1379,9 @@ __global__ void __launch_bounds__(GEMC_THREADS)
       td[6] = c.vol[0];
       td[7] = c.vol[1];
     }
+    drawn = ahead && S.pre_ok && !(acc && S.head[par ^ 1].m == m);
+    if (drawn)
+      cpend = cnext;
     __syncthreads();
     mark(pslot, 4);
     if (prof && pslot >= 0)

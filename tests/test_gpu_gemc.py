@@ -121,3 +121,32 @@ def test_gemc_continues_across_launches(gb):
     np.testing.assert_array_equal(a.state()["energy"], b.state()["energy"])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("mixed", [0, 1])
+@pytest.mark.parametrize("n0,n1,adj", [(1, 1, 1), (2, 1, 2), (9, 4, 3),
+                                       (200, 40, 50)])
+def test_gemc_moves_drawn_ahead(gb, mixed, n0, n1, adj):
+    """A launch of many steps draws moves while the ones before are decided, a
+    launch of one step cannot: both give the same run, bit for bit, also where
+    the next move often takes the same molecule, the settings change every
+    step, and the generator's block ends."""
+    from gomc_gb300.systems import lj_sphere_box
+    s0 = lj_sphere_box(n0, 30.0, seed=3, epsilon=148.0, sigma=3.73, min_sep=2.4,
+                       name="LJ")
+    s1 = lj_sphere_box(n1, 34.0, seed=4, epsilon=148.0, sigma=3.73, min_sep=2.4,
+                       name="LJ")
+    g = [gb.Gemc(s0.pos, s1.pos, s0.box, s1.box, 148.0, 3.73, 12.0, 150.0, 12.0,
+                 17, (0.8, 0.01, 0.19), adj, 10, precision=mixed)
+         for _ in range(2)]
+    n = 300
+    one = g[0].run(n, trace=True)
+    many = [g[1].run(1, trace=True) for _ in range(n)]
+    assert {0, 10} <= set(one["kind"].tolist())
+    for key in one:
+        np.testing.assert_array_equal(
+            one[key], np.concatenate([r[key] for r in many]), key)
+    for a, b in zip(g[0].coords(), g[1].coords()):
+        np.testing.assert_array_equal(a, b)
+    for h in g:
+        h.close()
