@@ -2093,8 +2093,10 @@ int mc_init(Box &b, const gb_mc_params &p) {
       return rc;
     // threads per real-space unit: as asked, else the smallest of 32, 64,
     // 128 that covers a cell's mean occupancy in one pass, 128 above that
-    // (timed on SPC/E water at Rcut 9-10 A: 64 lanes at 56 atoms per cell,
-    // 128 at 94 and 111; 256 was slower at each)
+    // (SPC/E water, Rcut 9-10 A, us per 100 moves at 64 / 128 / 256 lanes:
+    // 16 chains of 500, 56 atoms per cell, 3,247 / 4,450 / - (32: 3,309); 36
+    // chains of 8,000, 111 per cell, 3,827 / 3,477 / 3,608; 4 chains of 20,000,
+    // 3,041 / 2,872 / 2,896)
     int lanes = p.unit_lanes;
     if (lanes == 0) {
       const double cells = (double)b.dev.edge[0] * b.dev.edge[1] * b.dev.edge[2];

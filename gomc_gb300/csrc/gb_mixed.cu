@@ -22,6 +22,17 @@
 // FP32 remainder, about 48 bits) in shared memory, updated by an error-free
 // sum on every accepted move; they are read from and written back to the
 // box's FP64 arrays at launch boundaries.  Running energies are FP64.
+//
+// A move is a chain of latencies (36 chains of 8,000 waters, eight CTAs each,
+// two CTAs an SM, cycles of a move: unit counts 3,700, scan and sort 9,000,
+// pair terms 5,500, k-vectors 9,400, sums and barrier with the next header
+// 9,000, decision and commit 4,000, closing barrier 3,500), so what is not
+// needed before a load is issued is done elsewhere: the pairs are listed by
+// branch, the next move's units are listed by the warps that wait for the
+// decision, the hot part of the descriptor is in shared memory, two k-vectors
+// are in flight a thread, and settings adjustments are counted, not divided.
+// A pass of 100 moves: these 36 chains 9.3 -> 6.4 ms (3 ms of it reading the
+// coordinates back), twelve chains of 500 to 20,000 waters 6.7 -> 4.0 ms.
 #include "gb_cells.cuh"
 #include "gb_f32math.cuh"
 #include "gb_mc.h"
@@ -59,15 +70,32 @@ struct MPre {
   int ka[MAXA];
 };
 
+// What a move reads of the chain's descriptor, kept in shared memory: after
+// every cluster barrier a plain load of it would go to L2 and hold up the
+// loads that need it.
+struct MHot {
+  double L[3], half[3], invL[3], cellSize[3], invCell[3];
+  double *x, *y, *z, *cx, *cy, *cz;
+  const double *q;
+  const int *kind, *mstart, *nbr, *cell_count, *cell_meta, *atom_cell,
+      *atom_slot;
+  const uint4 *cell_fix;
+  const MoveRec *moves;
+  double *prop;
+  long long first;
+  int edge[3], cap, n, ulog;
+  int next_mol[2];  // the molecule of the move after a move, by its parity
+};
+
 struct MShared {
   MHdr hh[2];  // this move's header and the next one's, by move parity
   MPre pre;
+  MHot hot;
   Settings set;
   double e_run[5];
   double part[4];        // this CTA's partial: LJ, real, recip, overlap
   double tot[4];
   double wred[MT_THREADS / 32][4];
-  double prop[12];
   int accept;
 };
 
@@ -106,7 +134,8 @@ __host__ __device__ __forceinline__ size_t mixed_cold_bytes(int kc_max) {
 
 // Whether cells c1 and c2 are in one another's 27-cell neighbourhood (every
 // axis has at least 3 cells, src/CellList.cpp:138-161).
-__device__ __forceinline__ bool cells_adjacent(const DevBox &b, int c1, int c2) {
+template <class BOX>
+__device__ __forceinline__ bool cells_adjacent(const BOX &b, int c1, int c2) {
   const int e1 = b.edge[1], e2 = b.edge[2];
   int d[3] = {c2 / (e1 * e2) - c1 / (e1 * e2), (c2 / e2) % e1 - (c1 / e2) % e1,
               c2 % e2 - c1 % e2};
@@ -162,6 +191,15 @@ __device__ __forceinline__ double f64_of(float v) {
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// sin x for |x| < pi/4 (the polynomial of sin_f32)
+__device__ __forceinline__ float sin_small(float x) {
+  const float x2 = x * x;
+  float p = fmaf(x2, -2.5052108385e-8f, 2.7557319224e-6f);
+  p = fmaf(x2, p, -1.9841269841e-4f);
+  p = fmaf(x2, p, 8.3333333333e-3f);
+  p = fmaf(x2, p, -1.6666666667e-1f);
+  return fmaf(x * x2, p, x);
+}
 __device__ __forceinline__ float2 tabf(const float2 *row, int n) {
   float2 v = row[n < 0 ? -n : n];
   if (n < 0)
@@ -172,40 +210,37 @@ __device__ __forceinline__ float2 tabf(const float2 *row, int n) {
 // Header of move t into h (all threads of the CTA call it); prev is the
 // previous move's header, whose new positions are the current ones when
 // that move was accepted and touched the same molecule.
-// With `pre`, the inputs come from warp 7's loads (S.pre) instead of
-// global memory.
+// With `pre`, the inputs are in S.pre already (warp 7's loads, behind a CTA
+// barrier; another molecule than the previous move's) instead of in global
+// memory.
 __device__ void mixed_header(const MixedChain &C, MShared &S, int t,
                              bool prev_acc, int prev_m, int prev_kind,
                              const MHdr &prev, MHdr &h, bool pre = false) {
-  const DevBox &b = C.b;
-  const MoveRec &r = C.moves[t];
-  const MPre &P = S.pre;
+  const MHot &b = S.hot;
+  const MoveRec &r = b.moves[t];
+  MPre &P = S.pre;
   int m = pre ? P.m : r.mol;
   int a0 = pre ? P.a0 : b.mstart[m];
   int na = pre ? P.na : b.mstart[m + 1] - a0;
   const int rkind = pre ? P.kind : r.kind;
   const double rlpacc = pre ? P.lpacc : r.lpacc;
-  bool same = prev_acc && prev_m == m;
-  // the previous header still holds that move's new positions
-  __shared__ double oldp[MAXA][3], com[3];
-  if (threadIdx.x < 12)
-    S.prop[threadIdx.x] = pre ? P.prop[threadIdx.x]
-                              : C.prop[(size_t)t * 12 + threadIdx.x];
-  if (threadIdx.x < 3) {
-    int d = threadIdx.x;
-    const double *cs[3] = {b.cx, b.cy, b.cz};
-    com[d] = (same && prev_kind == 0) ? prev.newcom[d]
-             : pre                    ? P.com[d]
-                                      : __ldcg(cs[d] + m);
+  if (!pre) {
+    bool same = prev_acc && prev_m == m;
+    // the previous header still holds that move's new positions
+    if (threadIdx.x < 12)
+      P.prop[threadIdx.x] = b.prop[(size_t)t * 12 + threadIdx.x];
+    if (threadIdx.x < 3) {
+      int d = threadIdx.x;
+      const double *cs[3] = {b.cx, b.cy, b.cz};
+      P.com[d] = (same && prev_kind == 0) ? prev.newcom[d] : __ldcg(cs[d] + m);
+    }
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + 3 * na) {
+      int i = threadIdx.x - 32, a = i / 3, d = i % 3;
+      const double *xs[3] = {b.x, b.y, b.z};
+      P.oldp[a][d] = same ? prev.newp[a][d] : __ldcg(xs[d] + a0 + a);
+    }
+    __syncthreads();
   }
-  if (threadIdx.x >= 32 && threadIdx.x < 32 + 3 * na) {
-    int i = threadIdx.x - 32, a = i / 3, d = i % 3;
-    const double *xs[3] = {b.x, b.y, b.z};
-    oldp[a][d] = same ? prev.newp[a][d]
-                 : pre ? P.oldp[a][d]
-                       : __ldcg(xs[d] + a0 + a);
-  }
-  __syncthreads();
   // FP64 work costs a warp 64 cycles an instruction however many lanes take
   // part, so a lane has one coordinate and the parts are on warps of different
   // sub-partitions: warp 0 the new positions with their turns and cells, warp
@@ -214,19 +249,19 @@ __device__ void mixed_header(const MixedChain &C, MShared &S, int t,
   __shared__ int axis_cell[2][MAXA][3];
   if (warp < 2 && lane < 3 * na) {
     const int a = lane / 3, d = lane % 3;
-    double w = oldp[a][d];
+    double w = P.oldp[a][d];
     if (warp == 0) {
       if (rkind == 0) {
-        w = wrap1(__dadd_rn(w, S.prop[d]), b.L[d]);
+        w = wrap1(__dadd_rn(w, P.prop[d]), b.L[d]);
       } else {
         const unsigned act = __activemask();
-        const double v = __dadd_rn(unwrap1(w, com[d], b.L[d], b.half[d]), -com[d]);
+        const double v = __dadd_rn(unwrap1(w, P.com[d], b.L[d], b.half[d]), -P.com[d]);
         const double v0 = __shfl_sync(act, v, 3 * a), v1 = __shfl_sync(act, v, 3 * a + 1),
                      v2 = __shfl_sync(act, v, 3 * a + 2);
-        const double u = __dadd_rn(__dadd_rn(__dmul_rn(S.prop[3 * d], v0),
-                                             __dmul_rn(S.prop[3 * d + 1], v1)),
-                                   __dmul_rn(S.prop[3 * d + 2], v2));
-        w = wrap1(__dadd_rn(u, com[d]), b.L[d]);
+        const double u = __dadd_rn(__dadd_rn(__dmul_rn(P.prop[3 * d], v0),
+                                             __dmul_rn(P.prop[3 * d + 1], v1)),
+                                   __dmul_rn(P.prop[3 * d + 2], v2));
+        w = wrap1(__dadd_rn(u, P.com[d]), b.L[d]);
       }
       h.newp[a][d] = w;
       h.un[a][d] = to_turns(w, b.invL[d]);
@@ -254,8 +289,8 @@ __device__ void mixed_header(const MixedChain &C, MShared &S, int t,
       h.lpacc = rlpacc;
     }
     h.newcom[lane] = rkind == 0
-                         ? wrap1(__dadd_rn(com[lane], S.prop[lane]), b.L[lane])
-                         : com[lane];
+                         ? wrap1(__dadd_rn(P.com[lane], P.prop[lane]), b.L[lane])
+                         : P.com[lane];
   }
   __syncthreads();
   if (threadIdx.x < 3 * na) {
@@ -295,6 +330,7 @@ __global__ void __launch_bounds__(MT_THREADS)
   const DevBox &b = C.b;
   const FF &ff = *C.ff;
   __shared__ MShared S;
+  MHot &H = S.hot;
   extern __shared__ __align__(16) unsigned char dyn[];
   const int K = b.K;
   const int kc_max = (K + csize - 1) / csize;
@@ -327,6 +363,36 @@ __global__ void __launch_bounds__(MT_THREADS)
     S.set = *C.set;
     for (int i = 0; i < 5; ++i)
       S.e_run[i] = b.energy[i];
+    for (int d = 0; d < 3; ++d) {
+      H.L[d] = b.L[d];
+      H.half[d] = b.half[d];
+      H.invL[d] = b.invL[d];
+      H.cellSize[d] = b.cellSize[d];
+      H.invCell[d] = b.invCell[d];
+      H.edge[d] = b.edge[d];
+    }
+    H.x = b.x;
+    H.y = b.y;
+    H.z = b.z;
+    H.cx = b.cx;
+    H.cy = b.cy;
+    H.cz = b.cz;
+    H.q = b.q;
+    H.kind = b.kind;
+    H.mstart = b.mstart;
+    H.nbr = b.nbr;
+    H.cell_count = b.cell_count;
+    H.cell_meta = b.cell_meta;
+    H.atom_cell = b.atom_cell;
+    H.atom_slot = b.atom_slot;
+    H.cell_fix = b.cell_fix;
+    H.moves = C.moves;
+    H.prop = C.prop;
+    H.first = C.first;
+    H.cap = b.cap;
+    H.n = C.n;
+    H.ulog = C.ulog;
+    H.next_mol[0] = H.next_mol[1] = C.n > 1 ? C.moves[1].mol : -1;
   }
   __syncthreads();
   const int tpc = MT_THREADS * csize;
@@ -371,10 +437,10 @@ __global__ void __launch_bounds__(MT_THREADS)
   double pa_lp = 0.0, pb_lp = 0.0;
   auto pipe_record = [&](int t) {
     pa_m = -1;
-    if (t < C.n) {
-      pa_m = C.moves[t].mol;
-      pa_kind = C.moves[t].kind;
-      pa_lp = C.moves[t].lpacc;
+    if (t < H.n) {
+      pa_m = H.moves[t].mol;
+      pa_kind = H.moves[t].kind;
+      pa_lp = H.moves[t].lpacc;
     }
   };
   auto pipe_range = [&]() {
@@ -382,8 +448,8 @@ __global__ void __launch_bounds__(MT_THREADS)
     pb_kind = pa_kind;
     pb_lp = pa_lp;
     if (pb_m >= 0) {
-      pb_a0 = b.mstart[pb_m];
-      pb_a1 = b.mstart[pb_m + 1];
+      pb_a0 = H.mstart[pb_m];
+      pb_a1 = H.mstart[pb_m + 1];
     }
   };
   if (wid == 7) {
@@ -391,7 +457,50 @@ __global__ void __launch_bounds__(MT_THREADS)
     pipe_range();
     pipe_record(2);
   }
-  for (int t = 0; t < C.n; ++t) {
+  // The moved atoms' distinct cells of a header: the lane's cell (x), and the
+  // lanes that hold one first (y).
+  auto unit_cells = [&](const MHdr &hh) {
+    int cell = -1;  // one value for the idle lanes: the match takes a step a value
+    if (lid < 2 * hh.na)
+      cell = (lid & 1) ? hh.cell_new[lid >> 1] : hh.cell_old[lid >> 1];
+    const unsigned alike = __match_any_sync(0xffffffffu, cell);
+    return make_uint2((unsigned)cell,
+                      __ballot_sync(0xffffffffu, cell >= 0 && __ffs(alike) - 1 == lid));
+  };
+  // Neighbour cells of a header's units (below), -1 for one that an earlier
+  // unit has; by the warps from `first` on.
+  __shared__ int mu_c2[2 * MAXA * NB27], mu_n2[2 * MAXA * NB27];
+  auto list_units = [&](const MHdr &hh, int first) {
+    const uint2 cl = unit_cells(hh);
+    const int units = __popc(cl.y) * NB27;
+    for (int u0 = 0; u0 < units; u0 += MT_THREADS - 32 * first) {
+      const int u = u0 + threadIdx.x - 32 * first, d = min(u / NB27, 2 * MAXA - 1);
+      if (u0 + 32 * (wid - first) >= units)
+        continue;  // a whole warp
+      unsigned rest = cl.y;
+      bool seen = false;
+      int c2 = 0;
+      // this unit's cell is the d-th leader's; the earlier ones' are compared
+      for (int e = 0; rest; ++e, rest &= rest - 1) {
+        const int ce = (int)__shfl_sync(0xffffffffu, cl.x, __ffs(rest) - 1);
+        if (e == d && u < units)
+          c2 = H.nbr[ce * NB27 + (u - d * NB27)];
+      }
+      rest = cl.y;
+      for (int e = 0; rest; ++e, rest &= rest - 1) {
+        const int ce = (int)__shfl_sync(0xffffffffu, cl.x, __ffs(rest) - 1);
+        if (e < d && u < units)
+          seen = seen || cells_adjacent(H, ce, c2);
+      }
+      if (u < units)
+        mu_c2[u] = seen ? -1 : c2;
+    }
+  };
+  bool listed = false;  // this move's units were listed during the last one
+  // steps from the next move to a settings adjustment before it (0: now),
+  // counted: a 64-bit remainder is a hundred instructions a thread and move
+  int to_adj = H.n > 0 ? (int)(S.set.adj - 1 - (H.first + 1) % S.set.adj) : 0;
+  for (int t = 0; t < H.n; ++t, to_adj = to_adj ? to_adj - 1 : S.set.adj - 1) {
     const MHdr &h = S.hh[t & 1];
     // warp 7: the next move's inputs (their record and range loaded before)
     int n_m = -1, n_kind = 0, n_a0 = 0, n_na = 0;
@@ -405,19 +514,21 @@ __global__ void __launch_bounds__(MT_THREADS)
       n_na = pb_a1 - pb_a0;
       if (n_m >= 0) {
         if (lid < 12)
-          v_prop = C.prop[(size_t)(t + 1) * 12 + lid];
+          v_prop = H.prop[(size_t)(t + 1) * 12 + lid];
         if (lid < 3)
-          v_com = __ldcg((lid == 0 ? b.cx : lid == 1 ? b.cy : b.cz) + n_m);
+          v_com = __ldcg((lid == 0 ? H.cx : lid == 1 ? H.cy : H.cz) + n_m);
         if (lid < 3 * n_na) {
           const int a = lid / 3, d = lid % 3;
-          v_pos = __ldcg((d == 0 ? b.x : d == 1 ? b.y : b.z) + n_a0 + a);
+          v_pos = __ldcg((d == 0 ? H.x : d == 1 ? H.y : H.z) + n_a0 + a);
         }
         if (lid < n_na) {
-          v_q = b.q[n_a0 + lid];
-          v_k = b.kind[n_a0 + lid];
+          v_q = H.q[n_a0 + lid];
+          v_k = H.kind[n_a0 + lid];
         }
       }
       pipe_range();
+      if (lid == 0)
+        H.next_mol[(t + 1) & 1] = pb_m;
       pipe_record(t + 3);
     }
     const float2 *const tab = tabs + (t & 1) * tab_len;
@@ -425,14 +536,14 @@ __global__ void __launch_bounds__(MT_THREADS)
     // The next header does not depend on this move's outcome unless the
     // next move touches the same molecule or follows a settings adjustment:
     // then it is built during the cluster barrier before the decision.
-    const bool spec = t + 1 < C.n && C.moves[t + 1].mol != m &&
-                      (C.first + t + 2) % S.set.adj != 0;
+    const bool spec = t + 1 < H.n && H.next_mol[t & 1] != m &&
+                      to_adj != 0;
     // the moved atoms' current cells and slots, for the commit of rank 0
     // (loaded now, used after the decision)
     int cur_cell = -1, cur_slot = -1;
     if (rank == 0 && threadIdx.x < na) {
-      cur_cell = __ldcg(b.atom_cell + h.a0 + threadIdx.x);
-      cur_slot = __ldcg(b.atom_slot + h.a0 + threadIdx.x);
+      cur_cell = __ldcg(H.atom_cell + h.a0 + threadIdx.x);
+      cur_slot = __ldcg(H.atom_slot + h.a0 + threadIdx.x);
     }
     // ---------------- real space ----------------
     // Each neighbour j of an atom is taken once: inside the cutoff at both
@@ -446,45 +557,23 @@ __global__ void __launch_bounds__(MT_THREADS)
     // and each of their slots is loaded once and tested against every atom's
     // two positions (a unit per atom, position and neighbour loaded and
     // tested every slot six times for a water: 13,000 cycles a move).
-    int my_cell = -1 - (int)(threadIdx.x & 31);
-    if ((int)(threadIdx.x & 31) < 2 * na)
-      my_cell = (threadIdx.x & 1) ? h.cell_new[(threadIdx.x & 31) >> 1]
-                                  : h.cell_old[(threadIdx.x & 31) >> 1];
-    const unsigned alike = __match_any_sync(0xffffffffu, my_cell);
-    const unsigned lead = __ballot_sync(
-        0xffffffffu, my_cell >= 0 && __ffs(alike) - 1 == (int)(threadIdx.x & 31));
-    const int units = __popc(lead) * NB27;
+    int units;
+    if (!listed)
+      list_units(h, 0);
+    {
+      const unsigned lead = unit_cells(h).y;
+      units = __popc(lead) * NB27;
+    }
     // a unit's neighbour-cell slots are tiled over ul threads: slot lu,
     // lu + ul, ... of unit usub of this CTA's upc units per pass
-    const int ul = 1 << C.ulog, upc = MT_THREADS >> C.ulog;
-    const int lu = threadIdx.x & (ul - 1), usub = threadIdx.x >> C.ulog;
-    // the units' neighbour cells and slot counts, all at once
-    __shared__ int mu_c2[2 * MAXA * NB27], mu_n2[2 * MAXA * NB27];
-    for (int u0 = 0; u0 < units; u0 += MT_THREADS) {
-      const int u = u0 + threadIdx.x, d = min(u / NB27, 2 * MAXA - 1);
-      unsigned rest = lead;
-      int cell = -1;
-      bool seen = false;
-      int c2 = 0;
-      // this unit's cell is the d-th leader's; the earlier ones' are compared
-      for (int e = 0; rest; ++e, rest &= rest - 1) {
-        const int ce = __shfl_sync(0xffffffffu, my_cell, __ffs(rest) - 1);
-        if (e == d) {
-          cell = ce;
-          if (u < units)
-            c2 = b.nbr[cell * NB27 + (u - d * NB27)];
-        }
-      }
-      rest = lead;
-      for (int e = 0; rest; ++e, rest &= rest - 1) {
-        const int ce = __shfl_sync(0xffffffffu, my_cell, __ffs(rest) - 1);
-        if (e < d && u < units)
-          seen = seen || cells_adjacent(b, ce, c2);
-      }
-      if (u < units) {
-        mu_c2[u] = c2;
-        mu_n2[u] = seen ? 0 : __ldcg(b.cell_count + c2);
-      }
+    const int ul = 1 << H.ulog, upc = MT_THREADS >> H.ulog;
+    const int lu = threadIdx.x & (ul - 1), usub = threadIdx.x >> H.ulog;
+    // the units' slot counts, all at once
+    if (!listed)
+      __syncthreads();
+    for (int u = threadIdx.x; u < units; u += MT_THREADS) {
+      const int c2 = mu_c2[u];
+      mu_n2[u] = c2 < 0 ? 0 : __ldcg(H.cell_count + c2);
     }
     __syncthreads();
     // one candidate: atom a against cell slot s (meta mj, fixed-point slot f)
@@ -665,9 +754,9 @@ __global__ void __launch_bounds__(MT_THREADS)
     uint4 f = make_uint4(0, 0, 0, 0);
     auto load = [&](int v, int jj, int cnt, int &meta, uint4 &fix) {
       if (jj < cnt) {
-        const size_t s = (size_t)mu_c2[v + usub] * b.cap + jj;
-        meta = __ldcg(b.cell_meta + s);
-        fix = __ldcg(b.cell_fix + s);
+        const size_t s = (size_t)mu_c2[v + usub] * H.cap + jj;
+        meta = __ldcg(H.cell_meta + s);
+        fix = __ldcg(H.cell_fix + s);
       }
     };
     load(ub, j, n2, mj, f);
@@ -708,7 +797,7 @@ __global__ void __launch_bounds__(MT_THREADS)
         const unsigned mask = __ballot_sync(0xffffffffu, in);
         if (in) {
           const int pos = ln + __popc(mask & lt);
-          wl[pos] = (unsigned)mu_c2[ub + usub] * b.cap + j;
+          wl[pos] = (unsigned)mu_c2[ub + usub] * H.cap + j;
           wtag[pos] = (unsigned char)tag;
         }
         ln += __popc(mask);
@@ -789,45 +878,70 @@ __global__ void __launch_bounds__(MT_THREADS)
         if (32 * bt + lid < end) {
           const size_t s = sorted[32 * bt + lid];
           const int tag = stag[32 * bt + lid];
-          pair(tag >> 2, s, __ldcg(b.cell_meta + s), __ldcg(b.cell_fix + s));
+          pair(tag >> 2, s, __ldcg(H.cell_meta + s), __ldcg(H.cell_fix + s));
         }
       }
       // the lists are free for another round, or for dR/dI
     } while (__syncthreads_or(ub < units));
     // ---------------- reciprocal space ----------------
+    // Two k-vectors a thread at a time: the loop is bound by the latency of
+    // its row loads and products (some 0.4 instructions a cycle and scheduler
+    // with one).
     float de_h = 0.f, de_l = 0.f;
-    for (int i = threadIdx.x; i < kc; i += MT_THREADS) {
-      char4 n = kn[i];
-      float fx = (float)n.x, fy = (float)n.y, fz = (float)n.z;
-      float ddR = 0.f, ddI = 0.f;
+    for (int i = threadIdx.x; i < kc; i += 2 * MT_THREADS) {
+      const int i2[2] = {i, min(i + MT_THREADS, kc - 1)};
+      const bool two = i + MT_THREADS < kc;
+      char4 n[2];
+      float fx[2], fy[2], fz[2], ddR[2], ddI[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        n[u] = kn[i2[u]];
+        fx[u] = (float)n[u].x;
+        fy[u] = (float)n[u].y;
+        fz[u] = (float)n[u].z;
+        ddR[u] = ddI[u] = 0.f;
+      }
       for (int a = 0; a < na; ++a) {
-        float q = h.qf[a];
+        const float q = h.qf[a], qlo = h.qflo[a];
         if (q == 0.f)
           continue;
-        float arg = fmaf(fx, h.hf[a][0], fmaf(fy, h.hf[a][1], fz * h.hf[a][2]));
-        // mostly |k.h| < pi/4: the same polynomial without the reduction
-        float sa;
-        if (fabsf(arg) < 0.785f) {
-          const float x2 = arg * arg;
-          float ps = fmaf(x2, -2.5052108385e-8f, 2.7557319224e-6f);
-          ps = fmaf(x2, ps, -1.9841269841e-4f);
-          ps = fmaf(x2, ps, 8.3333333333e-3f);
-          ps = fmaf(x2, ps, -1.6666666667e-1f);
-          sa = fmaf(arg * x2, ps, arg);
-        } else {
-          sa = sin_f32(arg);
-        }
-        float w = 2.0f * fmaf(h.qflo[a], sa, q * sa);
+        const float hx = h.hf[a][0], hy = h.hf[a][1], hz = h.hf[a][2];
         const float2 *rx = tab + (size_t)(3 * a) * stride;
-        float2 e = cmulf(cmulf(rx[n.x], tabf(rx + stride, n.y)),
-                         tabf(rx + 2 * stride, n.z));
-        ddR = fmaf(-w, e.y, ddR);
-        ddI = fmaf(w, e.x, ddI);
+        float arg[2], sa[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          arg[u] = fmaf(fx[u], hx, fmaf(fy[u], hy, fz[u] * hz));
+        // mostly |k.h| < pi/4: the same polynomial without the reduction
+        if (fmaxf(fabsf(arg[0]), fabsf(arg[1])) < 0.785f) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            sa[u] = sin_small(arg[u]);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            sa[u] = fabsf(arg[u]) < 0.785f ? sin_small(arg[u]) : sin_f32(arg[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float w = 2.0f * fmaf(qlo, sa[u], q * sa[u]);
+          const float2 e = cmulf(cmulf(rx[n[u].x], tabf(rx + stride, n[u].y)),
+                                 tabf(rx + 2 * stride, n[u].z));
+          ddR[u] = fmaf(-w, e.y, ddR[u]);
+          ddI[u] = fmaf(w, e.x, ddI[u]);
+        }
       }
-      dR[i] = ddR;
-      dI[i] = ddI;
-      float sr = s32R[i], si = s32I[i];
-      two_sum_add(de_h, de_l, pf[i] * fmaf(2.0f * sr + ddR, ddR, (2.0f * si + ddI) * ddI));
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (u && !two)
+          break;
+        const int k = i2[u];
+        dR[k] = ddR[u];
+        dI[k] = ddI[u];
+        const float sr = s32R[k], si = s32I[k];
+        two_sum_add(de_h, de_l,
+                    pf[k] * fmaf(2.0f * sr + ddR[u], ddR[u],
+                                 (2.0f * si + ddI[u]) * ddI[u]));
+      }
     }
     // ---------------- reduce: warp (FP32), CTA (FP64) ----------------
     // compensated warp reduction, then FP64 across warps
@@ -922,7 +1036,11 @@ __global__ void __launch_bounds__(MT_THREADS)
           C.tr_d[3 * (size_t)t + 2] = dRc;
         }
       }
+    } else if (spec) {
+      // the next move's units, by the warps that wait for the decision
+      list_units(S.hh[(t + 1) & 1], 1);
     }
+    listed = spec;
     __syncthreads();
     const int acc = S.accept;
     const int prev_m = m, prev_kind = h.kind;
@@ -948,9 +1066,9 @@ __global__ void __launch_bounds__(MT_THREADS)
         if (a < na) {
           const double *np = h.newp[a];
           const int at = h.a0 + a;
-          b.x[at] = np[0];
-          b.y[at] = np[1];
-          b.z[at] = np[2];
+          H.x[at] = np[0];
+          H.y[at] = np[1];
+          H.z[at] = np[2];
           stay = cur_cell == h.cell_new[a];
           if (stay)
             cell_write_slot(b, cur_cell, cur_slot, at, np[0], np[1], np[2],
@@ -966,16 +1084,16 @@ __global__ void __launch_bounds__(MT_THREADS)
                              h.un[i]);
             }
           if (h.kind == 0) {
-            b.cx[m] = h.newcom[0];
-            b.cy[m] = h.newcom[1];
-            b.cz[m] = h.newcom[2];
+            H.cx[m] = h.newcom[0];
+            H.cy[m] = h.newcom[1];
+            H.cz[m] = h.newcom[2];
           }
         }
       }
     }
-    if (t + 1 < C.n) {
-      long long step = C.first + t + 1;
-      if ((step + 1) % S.set.adj == 0) {
+    if (t + 1 < H.n) {
+      long long step = H.first + t + 1;
+      if (to_adj == 0) {
         __syncthreads();
         if (threadIdx.x == 0)
           settings_adjust(S.set, step);
