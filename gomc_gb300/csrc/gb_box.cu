@@ -653,12 +653,11 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
       (rc = up(d.mstart, s.mstart.data(), (M + 1) * 4)))
     return rc;
   ff.erfc_tab = nullptr;
-  ff.vir_tab = nullptr;
   ff.pair_tab = nullptr;
   ff.etab_key0 = ff.etab_nseg = 0;
   if (c.ewald) {
     std::vector<double> et, vt;
-    double *d_et = nullptr, *d_vt = nullptr, *d_pt = nullptr;
+    double *d_et = nullptr, *d_pt = nullptr;
     erfc_table(ff.alpha, ff.rcutCoulSq, et, &ff.etab_key0, &ff.etab_nseg);
     erfc_table(ff.alpha, ff.rcutCoulSq, vt, &ff.etab_key0, &ff.etab_nseg,
                true);
@@ -676,12 +675,9 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
     if ((rc = Alloc(&d_pt, pt.size())) ||
         (rc = up(d_pt, pt.data(), pt.size() * sizeof(double))) ||
         (rc = Alloc(&d_et, et.size())) ||
-        (rc = up(d_et, et.data(), et.size() * sizeof(double))) ||
-        (rc = Alloc(&d_vt, vt.size())) ||
-        (rc = up(d_vt, vt.data(), vt.size() * sizeof(double))))
+        (rc = up(d_et, et.data(), et.size() * sizeof(double))))
       return rc;
     ff.erfc_tab = d_et;
-    ff.vir_tab = d_vt;
     ff.pair_tab = d_pt;
   }
   if ((rc = up(d_ff, &ff, sizeof(FF))))
@@ -1478,11 +1474,10 @@ int Box::SetBox(const double L[3], const double *xyz, const double *com) {
     return rc;
   // force-field constants that depend on the edges (the mixed form's FP32
   // turn length); the erfc table does not
-  const double *etab = ff.erfc_tab, *vtab = ff.vir_tab, *ptab = ff.pair_tab;
+  const double *etab = ff.erfc_tab, *ptab = ff.pair_tab;
   int key0 = ff.etab_key0, nseg = ff.etab_nseg;
   build_ff(s, cfg, &ff);
   ff.erfc_tab = etab;
-  ff.vir_tab = vtab;
   ff.pair_tab = ptab;
   ff.etab_key0 = key0;
   ff.etab_nseg = nseg;

@@ -61,12 +61,10 @@ struct FF {
   // only): 64 segments per binade of r^2 from 0.5 A^2, 9 coefficients each;
   // segment of r^2 = (its IEEE exponent and top 6 mantissa bits) - key0
   const double *erfc_tab;
-  // (erfc(alpha r) / r + 2 alpha / sqrt(pi) exp(-alpha^2 r^2)) / r^2, the
-  // Coulomb force factor of FFParticle::CalcCoulombVir, on the same segments
-  const double *vir_tab;
-  // both tables again in the layout of the box-wide pair walks: per segment
-  // 64 bytes of erfc(alpha r) / r and 64 of the force factor, each degrees
-  // 0-5 in FP64 and degrees 6-8 in FP32 (and a pad)
+  // the same on the same segments in the layout of the pair walks, with the
+  // Coulomb force factor of FFParticle::CalcCoulombVir, (erfc(alpha r) / r +
+  // 2 alpha / sqrt(pi) exp(-alpha^2 r^2)) / r^2: per segment 64 bytes of each,
+  // degrees 0-5 in FP64 and degrees 6-8 in FP32 (and a pad)
   const double *pair_tab;
   int etab_key0, etab_nseg;
   // soft-core settings at lambda < 1 (Forcefield::sc_*,

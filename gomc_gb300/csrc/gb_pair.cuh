@@ -75,18 +75,12 @@ __device__ __forceinline__ double coulomb_energy(const FF &ff, double distSq,
   return qq / sqrt(distSq);
 }
 
-// FFParticle::CalcCoulombVir (src/FFParticle.cpp:401-446)
+// FFParticle::CalcCoulombVir (src/FFParticle.cpp:401-446) by the formula; the
+// pair walks take the Ewald force factor from pair_poly inside its range.
 __device__ __forceinline__ double coulomb_virial(const FF &ff, double distSq,
                                                  double qq) {
   if (ff.rcutCoulSq < distSq)
     return 0.0;
-  if (ff.ewald) {
-    // the force factor from its table (same segments and accuracy as
-    // erfc_over_r), else the direct formula
-    double p;
-    if (seg_poly(ff, ff.vir_tab, distSq, &p))
-      return qq * p;
-  }
   double dist = sqrt(distSq);
   if (ff.ewald) {
     double constValue = ff.alpha * M_2_SQRTPI;
