@@ -12,21 +12,6 @@ __device__ __forceinline__ int pack_meta(int mol, int kind) {
 __device__ __forceinline__ int meta_mol(int meta) { return meta >> 4; }
 __device__ __forceinline__ int meta_kind(int meta) { return meta & 15; }
 
-// Neighbour nn of a cell (offsets dx, dy, dz in -1..1, dz fastest, each
-// axis wrapped): the entry of the 27-neighbour table Box::Init builds
-// (CellList::RebuildNeighbors order), computed instead of loaded.
-__device__ __forceinline__ int nbr_cell(const int *e, int cell, int nn) {
-  int z = cell % e[2], xy = cell / e[2];
-  int y = xy % e[1], x = xy / e[1];
-  x += nn / 9 - 1;
-  y += (nn / 3) % 3 - 1;
-  z += nn % 3 - 1;
-  x += x < 0 ? e[0] : (x >= e[0] ? -e[0] : 0);
-  y += y < 0 ? e[1] : (y >= e[1] ? -e[1] : 0);
-  z += z < 0 ? e[2] : (z >= e[2] ? -e[2] : 0);
-  return (x * e[1] + y) * e[2] + z;
-}
-
 // Write the packed slot data of atom `a` at (cell, slot); `tur`, when
 // given, holds the position's fixed-point turns (to_turns of x, y, z).
 __device__ __forceinline__ void cell_write_slot(const DevBox &b, int cell,
