@@ -35,10 +35,13 @@
 // core works on the last one; a seventeenth starts the products.  The other operand (X or C) is cut
 // beforehand and copied asynchronously by three more, a stage ahead (16-byte
 // copies: only the columns in use are copied, and bulk copies of that many
-// pieces took 75 cycles each to start).  The slices of that operand lie side by side
-// as columns, so digit i of Y meets digits 0 .. 6 - i of it in one product of
-// up to 256 columns (18 products a stage instead of 56, and each slice of Y
-// read once or twice, not up to seven times).
+// pieces took 75 cycles each to start).  The slices of that operand lie side by
+// side as columns, so digit i of Y meets several digits of it in one product.
+// Products started one after another run in that order only where their
+// accumulator and shape are the same, so the accumulators form three blocks
+// (d = 0, 1 .. 3, 4 .. 6) and every product writes one whole block: digit i of Y
+// meets slices d - i, those below 0 being zeros ahead of the operand's own (24
+// products a stage instead of 56, a fifth of their columns zeros).
 // Forming Y on the fly keeps its 7 x 2 bytes per element out of memory.  Pairs
 // are sorted by their largest n_x, so the columns beyond the k-sphere are
 // skipped (a third of the product).
@@ -66,6 +69,8 @@ namespace {
 constexpr int TM = 128;      // rows of D per CTA
 constexpr int TK = 32;       // terms per stage
 constexpr int NSL = 7;       // digits per operand
+constexpr int ZSL = 2;       // slices of zeros ahead of the right operand's
+constexpr int BSL = ZSL + NSL;
 constexpr int WIN = 4;       // stages per exact window: 128 terms
 constexpr int ET = 512;      // threads that form the left operand
 constexpr int CW = 3;        // warps that copy the right operand
@@ -195,25 +200,66 @@ __device__ __forceinline__ void mma_f16(unsigned lead, unsigned d, uint64_t a,
       "l"(a), "l"(b), "r"(idesc), "r"((unsigned)add), "r"(lead)
       : "memory");
 }
+// The products of 16 terms: digit i of Y on the slices from `b` on (ZSL is digit
+// 0's), `len` of them, into the accumulators d0 .. d0 + len - 1, for
+// d0 + len > i; three blocks of accumulators, digits ascending.
+struct Product {
+  int i, d0, len, b;
+};
+constexpr int NPROD = 12;
+constexpr Product product(int k) {
+  const int d0[3] = {0, 1, 4}, len[3] = {1, 3, 3};
+  for (int i = 0; i < NSL; ++i)
+    for (int g = 0; g < 3; ++g)
+      if (i < d0[g] + len[g] && k-- == 0)
+        return {i, d0[g], len[g], ZSL + d0[g] - i};
+  return {0, 0, 0, 0};
+}
+// Products that share a column have the same accumulator and shape; the first of
+// each block (which overwrites it) comes before the others; every i + j < NSL
+// is in exactly one; and none leaves the operand's slices or 256 columns.
+constexpr bool products_ordered() {
+  int met[NSL][NSL] = {};
+  for (int k = 0; k < NPROD; ++k) {
+    const Product p = product(k);
+    if (p.len < 1 || p.len * NT_MAX > 256 || p.b < 0 || p.b + p.len > BSL)
+      return false;
+    for (int m = 0; m < k; ++m) {
+      const Product o = product(m);
+      const bool share = o.d0 < p.d0 + p.len && p.d0 < o.d0 + o.len;
+      if (share && (o.d0 != p.d0 || o.len != p.len || o.i >= p.i))
+        return false;
+    }
+    for (int d = p.d0; d < p.d0 + p.len; ++d) {
+      const int j = p.b + d - p.d0 - ZSL;
+      if (p.i + (j < 0 ? d - p.i : j) != d || (j >= 0 && ++met[p.i][j] > 1))
+        return false;
+    }
+  }
+  for (int i = 0; i < NSL; ++i)
+    for (int j = 0; i + j < NSL; ++j)
+      if (!met[i][j])
+        return false;
+  return product(NPROD).len == 0;
+}
+static_assert(products_ordered(), "products of one accumulator out of order");
+
 // All products of a stage with N columns a slice.
 template <int N>
 __device__ __forceinline__ void mma_stage(unsigned lead, unsigned tmem,
                                           unsigned sa, unsigned sb, bool open) {
-  const uint64_t da = smem_desc(sa, A_KO), db = smem_desc(sb, NSL * N * 16);
-  constexpr int FIT = 256 / N;  // slices of one product
+  const uint64_t da = smem_desc(sa, A_KO), db = smem_desc(sb, BSL * N * 16);
 #pragma unroll
   for (int ks = 0; ks < TK / 16; ++ks)
 #pragma unroll
-    for (int i = 0; i < NSL; ++i)
-#pragma unroll
-      for (int j = 0; j < NSL - i; j += FIT) {
-        constexpr unsigned I0 = 1u << 4 | (unsigned)(TM / 16) << 24;
-        const int w = (FIT < NSL - i - j ? FIT : NSL - i - j) * N;
-        mma_f16(lead, tmem + (i + j) * N,
-                da + (ks * (2 * A_KO) + i * A_SLICE >> 4),
-                db + (uint64_t)(ks * (2 * NSL * N) + j * N),
-                I0 | (unsigned)(w >> 3) << 17, ks || i || !open);
-      }
+    for (int k = 0; k < NPROD; ++k) {
+      constexpr unsigned I0 = 1u << 4 | (unsigned)(TM / 16) << 24;
+      const Product p = product(k);
+      mma_f16(lead, tmem + p.d0 * N,
+              da + (ks * (2 * A_KO) + p.i * A_SLICE >> 4),
+              db + (uint64_t)(ks * (2 * BSL * N) + p.b * N),
+              I0 | (unsigned)(p.len * N >> 3) << 17, ks || p.i || !open);
+    }
 }
 __device__ __forceinline__ void tmem_ld4(unsigned addr, float (&v)[4]) {
   unsigned r[4];
@@ -337,7 +383,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
   __shared__ int s_bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int piece = A.nt * 16;  // bytes of one slice of 8 terms in A.b
-  const int b_stage = 4 * NSL * piece;
+  const int b_stage = 4 * NSL * piece, b_ring = 4 * BSL * piece;
   unsigned char *const smem_b = smem + 2 * A_STAGE;  // three stages
   const int ct = blockIdx.z;
   // columns needed where the largest n_x is nx
@@ -413,7 +459,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
         break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const unsigned sa = smem_u32(smem + buf * A_STAGE),
-                     sb = smem_u32(smem_b + it % 3 * b_stage);
+                     sb = smem_u32(smem_b + it % 3 * b_ring);
       switch (window_cols(it)) {
         case 16: mma_stage<16>(lead, tmem, sa, sb, open); break;
         case 32: mma_stage<32>(lead, tmem, sa, sb, open); break;
@@ -435,7 +481,9 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
     ok = ok && issued == ns;
   } else if (warp > ET / 32) {
     // ---- the right operand: stage `it` of [8-term group][slice][columns],
-    // the window's columns only, into its third of a ring ----
+    // the window's columns only, into its third of a ring, each group behind
+    // its slices of zeros (written anew where the window's columns differ from
+    // those of the third's last stage) ----
     const int ctid = tid - ET - 32;
     const unsigned char *bsrc = A.b;
     if constexpr (FORCE)
@@ -444,7 +492,14 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       bsrc += ((size_t)ct * A.nst + s0) * b_stage;
     auto copy = [&](int it) {
       const int n16 = window_cols(it) >> 4;
-      const unsigned dst = smem_u32(smem_b + it % 3 * b_stage) + ctid * 16;
+      unsigned char *const ring = smem_b + it % 3 * b_ring;
+      if (it < 3 || n16 != window_cols(it - 3) >> 4) {
+        const int nz = ZSL * 16 * n16;  // 16-byte rows a group
+        for (int r = ctid; r < 4 * nz; r += 32 * CW)
+          reinterpret_cast<uint4 *>(ring)[r / nz * (BSL * 16 * n16) + r % nz] =
+              make_uint4(0, 0, 0, 0);
+      }
+      const unsigned dst = smem_u32(ring) + (ctid & 15) * 16;
       const unsigned char *src = bsrc + (size_t)it * b_stage + (ctid & 15) * 16;
       // 256 bytes (16 columns) at a time: piece q is group-and-slice r = q /
       // n16, block q - r n16 of the window's columns (q < 112: the division
@@ -456,7 +511,8 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
         const unsigned q = (ctid >> 4) + 2 * CW * k;
         const unsigned r = q * inv >> 16;
         if (q < total)
-          copy16(dst + k * (512 * CW), src + r * piece + (q - r * n16) * 256);
+          copy16(dst + (q + (r / NSL + 1) * ZSL * n16) * 256,
+                 src + r * piece + (q - r * n16) * 256);
       }
     };
     if (ns > 0)
@@ -831,7 +887,7 @@ Shape shape_of(int kmax) {
   s.ncol = s.nt * s.nct;
   return s;
 }
-int stage_smem(int nt) { return 2 * A_STAGE + 3 * NSL * nt * TK * 2; }
+int stage_smem(int nt) { return 2 * A_STAGE + 3 * BSL * nt * TK * 2; }
 
 // bits to the right of the point such that `terms` values of at most 1 fit
 // 62 bits

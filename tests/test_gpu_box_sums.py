@@ -154,3 +154,36 @@ def test_cutoff_to_the_last_bit(gb):
     near(lj, rF[2])
     near(box.virial(), ref.virial())
     box.close()
+
+
+# column tiles of 16, 32, 48 and 64, and two of 48
+@pytest.mark.parametrize("edge,tol,kmax", [
+    (20.0, 1e-3, (4, 7)), (50.0, 1e-3, (8, 15)), (50.0, 1e-5, (16, 23)),
+    (70.0, 1e-5, (24, 31)), (97.0, 1e-5, (32, 47))])
+def test_structure_factor_digits(gb, edge, tol, kmax):
+    """Every digit product of the structure factor counts: 64 single charges
+    against extended precision.
+
+    A product of a y-z and an x factor, numbers below 1 to 2^-54 each (2^-55
+    off), misses the digit products i + j >= 7, six of at most 2^14 2^-68, five
+    of 2^8 times less and so on, 6.03 2^-54 in all: with the rounding of its
+    phases within 2^-51 of the charge unit (a power of two above the charges).
+    An atom has four in each part of a sum.  A digit product left out moves each
+    by up to 64 x 128 x 2^-60 and more."""
+    s = mixture((64, 0, 0), (edge,) * 3, 3)
+    cfg = SimConfig(temperature=298.0, rcut=9.0, tolerance=tol)
+    box = gb.Box(s, cfg)
+    assert kmax[0] <= box.num_kvectors()[1] <= kmax[1]
+    box.system_total()
+    sr, si = box.sums_new()
+    kv = box.kvectors()
+    n = np.rint(np.stack([kv[c] for c in ("kx", "ky", "kz")], 1) * edge /
+                (2 * np.pi)).astype(np.longdouble)
+    turns = np.asarray(box.coords(), np.longdouble) / np.longdouble(edge)
+    t = n @ turns.T
+    a = (t - np.rint(t)) * np.longdouble("6.28318530717958647692528676655900577")
+    q = s.atom_charge.astype(np.longdouble)
+    bar = 4 * 2.0 ** -51 * 64 * 0.5  # 64 charges below 2^-1
+    assert np.abs(sr - np.cos(a) @ q).max() <= bar
+    assert np.abs(si - np.sin(a) @ q).max() <= bar
+    box.close()
