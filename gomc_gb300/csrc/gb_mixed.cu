@@ -254,7 +254,7 @@ __device__ void mixed_header(const MixedChain &C, MShared &S, int t,
       if (rkind == 0) {
         w = wrap1(__dadd_rn(w, P.prop[d]), b.L[d]);
       } else {
-        const unsigned act = __activemask();
+        const unsigned act = (1u << 3 * na) - 1;  // the lanes in here
         const double v = __dadd_rn(unwrap1(w, P.com[d], b.L[d], b.half[d]), -P.com[d]);
         const double v0 = __shfl_sync(act, v, 3 * a), v1 = __shfl_sync(act, v, 3 * a + 1),
                      v2 = __shfl_sync(act, v, 3 * a + 2);
