@@ -715,11 +715,42 @@ int Box::CheckError() {
 int Box::CheckErrorWord(int word) {
   if (word & DERR_CELL_OVERFLOW)
     return Fail(ERR_CAPACITY, "a cell exceeded its slot capacity");
-  if (word & DERR_BARRIER_TIMEOUT)
+  if (word & (DERR_BARRIER_TIMEOUT | DERR_SUMS_TIMEOUT))
     return Fail(ERR_TIMEOUT, "a device-side wait ran out of iterations");
   if (word & DERR_BAD_INPUT)
     return Fail(ERR_ARG, "invalid input detected on the device");
   return OK;
+}
+
+int Box::QueueErrorWord() {
+  return CudaCheck(cudaMemcpyAsync(h_pinned + ERR_SLOT, dev.err, 4,
+                                   cudaMemcpyDeviceToHost, stream),
+                   "error read");
+}
+int Box::CheckQueuedSums() {
+  return CheckErrorWord(*(const int *)(h_pinned + ERR_SLOT) & DERR_SUMS_TIMEOUT);
+}
+int Box::CheckSums() {
+  int rc = QueueErrorWord();
+  if (rc || (rc = Sync()))
+    return rc;
+  return CheckQueuedSums();
+}
+
+int Box::SetWaitLimit(int64_t polls) {
+  if (polls < 0 || polls > 0xffffffffLL)
+    return Fail(ERR_ARG, "the wait limit must be 0 (default) to 2^32 - 1");
+  sums_spin = polls == 0 ? SUMS_SPIN : (unsigned)polls;
+  int rc = QueueErrorWord();
+  if (rc || (rc = Sync()))
+    return rc;
+  int *word = (int *)(h_pinned + ERR_SLOT);
+  if (!(*word & DERR_SUMS_TIMEOUT))
+    return OK;
+  *word &= ~DERR_SUMS_TIMEOUT;
+  rc = CudaCheck(cudaMemcpyAsync(dev.err, word, 4, cudaMemcpyHostToDevice, stream),
+                 "error reset");
+  return rc ? rc : Sync();
 }
 
 int Box::GridAll() {
@@ -774,25 +805,21 @@ int Box::BoxInter(double *inter, double *real) {
 int Box::RecipSums(const double *x, const double *y, const double *z) {
   if (!cfg.ewald)
     return OK;
-  return launch_recip_sums(*this, x, y, z, dev.sumRnew, dev.sumInew);
+  int rc = launch_recip_sums(*this, x, y, z, dev.sumRnew, dev.sumInew);
+  return rc ? rc : CheckSums();
+}
+
+int Box::RecipSetupAsync() {
+  if (!cfg.ewald)
+    return OK;
+  int rc = launch_recip_sums(*this, dev.x, dev.y, dev.z, dev.sumRnew, dev.sumInew);
+  // SetRecipRef
+  return rc ? rc : launch_adopt_sums(*this);
 }
 
 int Box::RecipSetup() {
-  if (!cfg.ewald)
-    return OK;
-  int rc = RecipSums(dev.x, dev.y, dev.z);
-  if (rc)
-    return rc;
-  // SetRecipRef: Ref <- New
-  size_t bytes = (size_t)dev.K * 8;
-  if ((rc = CudaCheck(cudaMemcpyAsync(dev.sumRref, dev.sumRnew, bytes,
-                                      cudaMemcpyDeviceToDevice, stream),
-                      "copy")) ||
-      (rc = CudaCheck(cudaMemcpyAsync(dev.sumIref, dev.sumInew, bytes,
-                                      cudaMemcpyDeviceToDevice, stream),
-                      "copy")))
-    return rc;
-  return OK;
+  int rc = RecipSetupAsync();
+  return rc || !cfg.ewald ? rc : CheckSums();
 }
 
 int Box::RecipEnergy(double *e, bool ref_sums) {
@@ -807,7 +834,7 @@ int Box::RecipEnergy(double *e, bool ref_sums) {
   if ((rc = CudaCheck(cudaMemcpyAsync(h_pinned, d_small, 8,
                                       cudaMemcpyDeviceToHost, stream),
                       "download")) ||
-      (rc = Sync()))
+      (rc = QueueErrorWord()) || (rc = Sync()) || (rc = CheckQueuedSums()))
     return rc;
   *e = h_pinned[0];
   return OK;
@@ -920,7 +947,7 @@ int Box::SystemTotal(double out[9]) {
     return rc;
   double recip = 0.0, self = 0.0, corr = 0.0;
   if (cfg.ewald) {
-    if ((rc = RecipSetup()) || (rc = RecipEnergy(&recip, true)) ||
+    if ((rc = RecipSetupAsync()) || (rc = RecipEnergy(&recip, true)) ||
         (rc = BoxCorrection(&corr)) || (rc = BoxSelf(&self)))
       return rc;
   }
@@ -1171,7 +1198,7 @@ int Box::BoxForceRecip(double *h_aR, double *h_mR) {
                                               cudaMemcpyDeviceToHost, stream),
                               "download")))
     return rc;
-  return Sync();
+  return CheckSums();
 }
 
 int Box::Torque(double *h_tq) {
@@ -1407,7 +1434,7 @@ int Box::RecipSumsCoords(const double *xyz, bool new_set) {
                                    dev.sumInew)))
     return rc;
   new_sums_set_ = new_set ? 1 : 0;
-  return Sync();
+  return CheckSums();
 }
 
 int Box::RecipEnergyNew(double *e, bool new_volume) {
@@ -1428,7 +1455,7 @@ int Box::RecipEnergyNew(double *e, bool new_volume) {
   if ((rc = CudaCheck(cudaMemcpyAsync(h_pinned, d_small, 8,
                                       cudaMemcpyDeviceToHost, stream),
                       "download")) ||
-      (rc = Sync()))
+      (rc = QueueErrorWord()) || (rc = Sync()) || (rc = CheckQueuedSums()))
     return rc;
   *e = h_pinned[0];
   return OK;

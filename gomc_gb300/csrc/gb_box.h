@@ -12,6 +12,9 @@ namespace gb {
 
 struct McState;  // Monte Carlo loop state (gb_mc.cu)
 
+constexpr unsigned SUMS_SPIN = 1u << 22;  // gb_box_set_wait_limit's default
+constexpr int ERR_SLOT = 4095;            // of h_pinned: the error word
+
 // One Ewald k-vector set (the kx/ky/kz/hsqr/prefact arrays and imageSize of
 // src/Ewald.h:202-211) with the box edges it was built for.  A box keeps the
 // current set (Ref) and a second one that RecipInit fills for trial edges
@@ -74,6 +77,8 @@ class Box {
   int SwapCorrection(int m, const double *pos, double *e);
   int BoxInter(double *inter, double *real);     // CalculateEnergy::BoxInter
   int RecipSetup();                              // Ewald::BoxReciprocalSetup
+  // the same without its check (CheckSums or RecipEnergy follows)
+  int RecipSetupAsync();
   int RecipSums(const double *d_x, const double *d_y, const double *d_z);
   int RecipEnergy(double *e, bool ref_sums);     // Ewald::BoxReciprocal
   int SystemTotal(double out9[9]);               // CalculateEnergy::SystemTotal
@@ -106,6 +111,12 @@ class Box {
   int GetSumNew(double *sr, double *si);
   int CheckError();
   int CheckErrorWord(int word);
+  // Whether the Ewald sums and forces launched so far are complete: queue the
+  // error word's copy, then, after Sync, look at it; or all of it
+  int QueueErrorWord();
+  int CheckQueuedSums();
+  int CheckSums();
+  int SetWaitLimit(int64_t polls);
 
   // ---- internals shared with the Monte Carlo loop ----
   DevBox dev{};
@@ -129,6 +140,8 @@ class Box {
   KSet kref, knew;
   size_t sums_cap = 0;
   TrialState trial;
+
+  unsigned sums_spin = SUMS_SPIN;  // polls of a wait of the Ewald sums
 
   // charges: |q| < 2^q_exp, and their sum in units of 2^q_exp
   int q_exp = 0;
@@ -202,6 +215,8 @@ int launch_recip_sums_view(Box &b, const DevBox &d, const double *x,
                            const double *y, const double *z, double *sumR,
                            double *sumI);
 size_t recip_sums_scratch(int n_atoms, int kmax, int npair);
+// Ref <- New, unless the New sums are incomplete
+int launch_adopt_sums(Box &b);
 // reciprocal forces without the intramolecular part as *nfp partials
 // [*nfp][3][n_atoms] in scratch, with `extra` doubles of it for the caller
 int launch_force_split(Box &b, const DevBox &d, const double *sumR,

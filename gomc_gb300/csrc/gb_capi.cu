@@ -267,6 +267,9 @@ int gb_get_sums_new(gb_box *box, double *sum_r, double *sum_i) {
     return gb::ERR_ARG;
   BOX_CALL(GetSumNew(sum_r, sum_i));
 }
+int gb_box_set_wait_limit(gb_box *box, int64_t polls) {
+  BOX_CALL(SetWaitLimit(polls));
+}
 int gb_box_reciprocal_setup(gb_box *box) { BOX_CALL(RecipSetup()); }
 int gb_box_reciprocal_sums(gb_box *box) {
   BOX_CALL(RecipSums(box->b->dev.x, box->b->dev.y, box->b->dev.z));

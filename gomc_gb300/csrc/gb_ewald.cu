@@ -80,7 +80,6 @@ constexpr int A_KO = TM * 16 + 32;              // bytes between 8-term groups
 constexpr int A_SLICE = TK / 8 * A_KO;          // bytes
 constexpr int A_STAGE = NSL * A_SLICE;
 constexpr int BATCH = 32768;                    // atoms per pass (bounds scratch)
-constexpr unsigned WAIT_LIMIT = 1u << 22;       // polls of a barrier
 
 // 2^-62 value as (hi, lo) with a signed low half, v = hi 2^32 + lo: a product
 // then takes three 32 x 32-bit multiplies
@@ -158,12 +157,20 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-// Bounded wait for a phase; false when it gives up, or when another warp has
+// Wait of at most `limit` polls for a phase, the first of them immediate, the
+// others suspended for a time; false when it gives up, or when another warp has
 // (*bad).
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity,
-                                          const int *bad) {
-  for (unsigned it = 0; it < WAIT_LIMIT; ++it) {
-    unsigned ok;
+                                          const int *bad, unsigned limit) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  for (unsigned it = 1; !ok && it < limit; ++it) {
     asm volatile(
         "{\n .reg .pred p;\n"
         " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
@@ -171,12 +178,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity,
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
-    if (ok)
-      return true;
     if (bad && (it & 63u) == 63u && *(volatile const int *)bad)
-      return false;
+      break;
   }
-  return false;
+  return ok;
 }
 // 16 bytes from global to shared memory, asynchronously
 __device__ __forceinline__ void copy16(unsigned dst, const void *src) {
@@ -361,6 +366,7 @@ struct SplitArgs {
                                    // |C_w| of each n_x
   double *fpart;                   // [nct][3][n_atoms]
   int atom0, na, n_atoms;
+  unsigned spin;  // polls of a wait
   int *err;
 };
 
@@ -453,8 +459,8 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       const int buf = it & 1;
       const bool open = it % WIN == 0;
       if (open && it)
-        ok = mbar_wait(&flushed, (it / WIN - 1) & 1, &s_bad);
-      ok = ok && mbar_wait(&full[buf], (it >> 1) & 1, &s_bad);
+        ok = mbar_wait(&flushed, (it / WIN - 1) & 1, &s_bad, A.spin);
+      ok = ok && mbar_wait(&full[buf], (it >> 1) & 1, &s_bad, A.spin);
       if (!__all_sync(0xffffffffu, ok))
         break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -474,9 +480,11 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       __syncwarp();
       issued = it + 1;
     }
-    // nothing may be in flight when the tensor memory goes back
+    // nothing may be in flight when the tensor memory goes back, whatever the
+    // limit of the other waits
     if (issued > 0)
-      ok = mbar_wait(&done[(issued - 1) & 1], ((issued - 1) >> 1) & 1, nullptr) &&
+      ok = mbar_wait(&done[(issued - 1) & 1], ((issued - 1) >> 1) & 1, nullptr,
+                     SUMS_SPIN) &&
            ok;
     ok = ok && issued == ns;
   } else if (warp > ET / 32) {
@@ -519,7 +527,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       copy(0);
     for (int it = 0; it < ns; ++it) {
       if (it >= 2)
-        ok = mbar_wait(&done[it & 1], ((it - 2) >> 1) & 1, &s_bad);
+        ok = mbar_wait(&done[it & 1], ((it - 2) >> 1) & 1, &s_bad, A.spin);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
@@ -654,7 +662,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       if (it + 1 < ns)
         load(it + 1);
       if (it >= 2)
-        ok = mbar_wait(&done[it & 1], ((it - 2) >> 1) & 1, &s_bad);
+        ok = mbar_wait(&done[it & 1], ((it - 2) >> 1) & 1, &s_bad, A.spin);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
@@ -667,7 +675,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       // the last window's accumulators, when its products are done; the next
       // stage's operand is ready by then
       if (it % WIN == 0 && it) {
-        ok = mbar_wait(&done[(it - 1) & 1], ((it - 1) >> 1) & 1, &s_bad);
+        ok = mbar_wait(&done[(it - 1) & 1], ((it - 1) >> 1) & 1, &s_bad, A.spin);
         if (!__all_sync(0xffffffffu, ok)) {
           ok = false;
           break;
@@ -681,7 +689,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
       }
     }
     if (ns > 0 && ok)
-      ok = mbar_wait(&done[(ns - 1) & 1], ((ns - 1) >> 1) & 1, &s_bad);
+      ok = mbar_wait(&done[(ns - 1) & 1], ((ns - 1) >> 1) & 1, &s_bad, A.spin);
     if (__all_sync(0xffffffffu, ok)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (ns > 0)
@@ -699,7 +707,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
   }
   if (!ok) {
     if (tid == 0)
-      atomicOr(A.err, DERR_BARRIER_TIMEOUT);
+      atomicOr(A.err, DERR_SUMS_TIMEOUT);
     return;
   }
   const int row = (warp & 3) * 32 + lane;
@@ -965,6 +973,7 @@ int launch_recip_sums_view(Box &bx, const DevBox &b, const double *x,
   A.nct = sh.nct;
   const int ub = unit_bits(bx.q_abs);  // of the whole sum
   A.acc = (unsigned long long *)(bx.d_scratch + d_yz + d_xs);
+  A.spin = bx.sums_spin;
   A.err = b.err;
   const size_t smem = stage_smem(sh.nt);
   raise_smem_limit((const void *)k_ewald_split<false>, smem);
@@ -989,6 +998,21 @@ int launch_recip_sums_view(Box &bx, const DevBox &b, const double *x,
       b.K, b.kn, b.pair_at, b.kmax, A.acc, sh.ncol,
       std::ldexp(1.0, bx.q_exp - ub), sumR, sumI);
   return bx.CudaCheck(cudaGetLastError(), "recip sums");
+}
+
+// SetRecipRef (src/Ewald.cpp:1021-1053); sums that a wait left incomplete stay
+// out of the Ref set.
+__global__ void k_adopt_sums(DevBox b) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= b.K || (*b.err & DERR_SUMS_TIMEOUT))
+    return;
+  b.sumRref[k] = b.sumRnew[k];
+  b.sumIref[k] = b.sumInew[k];
+}
+
+int launch_adopt_sums(Box &bx) {
+  k_adopt_sums<<<(bx.dev.K + 255) / 256, 256, 0, bx.stream>>>(bx.dev);
+  return bx.CudaCheck(cudaGetLastError(), "adopt sums");
 }
 
 // Reciprocal forces without the intramolecular part into *fpart, [*nfp][3]
@@ -1061,6 +1085,7 @@ int launch_force_split(Box &bx, const DevBox &b, const double *sumR,
   A.cmax = cmax;
   A.fpart = *fpart;
   A.n_atoms = b.n_atoms;
+  A.spin = bx.sums_spin;
   A.err = b.err;
   const size_t smem = stage_smem(sh.nt);
   raise_smem_limit((const void *)k_ewald_split<true>, smem);

@@ -42,6 +42,7 @@ enum DevErr : int {
   DERR_CELL_OVERFLOW = 1,
   DERR_BARRIER_TIMEOUT = 2,
   DERR_BAD_INPUT = 4,
+  DERR_SUMS_TIMEOUT = 8,  // a wait of the box-wide Ewald sums gave up
 };
 
 // Force-field constants, FlatIndex(i, j) = i + j * n_kinds

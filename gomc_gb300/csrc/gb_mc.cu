@@ -1780,7 +1780,10 @@ __global__ void __launch_bounds__(32) k_mp_accept(MpAcceptArgs P) {
     uint64_t r[4];
     philox4x64((uint64_t)b.n_mol, 0, 0, 0, P.step, P.seed, r);
     double pr = u01_64(r[0]);
-    int result = (*P.fail == 0) && pr < accept;
+    // a trial whose Ewald sums are incomplete is not accepted, and no forces
+    // are kept (gb_mc_run returns GB_ERR_TIMEOUT)
+    const bool torn = (*b.err & DERR_SUMS_TIMEOUT) != 0;
+    int result = (*P.fail == 0) && pr < accept && !torn;
     if (result) {
       e[0] = newInter;
       e[1] = newReal;
@@ -1790,6 +1793,8 @@ __global__ void __launch_bounds__(32) k_mp_accept(MpAcceptArgs P) {
     if (result)
       s.mp_iacc[P.type]++;
     settings_update(s, 2, result);
+    if (torn)
+      s.singleMoveAccepted = 1;
     P.out[0] = result;
     if (P.tr_i) {
       P.tr_i[0] = 2;
@@ -2900,6 +2905,7 @@ int mc_run_batch(const std::vector<Box *> &boxes, int64_t first,
     skip_to(*b->mc, first);
   }
   std::vector<int64_t> left(boxes.size(), nsteps), n(boxes.size());
+  std::vector<char> ran_mp(boxes.size(), 0);
   std::vector<Box *> leaders;
   for (;;) {
     bool any = false, more = false;
@@ -2938,9 +2944,14 @@ int mc_run_batch(const std::vector<Box *> &boxes, int64_t first,
     });
     if (rc)
       return rc;
-    for (size_t i : mp)
+    for (size_t i : mp) {
       left[i] -= 1;
+      ran_mp[i] = 1;
+    }
   }
+  for (size_t i = 0; i < boxes.size(); ++i)
+    if (ran_mp[i] && (rc = boxes[i]->CheckError()))
+      return rc;
   return OK;
 }
 

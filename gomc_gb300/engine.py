@@ -240,6 +240,11 @@ class Box:
         self._chk(lib().gb_get_sums_new(self.h, _dp(a), _dp(b)))
         return a[:K], b[:K]
 
+    def set_wait_limit(self, polls: int = 0) -> None:
+        """Polls after which the device waits of the box-wide Ewald sums give
+        up (gb_box_set_wait_limit; 0: the default)."""
+        self._chk(lib().gb_box_set_wait_limit(self.h, int(polls)))
+
     def box_reciprocal_setup(self) -> None:
         self._chk(lib().gb_box_reciprocal_setup(self.h))
 

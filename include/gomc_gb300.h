@@ -138,6 +138,14 @@ int gb_num_kvectors(gb_box *box, int32_t *k_count, int32_t *kmax);
  * src/Ewald.cpp:847-903) */
 int gb_get_kvectors(gb_box *box, double *out7);
 int gb_get_sums_new(gb_box *box, double *sum_r, double *sum_i);
+/* Polls after which a wait inside the kernels of the box-wide Ewald sums and
+ * reciprocal forces gives up, 0 for the default 2^22 (seconds of waiting).
+ * The call whose kernel gives up returns GB_ERR_TIMEOUT and leaves the Ref sums
+ * and the running energies as they were (a MultiParticle move is rejected);
+ * later calls that check the box return it too, until this call, which forgets
+ * the time-out, or gb_mc_init.  No reference counterpart (the reference has no
+ * device-side waits). */
+int gb_box_set_wait_limit(gb_box *box, int64_t polls);
 /* BoxReciprocalSetup (src/Ewald.cpp:193-274) + SetRecipRef (:1021-1053) */
 int gb_box_reciprocal_setup(gb_box *box);
 /* BoxReciprocalSums (src/Ewald.cpp:281-361) for the current coordinates */
