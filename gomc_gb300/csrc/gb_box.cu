@@ -602,6 +602,10 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
   build_ff(s, c, &ff);
   double qmax = 0.0, qsum = 0.0;
   for (int i = 0; i < N; ++i) {
+    if (!std::isfinite(s.q[i])) {
+      q_odd = true;
+      continue;
+    }
     qmax = std::max(qmax, std::fabs(s.q[i]));
     qsum += std::fabs(s.q[i]);
   }

@@ -143,8 +143,10 @@ class Box {
 
   unsigned sums_spin = SUMS_SPIN;  // polls of a wait of the Ewald sums
 
-  // charges: |q| < 2^q_exp, and their sum in units of 2^q_exp
+  // charges: |q| < 2^q_exp, and their sum in units of 2^q_exp, without those
+  // that are infinite or not a number (q_odd: there are some)
   int q_exp = 0;
+  bool q_odd = false;
   double q_abs = 0.0;
 
   // scratch buffers

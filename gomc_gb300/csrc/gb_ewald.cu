@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(128) k_ewald_phases(PhaseArgs A) {
     step = cis_q62(u);
     if (axis == 0 && A.xs) {
       const double q = A.q[A.atom0 + a];
-      qf = fabs(q) < 0.000000001 ? 0 : __double2ll_rn(q * A.q_unit);
+      qf = fabs(q) < 0.000000001 || !isfinite(q) ? 0 : __double2ll_rn(q * A.q_unit);
     }
   }
   const int nst = A.nap / TK, piece = A.nt * 16;
@@ -377,6 +377,11 @@ __device__ __forceinline__ int scale_exp(unsigned long long bits) {
 }
 __device__ __forceinline__ double pow2(int e) {
   return __longlong_as_double((long long)(e + 1023) << 52);
+}
+// what a column's digits are multiples of; not a number where the largest
+// value is infinite or not a number
+__device__ __forceinline__ double column_scale(unsigned long long bits) {
+  return bits >= 0x7ff0000000000000ull ? nan("") : pow2(scale_exp(bits));
 }
 
 template <bool FORCE>
@@ -722,7 +727,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
 #pragma unroll
       for (int i = 0; i < 16; ++i)
         if (n0 + i < 2 * (A.kmax + 1))
-          f = fma((double)acc[i] * pow2(scale_exp(cm[(n0 + i) / 2])),
+          f = fma((double)acc[i] * column_scale(cm[(n0 + i) / 2]),
                   A.xd[(size_t)(n0 + i) * A.nap + a], f);
     double *red = reinterpret_cast<double *>(smem);
     if (warp < ET / 32)
@@ -756,13 +761,14 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// From D to the structure factors, in the order of the k-vectors.
+// From D to the structure factors, in the order of the k-vectors.  Charges that
+// are infinite or not a number have no digits: their terms (odd) are added here.
 // ---------------------------------------------------------------------------
 __global__ void k_ewald_unfold(int K, const char4 *__restrict__ kn,
                                const int *__restrict__ pair_at, int kmax,
                                const unsigned long long *__restrict__ acc,
-                               int ncol, double unit, double *sumR,
-                               double *sumI) {
+                               int ncol, double unit, PhaseArgs odd,
+                               double *sumR, double *sumI) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= K)
     return;
@@ -789,8 +795,20 @@ __global__ void k_ewald_unfold(int K, const char4 *__restrict__ kn,
     c[3] = 0 - c[3];
     s[3] = 0 - s[3];
   }
-  sumR[k] = (double)(long long)(c[0] - c[3] - s[2] - s[1]) * unit;
-  sumI[k] = (double)(long long)(s[0] - s[3] + c[2] + c[1]) * unit;
+  double re = (double)(long long)(c[0] - c[3] - s[2] - s[1]) * unit;
+  double im = (double)(long long)(s[0] - s[3] + c[2] + c[1]) * unit;
+  for (int a = 0; a < odd.na; ++a) {
+    const double q = odd.q[a];
+    if (isfinite(q))
+      continue;
+    const Cis e = cis_q62(turn64(odd.x[a], odd.L[0]) * (unsigned long long)n.x +
+                          turn64(odd.y[a], odd.L[1]) * (unsigned long long)n.y +
+                          turn64(odd.z[a], odd.L[2]) * (unsigned long long)n.z);
+    re += q * (double)e.c;
+    im += q * (double)e.s;
+  }
+  sumR[k] = re;
+  sumI[k] = im;
 }
 
 // ---------------------------------------------------------------------------
@@ -845,13 +863,14 @@ __global__ void __launch_bounds__(128) k_force_coef(CoefArgs A) {
       }
     }
   for (int w = 0; w < 3; ++w) {
-    double m = 0.0;
+    // the largest by its bits: infinities and NaN are above all
+    unsigned long long m = 0;
     for (int i = 0; i < 8; ++i)
-      m = fmax(m, fabs(c[w][i]));
+      m = max(m, (unsigned long long)__double_as_longlong(fabs(c[w][i])));
     for (int o = 16; o > 0; o >>= 1)
-      m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0.0)
-      atomicMax(A.cmax + w * (A.ncol / 2) + nx, (unsigned long long)__double_as_longlong(m));
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0)
+      atomicMax(A.cmax + w * (A.ncol / 2) + nx, m);
     if (p < A.npair)
       for (int s = 0; s < 2; ++s)
         for (int i = 0; i < 4; ++i)
@@ -994,9 +1013,10 @@ int launch_recip_sums_view(Box &bx, const DevBox &b, const double *x,
         <<<dim3(tiles, (A.nst + A.per - 1) / A.per, sh.nct), CTA, smem,
            bx.stream>>>(A);
   }
+  P.na = bx.q_odd ? b.n_atoms : 0;
   k_ewald_unfold<<<(b.K + 127) / 128, 128, 0, bx.stream>>>(
       b.K, b.kn, b.pair_at, b.kmax, A.acc, sh.ncol,
-      std::ldexp(1.0, bx.q_exp - ub), sumR, sumI);
+      std::ldexp(1.0, bx.q_exp - ub), P, sumR, sumI);
   return bx.CudaCheck(cudaGetLastError(), "recip sums");
 }
 

@@ -187,3 +187,28 @@ def test_structure_factor_digits(gb, edge, tol, kmax):
     assert np.abs(sr - np.cos(a) @ q).max() <= bar
     assert np.abs(si - np.sin(a) @ q).max() <= bar
     box.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_charge_that_is_not_finite(gb, value):
+    """An infinite charge or one that is not a number shows in every sum and
+    force it enters, and in no other."""
+    from oracle import oracle as orc
+    s = mixture((60, 40, 3), (20.0, 23.1, 26.9), 5)
+    s.atom_charge[17] = value
+    cfg = SimConfig(temperature=298.0, rcut=9.0, tolerance=1e-5)
+    box, ref = gb.Box(s, cfg), orc.OracleBox(s, cfg)
+    st, rt = box.system_total(), ref.system_total()
+    for k in ("inter", "real", "recip", "self", "correction", "total"):
+        assert np.isfinite(st[k]) == np.isfinite(rt[k]), k
+    near(st["inter"], rt["inter"])
+    for got, want in zip(box.sums_new(), ref.sum_new()):
+        assert not np.isfinite(want).any() and not np.isfinite(got).any()
+    box.copy_recip()
+    ref.copy_recip()
+    for got, want in zip(box.box_force_reciprocal() + box.box_force()[:2],
+                         ref.box_force_recip()[:2] + ref.box_force()[:2]):
+        np.testing.assert_array_equal(np.isfinite(got), np.isfinite(want))
+    np.testing.assert_array_equal(np.isfinite(box.virial()),
+                                  np.isfinite(ref.virial()))
+    box.close()
