@@ -146,6 +146,7 @@ SIGNATURES = {
     "gb_num_kvectors": (C.c_int, [_P, _I, _I]),
     "gb_get_kvectors": (C.c_int, [_P, _D]),
     "gb_get_sums_new": (C.c_int, [_P, _D, _D]),
+    "gb_box_device_bytes": (C.c_int, [_P, _L]),
     "gb_box_set_wait_limit": (C.c_int, [_P, C.c_int64]),
     "gb_box_reciprocal_setup": (C.c_int, [_P]),
     "gb_box_reciprocal_sums": (C.c_int, [_P]),

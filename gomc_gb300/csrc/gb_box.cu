@@ -276,16 +276,28 @@ int Box::CudaCheck(cudaError_t e, const char *what) {
   return e == cudaErrorMemoryAllocation ? ERR_NOMEM : ERR_CUDA;
 }
 
-template <class T>
-int Box::Alloc(T **p, size_t n) {
+int Box::DevMalloc(void **p, size_t bytes, std::vector<void *> &allocs) {
   void *q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+  cudaError_t e = cudaMalloc(&q, std::max<size_t>(bytes, 1));
   if (e != cudaSuccess)
     return CudaCheck(e, "cudaMalloc");
-  allocs_.push_back(q);
-  dev_bytes += std::max<size_t>(n, 1) * sizeof(T);
-  *p = (T *)q;
+  allocs.push_back(q);
+  alloc_bytes_[q] = bytes;
+  dev_bytes += bytes;
+  *p = q;
   return OK;
+}
+
+void Box::DevFree(void *p, std::vector<void *> &allocs) {
+  cudaFree(p);
+  allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
+  dev_bytes -= alloc_bytes_[p];
+  alloc_bytes_.erase(p);
+}
+
+template <class T>
+int Box::Alloc(T **p, size_t n) {
+  return DevMalloc((void **)p, std::max<size_t>(n, 1) * sizeof(T), allocs_);
 }
 
 void Box::FreeAll() {
@@ -297,6 +309,8 @@ void Box::FreeAll() {
   for (void *p : trial.allocs)
     cudaFree(p);
   trial.allocs.clear();
+  alloc_bytes_.clear();
+  dev_bytes = 0;
   if (h_pinned)
     cudaFreeHost(h_pinned);
   h_pinned = nullptr;
@@ -309,19 +323,10 @@ void Box::FreeAll() {
 // (Re)allocate *p to hold `bytes`, dropping its old contents; the pointer is
 // owned by `allocs`.
 static int regrow(Box &b, void **p, size_t bytes, std::vector<void *> &allocs) {
-  if (*p) {
-    cudaFree(*p);
-    allocs.erase(std::remove(allocs.begin(), allocs.end(), *p), allocs.end());
-    *p = nullptr;
-  }
-  void *q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(bytes, 1));
-  if (e != cudaSuccess)
-    return b.CudaCheck(e, "cudaMalloc");
-  allocs.push_back(q);
-  b.dev_bytes += bytes;
-  *p = q;
-  return OK;
+  if (*p)
+    b.DevFree(*p, allocs);
+  *p = nullptr;
+  return b.DevMalloc(p, bytes, allocs);
 }
 
 // CellList::ResizeGrid / RebuildNeighbors (src/CellList.cpp:138-218) for
@@ -490,9 +495,7 @@ int Box::EnsureSums(size_t K) {
                           "copy")) ||
           (rc = Sync()))
         return rc;
-      cudaFree(old);
-      allocs_.erase(std::remove(allocs_.begin(), allocs_.end(), (void *)old),
-                    allocs_.end());
+      DevFree(old, allocs_);
     }
     *arr[i] = q;
   }

@@ -6,6 +6,7 @@
 
 #include <memory>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 namespace gb {
@@ -173,6 +174,9 @@ class Box {
   int new_sums_set_ = 0;  // 1 when the New sums came from the New k set
   void MirrorKRef();
   int CudaCheck(cudaError_t e, const char *what);
+  // device memory with its size kept in dev_bytes, owned by `allocs`
+  int DevMalloc(void **p, size_t bytes, std::vector<void *> &allocs);
+  void DevFree(void *p, std::vector<void *> &allocs);
   int EnsureScratch(size_t n);
   int Sync();
 
@@ -181,6 +185,7 @@ class Box {
   int Init(const HostSystem &sys, const BoxConfig &cfg);
   void FreeAll();
   std::vector<void *> allocs_;
+  std::unordered_map<void *, size_t> alloc_bytes_;
   size_t grid_cell_cap_ = 0, grid_nbr_cap_ = 0;
   template <class T>
   int Alloc(T **p, size_t n);

@@ -267,6 +267,13 @@ int gb_get_sums_new(gb_box *box, double *sum_r, double *sum_i) {
     return gb::ERR_ARG;
   BOX_CALL(GetSumNew(sum_r, sum_i));
 }
+int gb_box_device_bytes(gb_box *box, int64_t *bytes) {
+  int rc = guard(box);
+  if (rc || !bytes)
+    return rc ? rc : (int)gb::ERR_ARG;
+  *bytes = (int64_t)(box->b->dev_bytes + (box->b->mc ? box->b->mc->bytes : 0));
+  return gb::OK;
+}
 int gb_box_set_wait_limit(gb_box *box, int64_t polls) {
   BOX_CALL(SetWaitLimit(polls));
 }

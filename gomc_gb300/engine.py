@@ -240,6 +240,12 @@ class Box:
         self._chk(lib().gb_get_sums_new(self.h, _dp(a), _dp(b)))
         return a[:K], b[:K]
 
+    def device_bytes(self) -> int:
+        """Device memory the box holds (gb_box_device_bytes)."""
+        n = C.c_int64()
+        self._chk(lib().gb_box_device_bytes(self.h, C.byref(n)))
+        return n.value
+
     def set_wait_limit(self, polls: int = 0) -> None:
         """Polls after which the device waits of the box-wide Ewald sums give
         up (gb_box_set_wait_limit; 0: the default)."""

@@ -361,6 +361,9 @@ int gb_mc_autotune(gb_box *box, int32_t objective, int32_t trial_moves,
 /* The launch shape gb_mc_init (or the autotuner) chose for this box's
  * chain, its trial time zero.  No reference counterpart. */
 int gb_mc_shape_get(gb_box *box, gb_mc_shape *shape);
+/* Device memory the box holds now, its Monte Carlo loop's included (what a
+ * server charges a job for).  No reference counterpart. */
+int gb_box_device_bytes(gb_box *box, int64_t *bytes);
 /* The CUDA stream (cudaStream_t) every call on this machine is ordered on. */
 int gb_box_stream(gb_box *box, void **stream);
 

@@ -104,3 +104,26 @@ def test_chain_profile_accounts_for_the_chain(gb):
     again = box.mc_profile(enable=False)
     assert again["moves"] == [0, 0]
     box.close()
+
+
+def test_device_bytes_are_those_held(gb):
+    """Arrays that grow replace the ones before: a box that grew in steps
+    reports what one that grew at once does, and a loop that is started again
+    is counted once."""
+    z, meta = load("c0_water")
+    sysm, cfg = system_of(z, meta), config_of(meta)
+    frac, adj = move_fractions(meta), meta["config"]["adj_steps"]
+    held = []
+    for scales in ((1.02, 1.05, 1.12), (1.12,)):
+        box = gb.Box(sysm, cfg)
+        first, L, x = box.device_bytes(), box.edges(), box.coords()
+        for s in scales:
+            box.recip_init(L * s)
+            box.box_reciprocal_setup_coords(x)
+        box.virial()
+        for _ in scales:
+            box.mc_init(meta["config"]["random_seed"], frac, adj)
+        assert box.device_bytes() > first > 0
+        held.append(box.device_bytes())
+        box.close()
+    assert held[0] == held[1]
