@@ -49,7 +49,13 @@ struct BoxConfig {
   int device = 0;
   double sc_alpha = 0.0, sc_sigma = 0.0;  // soft-core settings
   int sc_power = 0, sc_coul = 0;
+  // atoms per pass of the box-wide Ewald sums (a multiple of 128), which bounds
+  // their scratch, held for the box's life: 35 MB for 8,000 waters in one pass,
+  // 2.4 MB in passes of SUMS_BATCH_SERVED, which a server's jobs take (their
+  // sums come once per thousands of moves)
+  int sums_batch = 32768;
 };
+constexpr int SUMS_BATCH_SERVED = 1024;
 
 class Box {
  public:
@@ -221,7 +227,7 @@ int launch_recip_sums(Box &b, const double *x, const double *y,
 int launch_recip_sums_view(Box &b, const DevBox &d, const double *x,
                            const double *y, const double *z, double *sumR,
                            double *sumI);
-size_t recip_sums_scratch(int n_atoms, int kmax, int npair);
+size_t recip_sums_scratch(int n_atoms, int kmax, int npair, int batch);
 // Ref <- New, unless the New sums are incomplete
 int launch_adopt_sums(Box &b);
 // reciprocal forces without the intramolecular part as *nfp partials

@@ -79,7 +79,6 @@ constexpr int NT_MAX = 64;   // columns per CTA: 7 x 64 of 512 TMEM columns
 constexpr int A_KO = TM * 16 + 32;              // bytes between 8-term groups
 constexpr int A_SLICE = TK / 8 * A_KO;          // bytes
 constexpr int A_STAGE = NSL * A_SLICE;
-constexpr int BATCH = 32768;                    // atoms per pass (bounds scratch)
 
 // 2^-62 value as (hi, lo) with a signed low half, v = hi 2^32 + lo: a product
 // then takes three 32 x 32-bit multiplies
@@ -952,9 +951,9 @@ void launch_phases(Box &bx, PhaseArgs &P, int atom0, int na) {
 }  // namespace
 
 // Doubles of scratch the structure factor takes.
-size_t recip_sums_scratch(int n_atoms, int kmax, int npair) {
+size_t recip_sums_scratch(int n_atoms, int kmax, int npair, int batch) {
   const Shape sh = shape_of(kmax);
-  const int nap = (std::min(n_atoms, BATCH) + TM - 1) / TM * TM;
+  const int nap = (std::min(n_atoms, batch) + TM - 1) / TM * TM;
   return dbl((size_t)4 * (kmax + 1) * nap * sizeof(int2)) +
          dbl((size_t)sh.nct * (nap / TK) * NSL * sh.nt * TK * 2) +
          dbl((size_t)npair * 4 * sh.ncol * 8);
@@ -971,13 +970,13 @@ int launch_recip_sums_view(Box &bx, const DevBox &b, const double *x,
                            const double *y, const double *z, double *sumR,
                            double *sumI) {
   const Shape sh = shape_of(b.kmax);
-  const int batch = std::min(b.n_atoms, BATCH);
+  const int batch = std::min(b.n_atoms, bx.cfg.sums_batch);
   const int nap = (batch + TM - 1) / TM * TM;
   const size_t b_stage = (size_t)NSL * sh.nt * TK * 2;
   const size_t d_yz = dbl((size_t)4 * (b.kmax + 1) * nap * sizeof(int2));
   const size_t d_xs = dbl((size_t)sh.nct * (nap / TK) * b_stage);
   const size_t acc_bytes = (size_t)b.npair * 4 * sh.ncol * 8;
-  int rc = bx.EnsureScratch(recip_sums_scratch(b.n_atoms, b.kmax, b.npair));
+  int rc = bx.EnsureScratch(recip_sums_scratch(b.n_atoms, b.kmax, b.npair, batch));
   if (rc)
     return rc;
   PhaseArgs P = phase_args(bx, b, x, y, z, sh);
@@ -1000,8 +999,8 @@ int launch_recip_sums_view(Box &bx, const DevBox &b, const double *x,
                          "memset")))
     return rc;
   const int tiles = b.npair / 32;
-  for (int a0 = 0; a0 < b.n_atoms; a0 += BATCH) {
-    launch_phases(bx, P, a0, std::min(BATCH, b.n_atoms - a0));
+  for (int a0 = 0; a0 < b.n_atoms; a0 += batch) {
+    launch_phases(bx, P, a0, std::min(batch, b.n_atoms - a0));
     A.nap = P.nap;
     A.nst = P.nap / TK;
     // about two CTAs per SM, of whole windows: tiles differ in their columns
@@ -1041,7 +1040,7 @@ int launch_force_split(Box &bx, const DevBox &b, const double *sumR,
                        const double *sumI, size_t extra, double **fpart,
                        int *nfp, double **extra_out) {
   const Shape sh = shape_of(b.kmax);
-  const int batch = std::min(b.n_atoms, BATCH);
+  const int batch = std::min(b.n_atoms, bx.cfg.sums_batch);
   const int nap = (batch + TM - 1) / TM * TM;
   const int rows = 4 * b.npair, nst = rows / TK;
   const size_t b_stage = (size_t)NSL * sh.nt * TK * 2;
@@ -1109,8 +1108,8 @@ int launch_force_split(Box &bx, const DevBox &b, const double *sumR,
   A.err = b.err;
   const size_t smem = stage_smem(sh.nt);
   raise_smem_limit((const void *)k_ewald_split<true>, smem);
-  for (int a0 = 0; a0 < b.n_atoms; a0 += BATCH) {
-    const int na = std::min(BATCH, b.n_atoms - a0);
+  for (int a0 = 0; a0 < b.n_atoms; a0 += batch) {
+    const int na = std::min(batch, b.n_atoms - a0);
     launch_phases(bx, P, a0, na);
     A.nap = P.nap;
     A.atom0 = a0;

@@ -207,9 +207,13 @@ size_t job_bytes(const Job &j, int K, int kmax, int csize, size_t moves) {
               (size_t)(2 * MAX_MOL_ATOMS * 3) * (kmax + 1) * 16 + 64 * 1024;
   if (mixed_smem(K, kmax, csize, true) > MIXED_SMEM_MAX)
     mc += mixed_cold_buffer(K, csize);
-  // reduction scratch of the set-up kernels and allocation rounding
-  size_t scratch = 8 * recip_sums_scratch((int)N, kmax, (kmax + 1) * (kmax + 1)) +
-                   ((size_t)1 << 20);
+  // scratch: the Ewald sums' or the coordinates on their way to the host;
+  // the other kernels' partials and allocation rounding
+  size_t scratch =
+      8 * std::max(recip_sums_scratch((int)N, kmax, (kmax + 1) * (kmax + 1),
+                                      SUMS_BATCH_SERVED),
+                   3 * (N + M)) +
+      ((size_t)1 << 18);
   return box + mc + scratch + 96 * 512;
 }
 
@@ -246,6 +250,7 @@ Job *make_job(const gb_system_desc *sys, const gb_config *cfg) {
   c.electrostatic = cfg->electrostatic ? 1 : 0;
   c.precision = GB_MIXED;
   c.device = cfg->device;
+  c.sums_batch = SUMS_BATCH_SERVED;
   c.sc_alpha = cfg->sc_alpha;
   c.sc_sigma = cfg->sc_sigma;
   c.sc_power = cfg->sc_power;

@@ -112,6 +112,19 @@ def test_memory_admission(srv_mod):
     srv.close()
 
 
+# device bytes a job was charged while the structure factor's scratch was K and
+# N sized (1.1 to 2.9 MB); passes of atoms hold it there
+@pytest.mark.parametrize("n,rcut,bytes_", [
+    (300, 9.0, 2505204), (700, 9.0, 3165020), (2000, 9.0, 7329576),
+    (8000, 10.0, 22555480), (20000, 9.0, 61603852)])
+def test_job_memory(srv_mod, n, rcut, bytes_):
+    srv = srv_mod.Server(quantum=300)
+    cfg = SimConfig(temperature=298.0, rcut=rcut, tolerance=1e-5)
+    est = srv.estimate(spce_water_box(n, water_box_length(n), seed=1), cfg)
+    assert est["bytes"] <= 1.12 * bytes_
+    srv.close()
+
+
 def test_worker_thread(srv_mod):
     import time
     srv = srv_mod.Server(quantum=500)
