@@ -170,10 +170,7 @@ __device__ __forceinline__ bool pair_energy_pipe(const ChainArgs &A,
     l = 0.0;
     const double eps = pt.eps[idx];
     if (bits64(eps) != 0) {
-      double y = widen_f64(__frcp_rn(trunc_f32(d2)));
-      const double r = fma(-d2, y, 1.0);
-      y = fma(y, fma(r, r, r), y);
-      const double rRat2 = pt.sig2[idx] * y;
+      const double rRat2 = pt.sig2[idx] * recip_cubic(d2);
       const double attract = rRat2 * rRat2 * rRat2;
       l = eps * fma(attract, attract, -attract);
     }

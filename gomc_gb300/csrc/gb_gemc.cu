@@ -135,13 +135,8 @@ __device__ __forceinline__ float mimgf(float raw, float ax, float half) {
 __device__ __forceinline__ double lj64(const GemcParams &p, double d2) {
   double rRat2;
   if (in_fast_range(d2)) {
-    // sigma^2 / r^2 from the FP32 reciprocal: one cubic step, the product
-    // and its correction, six FP64 instructions for the division's dozen
-    double y = widen_f64(__frcp_rn(trunc_f32(d2)));
-    const double e = fma(-d2, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
-    rRat2 = p.sigmaSq * y;
-    rRat2 = fma(fma(-rRat2, d2, p.sigmaSq), y, rRat2);
+    // six FP64 instructions for the division's dozen
+    rRat2 = quot_pos(p.sigmaSq, d2, recip_cubic(d2));
   } else {
     rRat2 = p.sigmaSq / d2;
   }

@@ -200,11 +200,9 @@ __device__ __forceinline__ bool lj_live(const FF &ff, double distSq, int idx) {
 __device__ __forceinline__ void lj_terms(const FF &ff, double s, int idx,
                                          double *en, double *vir) {
   if (bits64(ff.nexp[idx]) == bits64(12.0) && in_fast_range(s)) {
-    const double y = recip_pos(s);
-    // sigma^2 / r^2 to the last bit: its sixth power carries the error
-    const double sg = ff.sigmaSq[idx];
-    double rRat2 = y * sg;
-    rRat2 = fma(fma(-rRat2, s, sg), y, rRat2);
+    const double y = recip_cubic(s);
+    // (its sixth power carries the error of sigma^2 / r^2)
+    const double rRat2 = quot_pos(ff.sigmaSq[idx], s, y);
     const double attract = rRat2 * rRat2 * rRat2;
     const double repulse = attract * attract;
     if (en)

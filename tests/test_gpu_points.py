@@ -120,3 +120,42 @@ def test_long_molecules_against_oracle(gb, length):
             for g, w, k in zip(got[1:], want[1:], ("inter", "real", "recip")):
                 assert abs(g - w) <= REL * max(abs(tot[k]), abs(w), 1.0), (k, g, w)
     box.close()
+
+
+def test_lj_term_to_the_last_bits(gb):
+    """One pair's 12-6 energy over r^2 from 0.25 to 81 A^2, powers of two and
+    their neighbours among them, against exact rational arithmetic.
+
+    Separations are multiples of 2^-20 A along one axis, so r^2 is exact.  With
+    sigma^2 / r^2 within a unit of the last place (2u, u = 2^-53), its third power
+    has 3 x 2 + 2 = 8 u, the sixth 2 x 8 + 1 = 17 u, and the difference and the
+    factor epsilon one each: 19 u of the two terms' sum."""
+    from fractions import Fraction
+    sigma, eps, edge, rc = 2.9, 70.0, 64.0, 9.0
+    s = MolSystem(np.full(3, edge), [AtomKind("A", eps, sigma, 12.0)],
+                  [MoleculeType("T", ["X"], [0], [0.0])],
+                  np.array([[16.0, 16.0, 16.0], [60.0, 60.0, 60.0]]),
+                  np.zeros(2, np.int32), np.zeros(2),
+                  np.arange(2, dtype=np.int32), np.arange(3, dtype=np.int32),
+                  np.zeros(2, np.int32))
+    cfg = SimConfig(temperature=298.0, rcut=rc, ewald=False,
+                    electrostatic=False)
+    box = gb.Box(s, cfg)
+    box.cell_remove_mol(1)
+    unit = 2.0 ** -20
+    pow2 = np.concatenate([np.sqrt(2.0 ** k) * (1 + np.arange(-8, 8) * 2.0 ** -20)
+                           for k in range(-2, 7)])
+    rng = np.random.default_rng(6)
+    r = np.concatenate([pow2, rng.uniform(0.5, rc - 0.01, 1500)])
+    r = np.rint(r / unit) * unit
+    en = np.concatenate([
+        box.particle_inter(1, 0, np.stack([16.0 + c, 0 * c + 16.0, 0 * c + 16.0],
+                                          -1))[1]
+        for c in np.array_split(r, 8)])
+    e4 = Fraction(4.0 * eps)
+    s2 = Fraction(sigma * sigma)
+    for d, got in zip(r, en):
+        x = (s2 / Fraction(d) ** 2) ** 3
+        bar = 19 * Fraction(1, 2 ** 53) * e4 * (x * x + x)
+        assert abs(Fraction(got) - e4 * (x * x - x)) <= bar, (d, got)
+    box.close()
