@@ -38,10 +38,10 @@
 // pieces took 75 cycles each to start).  The slices of that operand lie side by
 // side as columns, so digit i of Y meets several digits of it in one product.
 // Products started one after another run in that order only where their
-// accumulator and shape are the same, so the accumulators form three blocks
-// (d = 0, 1 .. 3, 4 .. 6) and every product writes one whole block: digit i of Y
-// meets slices d - i, those below 0 being zeros ahead of the operand's own (24
-// products a stage instead of 56, a fifth of their columns zeros).
+// accumulator and shape are the same, so the accumulators form two or three
+// blocks and every product writes one whole block: digit i of Y meets slices
+// d - i, those below 0 being zeros ahead of the operand's own (18 or 24 products
+// a stage instead of 56, a third or a fifth of their columns zeros).
 // Forming Y on the fly keeps its 7 x 2 bytes per element out of memory.  Pairs
 // are sorted by their largest n_x, so the columns beyond the k-sphere are
 // skipped (a third of the product).
@@ -69,13 +69,17 @@ namespace {
 constexpr int TM = 128;      // rows of D per CTA
 constexpr int TK = 32;       // terms per stage
 constexpr int NSL = 7;       // digits per operand
-constexpr int ZSL = 2;       // slices of zeros ahead of the right operand's
-constexpr int BSL = ZSL + NSL;
 constexpr int WIN = 4;       // stages per exact window: 128 terms
 constexpr int ET = 512;      // threads that form the left operand
 constexpr int CW = 3;        // warps that copy the right operand
 constexpr int CTA = ET + 32 + 32 * CW;
 constexpr int NT_MAX = 64;   // columns per CTA: 7 x 64 of 512 TMEM columns
+// slices of zeros ahead of the right operand's with n columns a slice (product
+// below), and the rows of 8 terms of all of them where a tile has nt columns
+__host__ __device__ constexpr int zeros(int n) { return n <= 48 ? 4 : 2; }
+__host__ __device__ constexpr int ring_rows(int nt) {
+  return (zeros(nt) + NSL) * nt;  // 64 columns: more than 48 of its columns take
+}
 constexpr int A_KO = TM * 16 + 32;              // bytes between 8-term groups
 constexpr int A_SLICE = TK / 8 * A_KO;          // bytes
 constexpr int A_STAGE = NSL * A_SLICE;
@@ -204,39 +208,52 @@ __device__ __forceinline__ void mma_f16(unsigned lead, unsigned d, uint64_t a,
       "l"(a), "l"(b), "r"(idesc), "r"((unsigned)add), "r"(lead)
       : "memory");
 }
-// The products of 16 terms: digit i of Y on the slices from `b` on (ZSL is digit
-// 0's), `len` of them, into the accumulators d0 .. d0 + len - 1, for
-// d0 + len > i; three blocks of accumulators, digits ascending.
+// The products of 16 terms: digit i of Y on the slices from `b` on (digit 0's
+// follows the zeros), `len` of them, into the accumulators d0 .. d0 + len - 1, for
+// d0 + len > i; digits ascending.  The blocks are as few as 256 columns a product
+// and the shared memory for the zeros allow: what a stage takes goes with the
+// number of products more than with their width.  Forces of 8,000 waters (48
+// columns): two blocks, 9 products of 39 slices' width, 1,616 us; 12 of 34, 1,672;
+// 16 of 31, 1,744; seven blocks, 28 of 28, 2,053.
 struct Product {
   int i, d0, len, b;
 };
-constexpr int NPROD = 12;
-constexpr Product product(int k) {
-  const int d0[3] = {0, 1, 4}, len[3] = {1, 3, 3};
+constexpr Product product(int n, int k) {
+  const int wide[2] = {0, 2}, three[3] = {0, 1, 4};
+  const int blocks = n <= 48 ? 2 : 3;
   for (int i = 0; i < NSL; ++i)
-    for (int g = 0; g < 3; ++g)
-      if (i < d0[g] + len[g] && k-- == 0)
-        return {i, d0[g], len[g], ZSL + d0[g] - i};
+    for (int g = 0; g < blocks; ++g) {
+      const int d0 = n <= 48 ? wide[g] : three[g];
+      const int end = g + 1 == blocks ? NSL : n <= 48 ? wide[g + 1] : three[g + 1];
+      if (i < end && k-- == 0)
+        return {i, d0, end - d0, zeros(n) + d0 - i};
+    }
   return {0, 0, 0, 0};
+}
+constexpr int products(int n) {
+  int k = 0;
+  while (product(n, k).len)
+    ++k;
+  return k;
 }
 // Products that share a column have the same accumulator and shape; the first of
 // each block (which overwrites it) comes before the others; every i + j < NSL
 // is in exactly one; and none leaves the operand's slices or 256 columns.
-constexpr bool products_ordered() {
+constexpr bool products_ordered(int n) {
   int met[NSL][NSL] = {};
-  for (int k = 0; k < NPROD; ++k) {
-    const Product p = product(k);
-    if (p.len < 1 || p.len * NT_MAX > 256 || p.b < 0 || p.b + p.len > BSL)
+  for (int k = 0; k < products(n); ++k) {
+    const Product p = product(n, k);
+    if (p.len * n > 256 || p.b < 0 || p.b + p.len > zeros(n) + NSL)
       return false;
     for (int m = 0; m < k; ++m) {
-      const Product o = product(m);
+      const Product o = product(n, m);
       const bool share = o.d0 < p.d0 + p.len && p.d0 < o.d0 + o.len;
       if (share && (o.d0 != p.d0 || o.len != p.len || o.i >= p.i))
         return false;
     }
     for (int d = p.d0; d < p.d0 + p.len; ++d) {
-      const int j = p.b + d - p.d0 - ZSL;
-      if (p.i + (j < 0 ? d - p.i : j) != d || (j >= 0 && ++met[p.i][j] > 1))
+      const int j = p.b + d - p.d0 - zeros(n);
+      if (j >= 0 && (p.i + j != d || ++met[p.i][j] > 1))
         return false;
     }
   }
@@ -244,24 +261,27 @@ constexpr bool products_ordered() {
     for (int j = 0; i + j < NSL; ++j)
       if (!met[i][j])
         return false;
-  return product(NPROD).len == 0;
+  return true;
 }
-static_assert(products_ordered(), "products of one accumulator out of order");
+static_assert(products_ordered(16) && products_ordered(32) &&
+                  products_ordered(48) && products_ordered(64) && NT_MAX == 64,
+              "products of one accumulator out of order");
 
 // All products of a stage with N columns a slice.
 template <int N>
 __device__ __forceinline__ void mma_stage(unsigned lead, unsigned tmem,
                                           unsigned sa, unsigned sb, bool open) {
-  const uint64_t da = smem_desc(sa, A_KO), db = smem_desc(sb, BSL * N * 16);
+  constexpr int B_ROWS = (zeros(N) + NSL) * N;
+  const uint64_t da = smem_desc(sa, A_KO), db = smem_desc(sb, B_ROWS * 16);
 #pragma unroll
   for (int ks = 0; ks < TK / 16; ++ks)
 #pragma unroll
-    for (int k = 0; k < NPROD; ++k) {
+    for (int k = 0; k < products(N); ++k) {
       constexpr unsigned I0 = 1u << 4 | (unsigned)(TM / 16) << 24;
-      const Product p = product(k);
+      const Product p = product(N, k);
       mma_f16(lead, tmem + p.d0 * N,
               da + (ks * (2 * A_KO) + p.i * A_SLICE >> 4),
-              db + (uint64_t)(ks * (2 * BSL * N) + p.b * N),
+              db + (uint64_t)(ks * (2 * B_ROWS) + p.b * N),
               I0 | (unsigned)(p.len * N >> 3) << 17, ks || p.i || !open);
     }
 }
@@ -393,7 +413,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
   __shared__ int s_bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int piece = A.nt * 16;  // bytes of one slice of 8 terms in A.b
-  const int b_stage = 4 * NSL * piece, b_ring = 4 * BSL * piece;
+  const int b_stage = 4 * NSL * piece, b_ring = 4 * 16 * ring_rows(A.nt);
   unsigned char *const smem_b = smem + 2 * A_STAGE;  // three stages
   const int ct = blockIdx.z;
   // columns needed where the largest n_x is nx
@@ -505,10 +525,11 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
     auto copy = [&](int it) {
       const int n16 = window_cols(it) >> 4;
       unsigned char *const ring = smem_b + it % 3 * b_ring;
+      const int z16 = zeros(16 * n16) * n16;
       if (it < 3 || n16 != window_cols(it - 3) >> 4) {
-        const int nz = ZSL * 16 * n16;  // 16-byte rows a group
+        const int nz = 16 * z16;  // 16-byte rows a group
         for (int r = ctid; r < 4 * nz; r += 32 * CW)
-          reinterpret_cast<uint4 *>(ring)[r / nz * (BSL * 16 * n16) + r % nz] =
+          reinterpret_cast<uint4 *>(ring)[r / nz * (nz + NSL * 16 * n16) + r % nz] =
               make_uint4(0, 0, 0, 0);
       }
       const unsigned dst = smem_u32(ring) + (ctid & 15) * 16;
@@ -523,7 +544,7 @@ __global__ void __launch_bounds__(CTA, 1) k_ewald_split(SplitArgs A) {
         const unsigned q = (ctid >> 4) + 2 * CW * k;
         const unsigned r = q * inv >> 16;
         if (q < total)
-          copy16(dst + (q + (r / NSL + 1) * ZSL * n16) * 256,
+          copy16(dst + (q + (r / NSL + 1) * z16) * 256,
                  src + r * piece + (q - r * n16) * 256);
       }
     };
@@ -913,7 +934,7 @@ Shape shape_of(int kmax) {
   s.ncol = s.nt * s.nct;
   return s;
 }
-int stage_smem(int nt) { return 2 * A_STAGE + 3 * BSL * nt * TK * 2; }
+int stage_smem(int nt) { return 2 * A_STAGE + 3 * 4 * 16 * ring_rows(nt); }
 
 // bits to the right of the point such that `terms` values of at most 1 fit
 // 62 bits
