@@ -675,9 +675,9 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
       for (int w = 0; w < 2; ++w) {
         const double *cf = src[w]->data() + (size_t)seg * (ETAB_DEG + 1);
         double *o = pt.data() + ((size_t)seg * 2 + w) * 8;
-        const float hi[4] = {(float)cf[6], (float)cf[7], (float)cf[8], 0.0f};
-        std::memcpy(o, cf, 6 * sizeof(double));
-        std::memcpy(o + 6, hi, sizeof(hi));
+        const float hi[2] = {(float)cf[7], (float)cf[8]};
+        std::memcpy(o, cf, 7 * sizeof(double));
+        std::memcpy(o + 7, hi, sizeof(hi));
       }
     if ((rc = Alloc(&d_pt, pt.size())) ||
         (rc = up(d_pt, pt.data(), pt.size() * sizeof(double))) ||

@@ -101,7 +101,7 @@ __device__ __forceinline__ unsigned turn_wrap(const uint32_t *tp, uint4 f) {
 // pass over the pair list): the minimum image from the listed wrap bits
 // (the same FP64 differences: x - L is x + (-L)), added only where a lane
 // has one; the neighbour's charge stored times QQ_FACT; comparisons on the
-// bits; degrees 6-8 of the erfc(alpha r)/r segment in FP32 (pair_poly_at);
+// bits; degrees 7 and 8 of the erfc(alpha r)/r segment in FP32 (pair_poly_at);
 // and -- where every kind pair has the 12-6 form -- 1 / r^2 from the FP32
 // reciprocal by one cubic step (relative error below 2^-60 before the final
 // rounding) with sigma^2 / r^2 as a product, for pairs with an epsilon.
@@ -132,7 +132,7 @@ __device__ __forceinline__ double erfc_over_r_tab(const FF &ff,
   if (tab == nullptr || (unsigned)seg >= (unsigned)ff.etab_nseg)
     return erfc_over_r_far(&ff, s);
   const double2 *c = (const double2 *)(tab + (size_t)seg * 8);
-  return pair_poly_at(bits, c[0], c[1], c[2], *(const float4 *)(c + 3));
+  return pair_poly_at(bits, c[0], c[1], c[2], c[3]);
 }
 
 // One pair's terms, signed for the side (new position +, old -): false

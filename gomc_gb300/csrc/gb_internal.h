@@ -65,7 +65,7 @@ struct FF {
   // the same on the same segments in the layout of the pair walks, with the
   // Coulomb force factor of FFParticle::CalcCoulombVir, (erfc(alpha r) / r +
   // 2 alpha / sqrt(pi) exp(-alpha^2 r^2)) / r^2: per segment 64 bytes of each,
-  // degrees 0-5 in FP64 and degrees 6-8 in FP32 (and a pad)
+  // degrees 0-6 in FP64 and degrees 7 and 8 in FP32
   const double *pair_tab;
   int etab_key0, etab_nseg;
   // soft-core settings at lambda < 1 (Forcefield::sc_*,

@@ -140,18 +140,24 @@ __device__ __forceinline__ bool in_fast_range(double s) {
 }
 
 // A segment polynomial of ff.pair_tab at the position u in [-1, 1) that the
-// bits b of r^2 give: degrees 0-5 in FP64, 6-8 (f.x, f.y, f.z) in FP32, where
-// they add less than 1e-9 of the value.
+// bits b of r^2 give: degrees 0-6 in FP64, 7 and 8 (the halves of c6.y) in FP32.
+// Those two add less than 1e-11 of the value for alpha r up to 3.4 (a tolerance of
+// 1e-5; 1.2e-9 up to 4.8, 1e-10), so their rounding is below 2^-60 (2^-53) of it:
+// against 113 bits over r from 0.7 A to Rcut the largest and the rms error are
+// those of nine FP64 degrees to four digits (2.2e-16 and 6.6e-17; 2.8e-16 and
+// 7.1e-17 at 1e-10).  With degree 6 in FP32 too the largest was 5.6e-16 at 1e-10.
 __device__ __forceinline__ double pair_poly_at(long long b, double2 c01,
                                                double2 c23, double2 c45,
-                                               float4 f) {
+                                               double2 c6) {
   const double u = fma(
       2.0, __longlong_as_double(((b << 6) & 0x000fffffffffffffLL) |
                                 0x3ff0000000000000LL), -3.0);
   const float uf = fmaf(
       2.0f, __int_as_float(((int)(b >> 23) & 0x007fffff) | 0x3f800000), -3.0f);
-  const float t = fmaf(fmaf(f.z, uf, f.y), uf, f.x);
-  double p = fma(widen_f64(t), u, c45.y);
+  const long long f = bits64(c6.y);
+  const float t = fmaf(__int_as_float((int)(f >> 32)), uf, __int_as_float((int)f));
+  double p = fma(widen_f64(t), u, c6.x);
+  p = fma(p, u, c45.y);
   p = fma(p, u, c45.x);
   p = fma(p, u, c23.y);
   p = fma(p, u, c23.x);
@@ -170,7 +176,7 @@ __device__ __forceinline__ bool pair_poly(const FF &ff, int which, double s,
     return false;
   const double2 *c = (const double2 *)(ff.pair_tab + ((size_t)seg * 2 + which) * 8);
   *out = pair_poly_at(b, __ldg(c), __ldg(c + 1), __ldg(c + 2),
-                      __ldg((const float4 *)(c + 3)));
+                      __ldg(c + 3));
   return true;
 }
 // Soft-core squared distance at coupling lambda (src/FFParticle.cpp:301-308):

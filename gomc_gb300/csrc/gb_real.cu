@@ -108,8 +108,7 @@ __global__ void __launch_bounds__(RCT) k_reduce_cols(const double *__restrict__ 
 //     shift is added only where a lane of the batch needs one, Lennard-Jones
 //     terms are skipped for a batch without any (a hydrogen's whole walk),
 //     1 / r^2 starts from the FP32 reciprocal, and of the Coulomb segment
-//     polynomial only degrees 0-5 are FP64 (degrees 6-8 add less than 1e-9 of
-//     the value, so their FP32 rounding stays below 1e-16 of it).
+//     polynomial degrees 0-6 are FP64 (pair_poly_at).
 // One CTA of four warps takes every (grid.y * 4)-th atom of a cell; grid.y is
 // set so that a warp has one atom in small boxes and up to eight in large
 // ones (pair_split).  Measured on 8,000 waters, Rcut 10 A, against one CTA

@@ -159,3 +159,39 @@ def test_lj_term_to_the_last_bits(gb):
         bar = 19 * Fraction(1, 2 ** 53) * e4 * (x * x + x)
         assert abs(Fraction(got) - e4 * (x * x - x)) <= bar, (d, got)
     box.close()
+
+
+@pytest.mark.parametrize("tol", [1e-5, 1e-10])
+def test_ewald_term_to_the_last_bits(gb, tol):
+    """One pair's real-space Ewald energy near the cutoff, where the segment
+    polynomial bends most, against 40 digits.
+
+    r^2 is exact (as above) and the charge product is taken as the call rounds
+    it.  The polynomial interpolates to 1.1e-16 of the value, its constant term,
+    last step and the product with the charges round by 1.1e-16 each, and the
+    lower terms, a fifth of the value at most, by a fifth of that."""
+    mp = pytest.importorskip("mpmath")
+    import math
+    mp.mp.dps = 40
+    edge, rc, qa, qb = 64.0, 10.0, 0.75, -0.5
+    s = MolSystem(np.full(3, edge), [AtomKind("A", 0.0, 2.9, 12.0)],
+                  [MoleculeType("T", ["X"], [0], [qa])],
+                  np.array([[16.0, 16.0, 16.0], [60.0, 60.0, 60.0]]),
+                  np.zeros(2, np.int32), np.array([qa, qb]),
+                  np.arange(2, dtype=np.int32), np.arange(3, dtype=np.int32),
+                  np.zeros(2, np.int32))
+    box = gb.Box(s, SimConfig(temperature=298.0, rcut=rc, tolerance=tol))
+    box.cell_remove_mol(1)
+    unit = 2.0 ** -20
+    r = np.rint(np.random.default_rng(9).uniform(8.5, 9.99, 16384) / unit) * unit
+    re = np.concatenate([
+        box.particle_inter(1, 0, np.stack([16.0 + c, 0 * c + 16.0, 0 * c + 16.0],
+                                          -1))[2]
+        for c in np.array_split(r, 64)])
+    alpha = mp.mpf(math.sqrt(-math.log(tol)) / rc)
+    qq = mp.mpf((qb * 167103.208067979) * qa)
+    bar = (1.1 + 3 * 1.1 + 0.2 * 1.1) * 1e-16
+    for d, got in zip(r, re):
+        want = qq * mp.erfc(alpha * mp.mpf(d)) / mp.mpf(d)
+        assert abs(mp.mpf(got) - want) <= bar * abs(want), d
+    box.close()
