@@ -603,17 +603,9 @@ int Box::Init(const HostSystem &s0, const BoxConfig &c) {
   double half[3] = {s.L[0] * 0.5, s.L[1] * 0.5, s.L[2] * 0.5};
   calc_com(s);
   build_ff(s, c, &ff);
-  double qmax = 0.0, qsum = 0.0;
-  for (int i = 0; i < N; ++i) {
-    if (!std::isfinite(s.q[i])) {
-      q_odd = true;
-      continue;
-    }
-    qmax = std::max(qmax, std::fabs(s.q[i]));
-    qsum += std::fabs(s.q[i]);
-  }
-  std::frexp(qmax, &q_exp);
-  q_abs = std::ldexp(qsum, -q_exp);
+  for (int i = 0; i < N; ++i)
+    q_odd = q_odd || !std::isfinite(s.q[i]);
+  q_class = charge_classes(s.q);
   DevBox &d = dev;
   for (int k = 0; k < 3; ++k) {
     d.L[k] = s.L[k];

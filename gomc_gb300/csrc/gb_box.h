@@ -41,6 +41,15 @@ struct TrialState {
   std::vector<void *> allocs;
 };
 
+// Charges of 2^bottom <= |q| < 2^exp, and their sum in units of 2^exp.
+struct ChargeClass {
+  int exp = 0, bottom = 0;
+  double abs = 0.0;
+};
+// The classes that the structure factor takes in passes of their own, largest
+// first (gb_ewald.cu).
+std::vector<ChargeClass> charge_classes(const std::vector<double> &q);
+
 struct BoxConfig {
   double temperature = 298.0;
   double rcut = 9.0, rcut_low = 0.0, rcut_coulomb = 9.0, tolerance = 1e-5;
@@ -150,11 +159,10 @@ class Box {
 
   unsigned sums_spin = SUMS_SPIN;  // polls of a wait of the Ewald sums
 
-  // charges: |q| < 2^q_exp, and their sum in units of 2^q_exp, without those
-  // that are infinite or not a number (q_odd: there are some)
-  int q_exp = 0;
+  // charges by size (ChargeClass), without those that are infinite or not a
+  // number (q_odd: there are some)
+  std::vector<ChargeClass> q_class;
   bool q_odd = false;
-  double q_abs = 0.0;
 
   // scratch buffers
   double *d_scratch = nullptr;   // reduction partials

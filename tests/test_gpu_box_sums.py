@@ -212,3 +212,33 @@ def test_charge_that_is_not_finite(gb, value):
     np.testing.assert_array_equal(np.isfinite(box.virial()),
                                   np.isfinite(ref.virial()))
     box.close()
+
+
+def test_structure_factor_of_unequal_charges(gb):
+    """Two charges of 2 among 2,998 a thousand times smaller: a term is within
+    2^-51 of the power of two above the charges of its own size (four terms an
+    atom and part, as above), and the sum is rounded once for each size."""
+    n, edge = 3000, 44.0
+    rng = np.random.default_rng(2)
+    q = np.where(np.arange(n) % 2, 1e-3, -1e-3)
+    q[[5, 1700]] = 2.0, -2.0
+    s = MolSystem(np.full(3, edge), [AtomKind("A", 0.0, 2.9, 12.0)],
+                  [MoleculeType("T", ["X"], [0], [0.0])],
+                  rng.random((n, 3)) * edge, np.zeros(n, np.int32), q,
+                  np.arange(n, dtype=np.int32),
+                  np.arange(n + 1, dtype=np.int32), np.zeros(n, np.int32))
+    box = gb.Box(s, SimConfig(temperature=298.0, rcut=9.0, tolerance=1e-5))
+    box.system_total()
+    sr, si = box.sums_new()
+    kv = box.kvectors()
+    pick = rng.permutation(len(sr))[:1500]
+    k = np.rint(np.stack([kv[c] for c in ("kx", "ky", "kz")], 1)[pick] * edge /
+                (2 * np.pi)).astype(np.longdouble)
+    turns = np.asarray(box.coords(), np.longdouble) / np.longdouble(edge)
+    t = k @ turns.T
+    a = (t - np.rint(t)) * np.longdouble("6.28318530717958647692528676655900577")
+    ql = q.astype(np.longdouble)
+    bar = 2.0 ** -49 * (2 * 4.0 + 2998 * 2.0 ** -9) + 2 * 2.0 ** -53 * 4.1
+    assert np.abs(sr[pick] - np.cos(a) @ ql).max() <= bar
+    assert np.abs(si[pick] - np.sin(a) @ ql).max() <= bar
+    box.close()
