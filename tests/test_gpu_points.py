@@ -195,3 +195,21 @@ def test_ewald_term_to_the_last_bits(gb, tol):
         want = qq * mp.erfc(alpha * mp.mpf(d)) / mp.mpf(d)
         assert abs(mp.mpf(got) - want) <= bar * abs(want), d
     box.close()
+
+
+@pytest.mark.parametrize("n", [64, 65, 151, 152, 153, 256])
+def test_trial_counts_agree(gb, n):
+    """A trial's energies do not depend on how many others the call has (and so
+    on how many CTAs a trial gets) beyond the order of its sums: 1e-13 of the
+    sum of the terms' sizes, some 400 terms in FP64."""
+    s = mixture((301, 230, 17), (27.3, 31.1, 64.7), 11)
+    box = gb.Box(s, SimConfig(temperature=298.0, rcut=9.0, tolerance=1e-5))
+    box.cell_remove_mol(3)
+    t = np.random.default_rng(5).random((n, 3)) * s.box
+    ov, lj, re = box.particle_inter(3, 0, t)
+    for i in range(0, n, 7):
+        o, l, r = box.particle_inter(3, 0, t[i:i + 1])
+        assert o[0] == ov[i]
+        assert abs(l[0] - lj[i]) <= 1e-13 * max(abs(l[0]), 1e3)
+        assert abs(r[0] - re[i]) <= 1e-13 * max(abs(r[0]), 1e5)
+    box.close()
