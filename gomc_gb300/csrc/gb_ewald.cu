@@ -314,7 +314,7 @@ struct PhaseArgs {
   int2 *yz;            // [2][kmax + 1][2][nap]
   unsigned char *xs;   // slices, or NULL
   double *xd;          // FP64 rows, or NULL
-  int nt, nct;         // columns per CTA, column tiles
+  int nt;              // columns per CTA
 };
 
 __global__ void __launch_bounds__(128) k_ewald_phases(PhaseArgs A) {
@@ -957,7 +957,6 @@ PhaseArgs phase_args(const Box &bx, const DevBox &b, const double *x,
     P.L[d] = b.L[d];
   P.kmax = b.kmax;
   P.nt = sh.nt;
-  P.nct = sh.nct;
   return P;
 }
 

@@ -20,27 +20,10 @@ constexpr int RT = 128;  // threads per real-space CTA
 
 // Sum `n` partials of width `w` (stride w) into out[0..w), fixed order.
 __global__ void k_reduce_partials(const double *__restrict__ part, int n, int w,
-                                  double *out, int max_mode) {
+                                  double *out) {
   __shared__ double sh[RT / 32];
   for (int c = 0; c < w; ++c) {
     double v = 0.0;
-    if (max_mode && c == w - 1) {
-      for (int i = threadIdx.x; i < n; i += RT)
-        v = fmax(v, part[(size_t)i * w + c]);
-      for (int o = 16; o > 0; o >>= 1)
-        v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-      if ((threadIdx.x & 31) == 0)
-        sh[threadIdx.x >> 5] = v;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double r = 0;
-        for (int i = 0; i < RT / 32; ++i)
-          r = fmax(r, sh[i]);
-        out[c] = r;
-      }
-      __syncthreads();
-      continue;
-    }
     for (int i = threadIdx.x; i < n; i += RT)
       v += part[(size_t)i * w + c];
     double r = block_sum<RT>(v, sh);
@@ -667,7 +650,7 @@ int launch_single_mol_inter(Box &bx, int m, const double *d_lam4,
     return rc;
   k_single_mol_inter<<<units, RT, 0, bx.stream>>>(bx.dev, bx.d_ff, m, d_lam4,
                                                   bx.d_scratch);
-  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, units, 4, d_out4, 0);
+  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, units, 4, d_out4);
   return bx.CudaCheck(cudaGetLastError(), "single molecule inter");
 }
 
@@ -707,7 +690,7 @@ int launch_correction(Box &bx, double *d_out) {
   if (rc)
     return rc;
   k_correction<<<nb, RT, 0, bx.stream>>>(bx.dev, bx.d_ff, bx.d_scratch);
-  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, nb, 1, d_out, 0);
+  k_reduce_partials<<<1, RT, 0, bx.stream>>>(bx.d_scratch, nb, 1, d_out);
   return bx.CudaCheck(cudaGetLastError(), "correction");
 }
 
