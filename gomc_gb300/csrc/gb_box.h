@@ -60,8 +60,8 @@ struct BoxConfig {
   int sc_power = 0, sc_coul = 0;
   // atoms per pass of the box-wide Ewald sums (a multiple of 128), which bounds
   // their scratch, held for the box's life: 35 MB for 8,000 waters in one pass,
-  // 2.4 MB in passes of SUMS_BATCH_SERVED, which a server's jobs take (their
-  // sums come once per thousands of moves)
+  // 2.4 MB in passes of SUMS_BATCH_SERVED, which the jobs of a server with little
+  // memory take
   int sums_batch = 32768;
 };
 constexpr int SUMS_BATCH_SERVED = 1024;

@@ -17,8 +17,9 @@
 // jobs are retired at the start of the next round (final coordinates and
 // energies copied to the host, device memory returned to the budget).
 // A job's segment lengths depend only on the job (its quantum, recompute
-// frequency and step count), and its cluster size only on its own size, so
-// it computes the same moves with the same arithmetic alone or in any mix.
+// frequency and step count), its cluster size only on its own size, and the
+// passes of its Ewald sums on its size and the server's budget, so it computes
+// the same moves with the same arithmetic alone or in any mix.
 //
 // This has no counterpart in the reference, which runs one simulation per
 // process (src/Simulation.cpp:116-168).
@@ -171,7 +172,8 @@ void job_kvectors(const Job &j, int *K, int *kmax) {
 
 // Device bytes the job's box will hold (Box::Init + mc_init in the mixed
 // form, the move buffer sized to `moves`), from the same sizing rules.
-size_t job_bytes(const Job &j, int K, int kmax, int csize, size_t moves) {
+size_t job_bytes(const Job &j, int K, int kmax, int csize, size_t moves,
+                 int sums_batch) {
   const HostSystem &s = j.host;
   size_t N = s.n_atoms, M = s.n_mol;
   int edge[3];
@@ -211,10 +213,24 @@ size_t job_bytes(const Job &j, int K, int kmax, int csize, size_t moves) {
   // the other kernels' partials and allocation rounding
   size_t scratch =
       8 * std::max(recip_sums_scratch((int)N, kmax, (kmax + 1) * (kmax + 1),
-                                      SUMS_BATCH_SERVED),
+                                      sums_batch),
                    3 * (N + M)) +
       ((size_t)1 << 18);
   return box + mc + scratch + 96 * 512;
+}
+
+// Atoms per pass of a job's Ewald sums: all of them where a job that holds one
+// CTA slot may hold this much per slot and the resident jobs, which fill at most
+// two CTAs an SM, still take half the memory budget, so that memory is not what
+// stops an admission; else few (the rule knows the job and the server, not the
+// others, since sums over other passes round differently).  96 jobs of 500 to
+// 20,000 waters: 240,000 moves/s with one pass, 228,000 in passes of 1,024.
+int job_sums_batch(const Job &j, int K, int kmax, int csize, size_t moves,
+                   size_t budget, int sms) {
+  const int one = BoxConfig().sums_batch;
+  const size_t bytes = job_bytes(j, K, kmax, csize, moves, one);
+  return (double)bytes * 4 * sms <= (double)budget * csize ? one
+                                                           : SUMS_BATCH_SERVED;
 }
 
 // A job's host-side system and configuration, copied from the C structures.
@@ -250,7 +266,6 @@ Job *make_job(const gb_system_desc *sys, const gb_config *cfg) {
   c.electrostatic = cfg->electrostatic ? 1 : 0;
   c.precision = GB_MIXED;
   c.device = cfg->device;
-  c.sums_batch = SUMS_BATCH_SERVED;
   c.sc_alpha = cfg->sc_alpha;
   c.sc_sigma = cfg->sc_sigma;
   c.sc_power = cfg->sc_power;
@@ -258,15 +273,16 @@ Job *make_job(const gb_system_desc *sys, const gb_config *cfg) {
   return j;
 }
 
-// Admission estimate of a job: k-vectors, cluster size, device bytes.
+// Admission estimate of a job: k-vectors, cluster size, the device bytes it is
+// charged at least.
 size_t job_estimate(const Job &j, int quantum, int *csize_out) {
   int K, kmax;
   job_kvectors(j, &K, &kmax);
   int csize = job_cluster(j, K);
   if (csize_out)
     *csize_out = csize;
-  return job_bytes(j, K, kmax, csize,
-                   (size_t)job_quantum(quantum, K, csize));
+  return job_bytes(j, K, kmax, csize, (size_t)job_quantum(quantum, K, csize),
+                   SUMS_BATCH_SERVED);
 }
 
 }  // namespace
@@ -301,8 +317,9 @@ int Server::Admit() {
     int csize = job_cluster(*j, K);
     bool cold_smem = mixed_smem(K, kmax, csize, true) <= MIXED_SMEM_MAX;
     size_t smem = mixed_smem(K, kmax, csize, cold_smem);
-    size_t est =
-      job_bytes(*j, K, kmax, csize, (size_t)job_quantum(cfg.quantum, K, csize));
+    const size_t moves = (size_t)job_quantum(cfg.quantum, K, csize);
+    const int batch = job_sums_batch(*j, K, kmax, csize, moves, budget, slots.sms);
+    size_t est = job_bytes(*j, K, kmax, csize, moves, batch);
     std::lock_guard<std::mutex> g(mu);
     // CTA slots: shared memory and two CTAs per SM by registers
     size_t used_smem = 0;
@@ -330,6 +347,7 @@ int Server::Admit() {
     }
     queue.pop_front();
     j->csize = csize;
+    j->cfg.sums_batch = batch;
     j->quantum = job_quantum(cfg.quantum, K, csize);
     j->smem = smem;
     j->mem = est;

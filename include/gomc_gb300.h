@@ -450,7 +450,8 @@ int gb_mc_set_gomc_state(gb_box *box, const gb_gomc_chk *in);
  * memory fits `mem_budget` and their chains fit the GPU's free CTA slots,
  * and retires finished jobs (their final coordinates and running energies
  * are kept on the host).  A job's results do not depend on which other jobs
- * share its rounds.  Rounds run either on the caller's thread
+ * share its rounds; where mem_budget is short its Ewald sums take their atoms in
+ * smaller passes, which round differently.  Rounds run either on the caller's thread
  * (gb_server_step) or on a worker thread (gb_server_start .. gb_server_drain);
  * gb_server_submit may be called from any thread at any time. */
 typedef struct gb_server gb_server;
@@ -480,8 +481,9 @@ void gb_server_destroy(gb_server *srv);
 int gb_server_submit(gb_server *srv, const gb_system_desc *sys,
                      const gb_config *cfg, const gb_mc_params *mc,
                      int64_t nsteps, int64_t sweep_moves, int64_t *job_id);
-/* The device bytes the server would reserve for such a job at admission
- * (its memory estimate) and the CTAs per chain it would give it. */
+/* The device bytes the server would reserve at least for such a job at admission
+ * (its memory estimate; more, for faster Ewald sums, where mem_budget is ample)
+ * and the CTAs per chain it would give it. */
 int gb_server_estimate(gb_server *srv, const gb_system_desc *sys,
                        const gb_config *cfg, const gb_mc_params *mc,
                        int64_t *bytes, int32_t *ctas_per_chain);

@@ -113,7 +113,7 @@ def test_memory_admission(srv_mod):
 
 
 # device bytes a job was charged while the structure factor's scratch was K and
-# N sized (1.1 to 2.9 MB); passes of atoms hold it there
+# N sized (1.1 to 2.9 MB); passes of atoms hold it there where memory is short
 @pytest.mark.parametrize("n,rcut,bytes_", [
     (300, 9.0, 2505204), (700, 9.0, 3165020), (2000, 9.0, 7329576),
     (8000, 10.0, 22555480), (20000, 9.0, 61603852)])
@@ -123,6 +123,21 @@ def test_job_memory(srv_mod, n, rcut, bytes_):
     est = srv.estimate(spce_water_box(n, water_box_length(n), seed=1), cfg)
     assert est["bytes"] <= 1.12 * bytes_
     srv.close()
+
+
+def test_short_memory_gives_the_same_ensemble_start(srv_mod):
+    """A job whose Ewald sums take their atoms in passes (a small budget) starts
+    from the energies of one that takes them at once: sums over other passes
+    round differently, by less than 1e-13 of the energy."""
+    ends = []
+    for budget in (0, 64 << 20):
+        srv = srv_mod.Server(quantum=400, mem_budget=budget)
+        i = srv.submit(system(2000, 3), CFG, seed=7, nsteps=1,
+                       scales=[0.0, 0.0, 0.02, 0.03], adj_steps=500)
+        srv.run_until_idle()
+        ends.append(srv.result(i)["energy"])
+        srv.close()
+    np.testing.assert_allclose(ends[1], ends[0], rtol=1e-13)
 
 
 def test_worker_thread(srv_mod):
