@@ -95,16 +95,6 @@ __device__ __forceinline__ unsigned turn_wrap(const uint32_t *tp, uint4 f) {
   return w;
 }
 
-// pair_term of the chain with two moves in flight, with fewer FP64
-// instructions (a warp's FP64 instruction holds its SM sub-partition's FP64
-// unit for about 64 cycles on GB300, so their count sets the time of a
-// pass over the pair list): the minimum image from the listed wrap bits
-// (the same FP64 differences: x - L is x + (-L)), added only where a lane
-// has one; the neighbour's charge stored times QQ_FACT; comparisons on the
-// bits; degrees 7 and 8 of the erfc(alpha r)/r segment in FP32 (pair_poly_at);
-// and -- where every kind pair has the 12-6 form -- 1 / r^2 from the FP32
-// reciprocal by one cubic step (relative error below 2^-60 before the final
-// rounding) with sigma^2 / r^2 as a product, for pairs with an epsilon.
 // The force field's pair tables held in shared memory by the chain with two
 // moves in flight: the erfc(alpha r)/r segments in the layout of FF::pair_tab
 // without the force factors (NULL: read from global memory) and the LJ
@@ -135,8 +125,15 @@ __device__ __forceinline__ double erfc_over_r_tab(const FF &ff,
   return pair_poly_at(bits, c[0], c[1], c[2], c[3]);
 }
 
-// One pair's terms, signed for the side (new position +, old -): false
-// outside the cutoff.  a, side: the moved atom and whether its new position;
+// One pair's terms, with fewer FP64 instructions than pair_term (a warp's FP64
+// instruction holds its SM sub-partition's FP64 unit for about 64 cycles on
+// GB300, so their count sets the time of a pass over the pair list): the minimum
+// image from the listed wrap bits (the same FP64 differences: x - L is x + (-L)),
+// added only where a lane has one; the neighbour's charge stored times QQ_FACT;
+// comparisons on the bits; degrees 7 and 8 of the erfc(alpha r)/r segment in FP32
+// (pair_poly_at); and -- where every kind pair has the 12-6 form -- sigma^2 / r^2
+// as a product with recip_cubic, for pairs with an epsilon.
+// Signed for the side (new position +, old -): false outside the cutoff.  a, side: the moved atom and whether its new position;
 // pzq: the neighbour's z and charge times QQ_FACT.
 __device__ __forceinline__ bool pair_energy_pipe(const ChainArgs &A,
                                                  const double *hdr, int a,

@@ -19,14 +19,19 @@
 // component.  On the FP64 pipe (two lanes per SM and clock) they cannot run
 // below 2 ms / 6 ms on 8,000 waters; FP32 pairs would cost accuracy.  Instead
 // both factors are 55-bit fixed-point numbers cut into seven signed 8-bit
-// digits, held exactly in FP16: a product of digit i and digit j is exact,
-// sums over 128 terms of the digit pairs with i + j = d stay below 2^24 and
-// are exact in the FP32 accumulators, so 28 tcgen05 products (d = 0..6)
-// give the sum to 2^-53 of the largest term.  The seven accumulators (d) sit
-// side by side in tensor memory; every 128 terms the CTA adds them into one
-// 64-bit integer per output.  Integer sums do not depend on their order, so
-// chunks of atoms are added by 64-bit integer atomics and results are equal
-// run to run.
+// digits, held exactly in FP16 (the scheme of Ozaki, Ogita, Oishi and Rump,
+// Numer. Algorithms 59 (2012) 95, with digits of a fixed scale): a product of
+// digit i and digit j is exact, and sums over 128 terms of the digit pairs with
+// i + j = d stay below 2^24 and are exact in the FP32 accumulators of d = 0..6.
+// Pairs with i + j >= 7 are left out: with the rounding of the factors a term is
+// within 2^-51 of the unit (the power of two above the largest charge of its
+// class, or above a column's largest C), some 2^-54 rms, and the errors of n terms
+// add up as sqrt(n).  Measured against sums of exact phases, in units of the sums'
+// rms: 3.8e-16 (256 waters), 5.5e-16 (8,000), 8.3e-16 (20,000), where an FP64
+// recurrence had 2.3e-15, 1.0e-14 and 1.3e-14.  The seven accumulators sit side by
+// side in tensor memory; every 128 terms the CTA adds them into one 64-bit integer
+// per output.  Integer sums do not depend on their order, so chunks of atoms are
+// added by 64-bit integer atomics and results are equal run to run.
 //
 // A CTA has 128 rows of D and up to 64 columns, one CTA per SM (two stages of
 // 32 terms of Y and three of the other operand in shared memory).  Sixteen
@@ -45,11 +50,11 @@
 // Forming Y on the fly keeps its 7 x 2 bytes per element out of memory.  Pairs
 // are sorted by their largest n_x, so the columns beyond the k-sphere are
 // skipped (a third of the product).
-// Measured on 8,000 waters (24,658 k-vectors), per launch: sums 131 us, forces
-// 390 us (the FP64 kernels before: 11 ms and 12.1 ms); sums of 20,000 waters
-// 624 us.  A stage takes some 3,600 cycles: its products 1,250 (22-31 % of the
-// tensor peak as counted), issue of the warps that form Y and add the windows
-// 1,900 a scheduler, the rest their load latency.
+// Measured on 8,000 waters (24,658 k-vectors), per launch: sums 141 us, forces
+// 429 us (the FP64 kernels before: 11 ms and 12.1 ms); sums of 20,000 waters
+// 692 us.  A stage takes some 3,900 cycles: its products read 193 KB of shared
+// memory (1,510 cycles) and keep the tensor pipe 39-42 % busy; the warps that form
+// Y and add the windows issue 56 % of the cycles, the rest is their load latency.
 //
 // Phases: u = (x / L) 2^64 is a fraction of a turn to 2^-64, n u is exact
 // integer arithmetic, and cos and sin come from their Taylor series in 62-bit

@@ -404,7 +404,8 @@ struct ChainArgs {
   double *prop;   // [n][12]
   int64_t first;
   int n;
-  double *part;   // [2][grid][4], by move parity
+  double *part;   // [2][grid][4], by move parity; two moves in flight
+                  // [3][grid][8], by move modulo 3, four on each outcome
   unsigned *bar;  // [0..1] grid barrier
   unsigned *seq;  // [0] decision published (2 (t + 1) + accept); from
                   // SEQ_CTX: per CTA, its part of the context of move t

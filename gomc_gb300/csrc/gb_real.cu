@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(RCT) k_reduce_cols(const double *__restrict__ 
 // per cell pair (energies, virial) or per third of a neighbour shell
 // (forces): the calls forces + reciprocal + torque 31.4 -> 24.6 ms, virial
 // 15.9 -> 12.7 ms; SystemTotal of 20,000 waters 72.9 -> 70.6 ms.  Per launch
-// now: forces 774 us and virial 515 us (8,000 waters), energies 815 us
-// (20,000), the FP64 pipe 83 % busy (72-76 % with the last wave).
+// now: forces 782 us and virial 509 us (8,000 waters), energies 776 us
+// (20,000), the FP64 pipe 83 % busy (75-78 % with the last wave).
 // ---------------------------------------------------------------------------
 constexpr int PW = RT / 32;  // warps per CTA
 constexpr int PQ = 64;       // queue slots per warp: one batch plus a scan step
