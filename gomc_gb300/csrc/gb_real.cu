@@ -387,12 +387,14 @@ int launch_box_inter_view(Box &bx, const DevBox &b, double *d_out2) {
 // CTAs of four warps (one a sub-partition, each with its FP64 unit to itself)
 // walk the 27 cells around a point with the FP32 scan and FP64 batches of the
 // pair walk, and the last CTA adds the points' sums and writes them to the
-// host's pinned memory.  With no more points than SMs a point has seven CTAs, a
+// host's pinned memory.  With no more trials than SMs a trial has seven CTAs, a
 // warp one cell and so one batch (2,400-sphere liquid, 10 trials: one CTA of nine
 // warps a point took 14.7 us, two batches a warp and two warps a sub-partition);
 // beyond, one, which fills its batches better.  us a call, seven CTAs / one: 65
 // trials 34 / 39 (8,000 waters 43 / 48), 100 37 / 40 (44 / 49), 152 40 / 41
-// (49 / 51), 200 45 / 42 (55 / 53), 256 51 / 42 (62 / 54).
+// (49 / 51), 200 45 / 42 (55 / 53), 256 51 / 42 (62 / 54).  A molecule's points
+// meet in one warp of the last CTA, so there the line is 64 points: molecules of
+// 33 sites 28.7 / 28.6, of 48 33.3 / 30.9, of 64 38.3 / 33.7.
 // ---------------------------------------------------------------------------
 constexpr int PTW = 4;       // warps per CTA
 constexpr int PT_SPLIT = 7;  // CTAs per point of a call of few points
@@ -552,7 +554,7 @@ template <bool MOL, int N>
 static int launch_points(Box &bx, const double *xyz, int n, int m, int kind,
                          double charge, const char *what) {
   const DevBox &b = bx.dev;
-  const int pts = MOL ? 2 * n : n, parts = pts <= bx.sm_count ? PT_SPLIT : 1;
+  const int pts = MOL ? 2 * n : n, parts = pts <= (MOL ? 64 : bx.sm_count) ? PT_SPLIT : 1;
   int rc = bx.EnsureScratch((size_t)3 * pts * parts);
   if (rc)
     return rc;
