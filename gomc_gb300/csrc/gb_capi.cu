@@ -268,7 +268,7 @@ int gb_get_sums_new(gb_box *box, double *sum_r, double *sum_i) {
   BOX_CALL(GetSumNew(sum_r, sum_i));
 }
 int gb_box_device_bytes(gb_box *box, int64_t *bytes) {
-  int rc = guard(box);
+  int rc = guard_box(box);
   if (rc || !bytes)
     return rc ? rc : (int)gb::ERR_ARG;
   *bytes = (int64_t)(box->b->dev_bytes + (box->b->mc ? box->b->mc->bytes : 0));

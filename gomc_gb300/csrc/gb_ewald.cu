@@ -978,8 +978,9 @@ void launch_phases(Box &bx, PhaseArgs &P, int atom0, int na) {
 // A term is rounded to 2^-54 of its class's 2^exp (and misses digit products of
 // that size), whatever its own charge, so the errors add up to 2^exp sqrt(n) for n
 // charges, beside sums of sqrt(sum q^2).  A class ends where that reaches
-// 4 sqrt(sum q^2) (water 1.7, where the sums' error is a sixth to a fifteenth of
-// an FP64 recurrence's): smaller charges then have a pass of their own.  Two ions
+// 8 sqrt(sum q^2) (water 1.7, where the sums' error is a sixth to a fifteenth of
+// an FP64 recurrence's; with divalent ions 6.6, still one pass): smaller charges
+// then have a pass of their own.  Two ions
 // of 2 among 60,000 of 0.001, one pass: error 4.1e-14 of the sums' rms and 4.4e-14
 // of the forces' (the FP64 kernels: 1.0e-14, 1.4e-14); two passes: 4.5e-16, 5.1e-15.
 std::vector<ChargeClass> charge_classes(const std::vector<double> &q) {
@@ -1009,7 +1010,7 @@ std::vector<ChargeClass> charge_classes(const std::vector<double> &q) {
     const int e = i + E0;
     count += n[i];
     if (out.empty() || std::ldexp(std::sqrt(count), out.back().exp) >
-                           4.0 * std::sqrt(sq)) {
+                           8.0 * std::sqrt(sq)) {
       out.push_back({e, e - 1, 0.0});
       count = n[i];
     }

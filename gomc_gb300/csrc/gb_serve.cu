@@ -219,18 +219,20 @@ size_t job_bytes(const Job &j, int K, int kmax, int csize, size_t moves,
   return box + mc + scratch + 96 * 512;
 }
 
-// Atoms per pass of a job's Ewald sums: all of them where a job that holds one
+// Atoms per pass of a job's Ewald sums, and the bytes the job then takes: all of them where a job that holds one
 // CTA slot may hold this much per slot and the resident jobs, which fill at most
 // two CTAs an SM, still take half the memory budget, so that memory is not what
 // stops an admission; else few (the rule knows the job and the server, not the
 // others, since sums over other passes round differently).  96 jobs of 500 to
 // 20,000 waters: 240,000 moves/s with one pass, 228,000 in passes of 1,024.
 int job_sums_batch(const Job &j, int K, int kmax, int csize, size_t moves,
-                   size_t budget, int sms) {
+                   size_t budget, int sms, size_t *bytes) {
   const int one = BoxConfig().sums_batch;
-  const size_t bytes = job_bytes(j, K, kmax, csize, moves, one);
-  return (double)bytes * 4 * sms <= (double)budget * csize ? one
-                                                           : SUMS_BATCH_SERVED;
+  *bytes = job_bytes(j, K, kmax, csize, moves, one);
+  if ((double)*bytes * 4 * sms <= (double)budget * csize)
+    return one;
+  *bytes = job_bytes(j, K, kmax, csize, moves, SUMS_BATCH_SERVED);
+  return SUMS_BATCH_SERVED;
 }
 
 // A job's host-side system and configuration, copied from the C structures.
@@ -317,9 +319,10 @@ int Server::Admit() {
     int csize = job_cluster(*j, K);
     bool cold_smem = mixed_smem(K, kmax, csize, true) <= MIXED_SMEM_MAX;
     size_t smem = mixed_smem(K, kmax, csize, cold_smem);
-    const size_t moves = (size_t)job_quantum(cfg.quantum, K, csize);
-    const int batch = job_sums_batch(*j, K, kmax, csize, moves, budget, slots.sms);
-    size_t est = job_bytes(*j, K, kmax, csize, moves, batch);
+    size_t est;
+    const int batch = job_sums_batch(*j, K, kmax, csize,
+                                     (size_t)job_quantum(cfg.quantum, K, csize),
+                                     budget, slots.sms, &est);
     std::lock_guard<std::mutex> g(mu);
     // CTA slots: shared memory and two CTAs per SM by registers
     size_t used_smem = 0;
